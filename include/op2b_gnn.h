@@ -45,6 +45,49 @@ int op2b_gemm_bf16(int M, int N, int K, const void *A, long a_m, long a_k, const
                    long b_n, long b_k, void *C, long ldc, int epi, const float *bias, void *Z,
                    const void *R, long ldr, int split_k, int engine, void *stream);
 
+/* One MLP of the network in one launch: y = L2(silu(L1(silu(L0(x))))) (+ R),
+ * L_l(x) = x W_l^T + b_l, hidden width 128, bf16 operands with FP32
+ * accumulation, hidden activations rounded to bf16: the same values as three
+ * op2b_gemm_bf16 calls.  The M x k input x is the concatenation of `nparts`
+ * (1 to 3) parts of 128 columns (a single part may have 8 to 64): row r of a
+ * part is x[r] or, with `rows`, x[rows[r]]; the first part has no `rows`.
+ * w[l]: [n_out][k_in] bf16; b[l]: floats.  nout 128: y (and R, or null) bf16,
+ * 32-byte aligned rows; nout 8 or 16: y FP32, no residual.  z0, a0, z1, a1 (M x 128 bf16
+ * rows): the hidden pre-activations and activations, all kept or all null. */
+typedef struct {
+  const void *x;   /* bf16 */
+  const int *rows; /* null: direct */
+  long ld;
+  int cols;
+} op2b_mlp_part;
+int op2b_gnn_mlp(int M, int nparts, const op2b_mlp_part *parts, const void *const *w,
+                 const float *const *b, int nout, const void *R, long ldr, void *y, long ldy,
+                 void *z0, void *a0, void *z1, void *a1, void *stream);
+
+/* Backward through one MLP in one launch: from dy (M x nout, bf16, leading
+ * dimension ldy) d1 = (dy W2) silu'(z1), d0 = (d1 W1) silu'(z0) (both M x 128,
+ * bf16) and, for each of the `nparts` (0 to 3) 128-column blocks of the input,
+ * dx[p] = or, with add[p], += the block of d0 W0 (FP32, leading dimension
+ * lddx[p]; 32-byte aligned rows).  kin: W0's columns. */
+int op2b_gnn_mlp_backward(int M, const void *dy, long ldy, int nout, const void *const *w,
+                          int kin, const void *z0, const void *z1, void *d0, void *d1,
+                          int nparts, float *const *dx, const long *lddx, const int *add,
+                          void *stream);
+
+/* The gradients of one MLP's weights and biases in one launch: for the layers
+ * l = 0, 1, 2 with inputs x (the parts, as op2b_gnn_mlp takes them), a0, a1,
+ * gw[l] ([n_out][k_in], 16-byte aligned) += d[l]^T x_l and gb[l] += column sums of d[l]
+ * (d[l]: M rows of bf16, leading dimension ldd[l]; 128 columns, d[2] nout). */
+int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int nout, int nparts,
+                    const op2b_mlp_part *parts, const void *a0, const void *a1,
+                    float *const *gw, float *const *gb, void *stream);
+
+/* dH[n] += sum over n's incoming edges k of dX[k, D:2D] + dX[rev[k], :D]: the
+ * node part of op2b_gnn_cat_grad for gradients dX (E x 2D, FP32) of the two
+ * gathered blocks alone. */
+int op2b_gnn_node_grad(int N, int D, const float *dX, long ldx, const int *off, const int *idx,
+                       const int *rev, float *dH, void *stream);
+
 /* Nonzero if a tensor-core GEMM gave up waiting on its tensor-core commit (a
  * bounded wait ran out); reset clears the flag.  Synchronises the device. */
 int op2b_gemm_error(int reset);

@@ -29,16 +29,12 @@
 
 #include "op2b_gnn.h"
 #include "op2b_runtime.h"
+#include "tc.cuh"
 
 namespace op2b {
 namespace {
 
-constexpr int kTileM = 128;
-constexpr int kTileN = 128;
-constexpr int kTileK = 64;
 constexpr int kThreads = 128;
-constexpr int kStageBytes = kTileM * kTileK * 2;  // one operand tile (16 KiB)
-constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s per mbarrier wait
 
 // i over the first n of 16 columns, unrolled so per-column arrays stay in registers
 #define FOR_LT_N(i) _Pragma("unroll") for (int i = 0; i < 16; i++) if (i < n)
@@ -61,90 +57,6 @@ struct GemmArgs {
   int staged;  // k_gemm_ws<16>: C (and Z) 16-byte aligned rows: stores through shared memory
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// shared-memory matrix descriptor, version 1 (sm_100), K-major with the
-// 128-byte swizzle (layout type 2 in bits 61-63): start address >> 4 in bits
-// 0-13, leading byte offset >> 4 in 16-29 (unused by a swizzled K-major
-// operand whose K step fits in the 128-byte row; 1 by convention), stride
-// byte offset >> 4 in 32-45 (1024: the distance between 8-row groups)
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// The same descriptor for an MN-major operand tile (128 MN x 64 K) as TMA
-// writes it with the 128-byte swizzle: two boxes of 64 MN x 64 K, 8 KiB
-// apart, each 64 rows of 128 bytes (64 MN values of one k) in 1024-byte
-// groups of 8 rows.  In the canonical MN-major layout ((8,n),(8,k)) :
-// ((1,LBO),(8,SBO)) in 16-byte units the leading byte offset is the 8 KiB
-// between the two 64-wide MN blocks and the stride byte offset the 1024 bytes
-// between groups of 8 k; a K step of 16 starts 2048 bytes further on.
-__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-  d |= (uint64_t)(8192 >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-// instruction descriptor, kind::f16: FP32 accumulator (bits 4-5 = 1), A and B
-// bf16 (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in
-// bits 17-22, M >> 4 in bits 24-28
-__device__ __forceinline__ uint32_t umma_idesc(int nt) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) |
-         ((uint32_t)(kTileM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer();
-  while (!mbar_try(bar, parity))
-    if (globaltimer() - t0 > kWaitNs) return false;
-  return true;
-}
-
-// SiLU and its derivative with the fast exponential and division (a few
-// ulp in FP32; the results are rounded to BF16).  Below z = -87 the
-// denominator passes 2^126 and the fast division gives 0, as the values
-// round to next to nothing anyway.
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
-  return s * (1.0f + z * (1.0f - s));
-}
-
 // bias[col .. col + n) into v (16-byte loads when aligned)
 __device__ __forceinline__ void add_bias16(float *v, const float *bias, int col, int n) {
   const float *b = bias + col;
@@ -160,15 +72,6 @@ __device__ __forceinline__ void add_bias16(float *v, const float *bias, int col,
   } else {
     FOR_LT_N(i) v[i] += b[i];
   }
-}
-
-// Shared-memory tile layout: K-major with the 128-byte swizzle.  Row r of the
-// 128 x 64 tile is 128 bytes (64 bf16) at (r / 8) * 1024 + (r % 8) * 128; its
-// 16-byte chunk j (k = 8j .. 8j+7) sits at chunk position j ^ (r % 8).  The
-// XOR spreads both the k-contiguous and the transposed staging stores over
-// all 32 banks; the tensor core undoes it from the descriptor's swizzle mode.
-__device__ __forceinline__ uint32_t sw128(int row, int kc) {
-  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((kc ^ (row & 7)) << 4));
 }
 
 // Stage one operand tile (128 rows x 64 k); rows >= nrows and k >= kend read
@@ -446,20 +349,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(GemmArgs g) {
 // tensor memory and returns.
 constexpr int kTmaStages = 3;
 
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 2)
 k_gemm_tma(GemmArgs g, const __grid_constant__ CUtensorMap ta,
            const __grid_constant__ CUtensorMap tb) {
@@ -616,17 +505,6 @@ k_gemm_tma(GemmArgs g, const __grid_constant__ CUtensorMap ta,
 // waits (bounded) for its issued loads and MMAs, frees tensor memory and
 // returns.
 constexpr int kWsStages = 4;
-
-__device__ __forceinline__ bool mbar_wait_or_fail(uint32_t bar, uint32_t parity,
-                                                  const volatile int *fail) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer();
-  while (!mbar_try(bar, parity)) {
-    if (*fail) return false;
-    if (globaltimer() - t0 > kWaitNs) return false;
-  }
-  return true;
-}
 
 struct WsTile {
   int m0, n0, nt, kb, nk;
@@ -1078,6 +956,22 @@ cudaError_t launch_ws(const GemmArgs &g, const CUtensorMap &ta, const CUtensorMa
 }
 
 }  // namespace
+
+int *tc_error_flag(const char *what, int *device) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) {
+    set_error("%s: device %d out of range", what, dev);
+    return nullptr;
+  }
+  if (!g_err_dev[dev]) {
+    if (!cuda_ok(cudaMalloc(&g_err_dev[dev], sizeof(int)), what)) return nullptr;
+    cudaMemset(g_err_dev[dev], 0, sizeof(int));
+  }
+  if (device) *device = dev;
+  return g_err_dev[dev];
+}
+
 }  // namespace op2b
 
 using namespace op2b;
@@ -1112,20 +1006,12 @@ extern "C" int op2b_gemm_bf16(int M, int N, int K, const void *A, long a_m, long
     return -1;
   }
   int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) {
-    set_error("op2b_gemm_bf16: device %d out of range", dev);
-    return -1;
-  }
-  if (!g_err_dev[dev]) {
-    if (!cuda_ok(cudaMalloc(&g_err_dev[dev], sizeof(int)), "op2b_gemm_bf16: error flag"))
-      return -1;
-    cudaMemset(g_err_dev[dev], 0, sizeof(int));
-  }
+  int *err = tc_error_flag("op2b_gemm_bf16", &dev);
+  if (!err) return -1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GemmArgs g{M,   N,   K,   (const __nv_bfloat16 *)A, a_m, a_k, (const __nv_bfloat16 *)B,
              b_n, b_k, C,   ldc, bias, (__nv_bfloat16 *)Z,     (const __nv_bfloat16 *)R,
-             ldr, epi, 0,   g_err_dev[dev]};
+             ldr, epi, 0,   err};
   {  // rows of C (and Z) that 16-byte stores can cover
     const long esize = epi == OP2B_EPI_STORE_F32 ? 4 : 2;
     g.staged = rt().opt_gemm_rows && epi != OP2B_EPI_ATOMIC_F32 &&

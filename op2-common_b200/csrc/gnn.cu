@@ -357,6 +357,19 @@ int op2b_gnn_cat_grad(int E, int N, int D, const float *dCat, long ldcat, float 
   return 0;
 }
 
+int op2b_gnn_node_grad(int N, int D, const float *dX, long ldx, const int *off, const int *idx,
+                       const int *rev, float *dH, void *stream) {
+  if (N < 0 || D <= 0 || D % 8 || ldx % 4 || ldx < 2 * D || !aligned16(dX) || !aligned16(dH)) {
+    set_error("op2b_gnn_node_grad: D a multiple of 8, ldx >= 2D, aligned arrays");
+    return -1;
+  }
+  if (N == 0) return 0;
+  // the kernel's blocks follow the one of the edge's own state, absent here
+  k_cat_grad_nodes<<<grid_for((long)N * (D / 8)), kBlock, 0, S_>>>(N, D, dX - D, ldx, off, idx,
+                                                                  rev, dH);
+  return launched("op2b_gnn_node_grad") ? 0 : -1;
+}
+
 int op2b_gnn_colsum(int M, int N, const void *dz, long ld, float *db, void *stream) {
   if (M < 0 || N <= 0 || ld < N) {
     set_error("op2b_gnn_colsum: bad sizes");

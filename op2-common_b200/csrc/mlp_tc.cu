@@ -1,0 +1,1272 @@
+// The graph network's three-layer MLPs (Linear-SiLU-Linear-SiLU-Linear, hidden
+// width 128) as ONE persistent tensor-core kernel a pass over the rows, forward
+// (k_mlp_fwd).  A layer by layer product writes each hidden activation to
+// memory and reads it back, and the edge MLP's input [e, h_src, h_dst] had to
+// be gathered into a 384-wide array first; here
+//   * the three weight matrices stay in shared memory (K-major, 128-byte
+//     swizzle) for the whole kernel: 160 KiB for the edge MLP (K = 384);
+//   * warps 0-1 load the 128-row input tile in 64-column blocks by cp.async
+//     into a ring of four 16 KiB stages, each row from its own address: a
+//     direct row, or the row of h an index names, so no gathered copy exists;
+//   * warp 2 issues the MMAs: layer 0 of a tile runs two tiles ahead, layers 1
+//     and 2 as their operands appear, so the tensor core and the activations
+//     of two tiles overlap;
+//   * warps 4-19 are the epilogues, eight for even and eight for odd tiles (two
+//     a TMEM lane quarter, 64 columns each): bias and SiLU on the FP32
+//     accumulator, rounded to BF16 and put back into TENSOR MEMORY as the next
+//     layer's A operand -- the hidden activations never leave the SM (in
+//     training they are also stored);
+//   * tensor memory: three 128-column accumulators taken in turn and two
+//     64-column BF16 operands, all 512 columns.
+// The MMAs run over K in the order of k_gemm_ws and every value is rounded
+// where the layer-by-layer products rounded it, so the results are the same
+// bits.  Every wait is bounded and also ends when another role has recorded a
+// failure; the CTA then stops, waits (bounded) for the MMAs it issued, frees
+// tensor memory and returns.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "op2b_gnn.h"
+#include "op2b_runtime.h"
+#include "tc.cuh"
+
+namespace op2b {
+namespace {
+
+constexpr int kW = 128;                 // hidden width
+constexpr int kRing = 4;                // input stages of 128 rows x 64 columns
+constexpr int kLag = 2;                 // cp.async groups left in flight before a stage is handed on
+constexpr int kProducerWarps = 2, kRowReps = kTileM / (4 * kProducerWarps);
+constexpr int kMmaWarp = 2, kEpiWarp0 = 4, kEpiWarps = 16;
+// 20 warps (one idle): five a scheduler, whose 16K registers allow 96 a thread
+constexpr int kMlpThreads = 32 * (kEpiWarp0 + kEpiWarps);
+
+struct MlpPart {
+  const __nv_bfloat16 *p;
+  const int *rows;  // null: row r is row r
+  long ld;
+  int cols;
+};
+
+struct MlpArgs {
+  int M, k0, nout;
+  MlpPart part[3];
+  const __nv_bfloat16 *W[3];
+  const float *b[3];
+  __nv_bfloat16 *Z0, *A0, *Z1, *A1;  // training: pre-activations and activations (rows of 128)
+  const __nv_bfloat16 *R;            // residual added to the result, or null
+  long ldr;
+  void *Y;
+  long ldy;
+  int *err;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in) {
+  const int n = in ? 16 : 0;  // 0 source bytes: the chunk is zero-filled
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n)
+               : "memory");
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+      : "memory");
+}
+
+// D (+)= A B with A in shared memory / in tensor memory
+__device__ __forceinline__ void umma_ss(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc,
+                                        uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+}
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t db, uint32_t idesc,
+                                        uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(db), "r"(idesc), "r"(acc));
+}
+
+// 32 columns of the lane's row
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float *v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t *r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
+
+// one 32-byte sector of a lane's row
+__device__ __forceinline__ void st_sector(void *p, const uint32_t *r) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void ld_sector(const void *p, uint32_t *r) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "l"(p)
+               : "memory");
+}
+
+// 16 floats to 16 BF16 (element 2i in the low half of word i)
+__device__ __forceinline__ void pack16(const float *v, uint32_t *r) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    r[i] = *reinterpret_cast<const uint32_t *>(&t);
+  }
+}
+
+// add 16 floats of shared memory (the same address in every lane)
+__device__ __forceinline__ void add_smem16(float *v, const float *b) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float4 t = reinterpret_cast<const float4 *>(b)[i];
+    v[4 * i] += t.x, v[4 * i + 1] += t.y, v[4 * i + 2] += t.z, v[4 * i + 3] += t.w;
+  }
+}
+
+// a weight matrix [nrows][k] into K-major tiles of 128 rows x 64 columns,
+// zeros past its rows and columns (asynchronous: wait for the cp.async group)
+__device__ __forceinline__ void load_weights(uint32_t dst, const __nv_bfloat16 *w, int nrows,
+                                             int k, int tiles) {
+  for (int i = threadIdx.x; i < tiles * 1024; i += kMlpThreads) {
+    const int t = i >> 10, row = (i >> 3) & 127, kc = i & 7, col = t * 64 + kc * 8;
+    const bool in = row < nrows && col < k;
+    cp_async16(dst + t * kStageBytes + sw128(row, kc), in ? w + (long)row * k + col : w, in);
+  }
+}
+
+// NC: 64-column blocks of the input (1, 2, 4 or 6); STORE: keep Z0, A0, Z1, A1
+template <int NC, bool STORE>
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constant__ MlpArgs g,
+                                                            int ntiles) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t *s_w0 = smem, *s_w1 = s_w0 + NC * kStageBytes, *s_w2 = s_w1 + 2 * kStageBytes;
+  uint8_t *s_ring = s_w2 + 2 * kStageBytes;
+  float *s_bias = reinterpret_cast<float *>(s_ring + kRing * kStageBytes);  // 3 x 128
+  // full[kRing], empty[kRing], first_full[2], acc_full[2], h_full[2], d_free[3], done
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_bias + 3 * kW);
+  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 10);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto full = [&](int s) { return smem_u32(&bars[s]); };
+  auto empty = [&](int s) { return smem_u32(&bars[kRing + s]); };
+  auto first_full = [&](int s) { return smem_u32(&bars[2 * kRing + s]); };  // layer 0 done
+  auto acc_full = [&](int s) { return smem_u32(&bars[2 * kRing + 2 + s]); };  // layer 1, 2 done
+  auto h_full = [&](int s) { return smem_u32(&bars[2 * kRing + 4 + s]); };
+  auto d_free = [&](int d) { return smem_u32(&bars[2 * kRing + 6 + d]); };
+  const uint32_t done = smem_u32(&bars[2 * kRing + 9]);
+  volatile int *fail = &s_fail;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRing; s++) {
+      mbar_init(full(s), kProducerWarps);
+      mbar_init(empty(s), 1);
+    }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(first_full(s), 1);
+      mbar_init(acc_full(s), 1);
+      mbar_init(h_full(s), kEpiWarps / 2);
+    }
+    for (int d = 0; d < 3; d++) mbar_init(d_free(d), kEpiWarps / 2);
+    mbar_init(done, 1);
+    s_fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&s_taddr)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  load_weights(smem_u32(s_w0), g.W[0], kW, g.k0, NC);
+  load_weights(smem_u32(s_w1), g.W[1], kW, kW, 2);
+  load_weights(smem_u32(s_w2), g.W[2], g.nout, kW, 2);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int i = threadIdx.x; i < 3 * kW; i += kMlpThreads) {
+    const int l = i / kW, c = i - l * kW;
+    s_bias[i] = l < 2 || c < g.nout ? g.b[l][c] : 0.0f;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_taddr;
+  const int nloc = ntiles > (int)blockIdx.x
+                       ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1
+                       : 0;  // this CTA's tiles
+  // the accumulator of local tile j, the BF16 operand of slot j & 1
+  const auto acc_of = [&](int j) { return tmem + (uint32_t)(j % 3) * kW; };
+  const auto hid_of = [&](int s) { return tmem + 3u * kW + (uint32_t)(s * 64); };
+
+  if (warp < kProducerWarps) {
+    // a stage is 1024 chunks of 16 bytes: thread t copies chunk t % 8 of the
+    // rows t / 8 + 8 i, eight lanes a row, so its place in the swizzled tile
+    // moves by 1024 bytes with i
+    const int kc = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const uint32_t place = smem_u32(s_ring) + sw128(r0, kc);
+    int it = 0, handed = 0;  // stages issued, stages handed to the MMAs
+    bool ok = true;
+    auto hand_on = [&](int upto) {  // the copies of stages [handed, upto) have landed
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kRing));
+      handed = upto;
+    };
+    int rows[2][kRowReps];  // the indexed parts' rows; loaded a tile ahead
+    auto load_rows = [&](int p, int j) {
+      const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + r0;
+      const int *idx = g.part[p + 1].rows;
+#pragma unroll
+      for (int i = 0; i < kRowReps; i++) {
+        const int r = m0 + 8 * i;
+        rows[p][i] = idx && r < g.M ? __ldg(idx + r) : r;
+      }
+    };
+    if (NC > 2 && nloc > 0) load_rows(0, 0);
+    if (NC > 4 && nloc > 0) load_rows(1, 0);
+    for (int j = 0; j < nloc && ok; j++) {
+      const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM;
+      const bool whole = m0 + kTileM <= g.M;
+#pragma unroll
+      for (int c = 0; c < NC; c++, it++) {
+        const int st = it % kRing;
+        if (it >= kRing) {
+          const uint32_t par = (uint32_t)((it / kRing - 1) & 1);
+          if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
+            if (handed < it) {  // nothing to overlap with: hand on what is in flight
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+              hand_on(it);
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), par, fail));
+            if (!ok) {
+              if (lane == 0) atomicExch(&s_fail, 1);
+              break;
+            }
+          }
+        }
+        const int part = NC == 1 ? 0 : c / 2, col = (NC == 1 ? 0 : (c & 1) * 64) + kc * 8;
+        const MlpPart &P = g.part[part];
+        const __nv_bfloat16 *base = P.p + col;
+        const uint32_t dst = place + (uint32_t)st * kStageBytes;
+        const bool incol = NC > 1 || col < P.cols;
+        if (whole && incol) {
+#pragma unroll
+          for (int i = 0; i < kRowReps; i++)
+            cp_async16(dst + i * 1024,
+                       base + (part > 0 ? rows[part > 0 ? part - 1 : 0][i] : m0 + r0 + 8 * i) * P.ld);
+        } else {
+#pragma unroll
+          for (int i = 0; i < kRowReps; i++) {
+            const bool in = incol && m0 + r0 + 8 * i < g.M;
+            cp_async16(dst + i * 1024,
+                       in ? base + (part > 0 ? rows[part > 0 ? part - 1 : 0][i] : m0 + r0 + 8 * i) * P.ld
+                          : P.p, in);
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (part > 0 && (c & 1) && j + 1 < nloc) load_rows(part - 1, j + 1);
+        if (it + 1 - handed > kLag) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
+          hand_on(it + 1 - kLag);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    hand_on(it);
+  } else if (warp == kMmaWarp) {
+    if (lane == 0) {  // MMA issuer: whatever has its operands next
+      const uint32_t idesc = umma_idesc(kW), idesc2 = umma_idesc((g.nout + 15) & ~15);
+      const uint32_t w0 = smem_u32(s_w0), w1 = smem_u32(s_w1), w2 = smem_u32(s_w2);
+      int jf = 0, cf = 0, it = 0;            // layer 0: next tile and block; stages used
+      int jn[2] = {0, 1}, layer[2] = {1, 1};  // per slot: next tile and layer (1 or 2)
+      unsigned long long t0 = 0;
+      while (jf < nloc || jn[0] < nloc || jn[1] < nloc) {
+        bool moved = false;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+          const int j = jn[s];
+          if (j >= nloc || !mbar_test(h_full(s), (uint32_t)((layer[s] - 1) & 1))) continue;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t b = layer[s] == 1 ? w1 : w2;
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            umma_ts(acc_of(j), hid_of(s) + k * 8,
+                    umma_desc(b + (uint32_t)(k >> 2) * kStageBytes + (k & 3) * 32),
+                    layer[s] == 1 ? idesc : idesc2, k > 0);
+          umma_commit(acc_full(s));
+          if (++layer[s] == 3) layer[s] = 1, jn[s] = j + 2;
+          moved = true;
+        }
+        // the tile's accumulator must have been read, and the slot's tile
+        // before it must be past layer 0 (one completion of first_full ahead)
+        const int sf = jf & 1;
+        if (jf < nloc && (jn[sf] == jf || (jn[sf] == jf - 2 && layer[sf] == 2)) &&
+            (cf > 0 || jf < 3 || mbar_test(d_free(jf % 3), (uint32_t)((jf / 3 - 1) & 1)))) {
+          const int st = it % kRing;
+          if (mbar_test(full(st), (uint32_t)((it / kRing) & 1))) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(s_ring + (size_t)st * kStageBytes);
+            const uint32_t b = w0 + (uint32_t)cf * kStageBytes;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              umma_ss(acc_of(jf), umma_desc(a + k * 32), umma_desc(b + k * 32), idesc,
+                      cf + k > 0);
+            umma_commit(empty(st));
+            it++;
+            if (++cf == NC) {
+              umma_commit(first_full(sf));
+              cf = 0;
+              jf++;
+            }
+            moved = true;
+          }
+        }
+        if (moved) {
+          t0 = 0;
+        } else {
+          if (*fail) break;
+          const unsigned long long t = globaltimer();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > kWaitNs) {
+            atomicExch(&s_fail, 1);
+            break;
+          }
+        }
+      }
+      umma_commit(done);
+    }
+  } else if (warp >= kEpiWarp0) {  // epilogue
+    const int s = (warp - kEpiWarp0) >> 3, quarter = warp & 3;
+    const int c0 = (((warp - kEpiWarp0) >> 2) & 1) * 64;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
+    bool ok = true;
+    auto wait_for = [&](uint32_t bar, int n) {  // the n-th completion (from 0) of bar
+      ok = __all_sync(0xffffffffu, mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail));
+      if (!ok && lane == 0) atomicExch(&s_fail, 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return ok;
+    };
+    auto signal = [&](uint32_t bar) {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    for (int j = s, jj = 0; j < nloc; j += 2, jj++) {
+      const long row = (long)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + quarter * 32 + lane;
+      const bool live = row < g.M;
+      const uint32_t acc = acc_of(j) + lanes + (uint32_t)c0;
+#pragma unroll 1
+      for (int l = 0; l < 2; l++) {
+        if (!(l == 0 ? wait_for(first_full(s), jj) : wait_for(acc_full(s), 2 * jj))) break;
+        __nv_bfloat16 *Z = l == 0 ? g.Z0 : g.Z1, *A = l == 0 ? g.A0 : g.A1;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          float v[32];
+          tmem_ld32(acc + k * 32, v);
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            float *u = v + 16 * m;
+            const int c = c0 + k * 32 + m * 16;
+            uint32_t p[8];
+            add_smem16(u, s_bias + l * kW + c);
+            if (STORE) {
+              pack16(u, p);
+              if (live) st_sector(Z + row * kW + c, p);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) u[i] = silu(u[i]);
+            pack16(u, p);
+            if (STORE && live) st_sector(A + row * kW + c, p);
+            tmem_st8(hid + k * 16 + m * 8, p);
+          }
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        signal(h_full(s));
+      }
+      if (!ok) break;
+      if (g.nout == kW) {
+        uint32_t res[4][8];
+        if (g.R && live) {  // in flight while the last layer's MMAs run
+#pragma unroll
+          for (int k = 0; k < 4; k++) ld_sector(g.R + row * g.ldr + c0 + k * 16, res[k]);
+        }
+        if (!wait_for(acc_full(s), 2 * jj + 1)) break;
+        __nv_bfloat16 *y = reinterpret_cast<__nv_bfloat16 *>(g.Y) + row * g.ldy + c0;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          float v[32];
+          tmem_ld32(acc + k * 32, v);
+          if (k == 1) signal(d_free(j % 3));  // the accumulator has been read
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            float *u = v + 16 * m;
+            uint32_t p[8];
+            add_smem16(u, s_bias + 2 * kW + c0 + k * 32 + m * 16);
+            if (g.R && live) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                const float2 t = __bfloat1622float2(
+                    *reinterpret_cast<__nv_bfloat162 *>(&res[2 * k + m][i]));
+                u[2 * i] += t.x;
+                u[2 * i + 1] += t.y;
+              }
+            }
+            pack16(u, p);
+            if (live) st_sector(y + k * 32 + m * 16, p);
+          }
+        }
+      } else {  // the decoder: nout <= 16 FP32 columns
+        if (!wait_for(acc_full(s), 2 * jj + 1)) break;
+        float v[32];
+        if (c0 == 0) tmem_ld32(acc, v);
+        signal(d_free(j % 3));
+        if (c0 == 0 && live) {
+          add_smem16(v, s_bias + 2 * kW);
+          float *y = reinterpret_cast<float *>(g.Y) + row * g.ldy;
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            if (i < g.nout)
+              *reinterpret_cast<float4 *>(y + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // every issued MMA has finished once "done" has arrived
+  if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+  if (threadIdx.x == 0 && s_fail) atomicExch(g.err, 1);
+}
+
+int sm_count(int dev) {
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm > 0 ? nsm : 148;
+}
+
+constexpr size_t mlp_smem(int nc) {
+  return (size_t)(nc + 4 + kRing) * kStageBytes + 3 * kW * sizeof(float) +
+         (2 * kRing + 11) * sizeof(uint64_t) + 1024;
+}
+
+template <int NC, bool STORE>
+cudaError_t launch_mlp(const MlpArgs &g, cudaStream_t s, int dev) {
+  static bool attr[16] = {};  // per device, once
+  if (!attr[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_mlp_fwd<NC, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem(NC));
+    if (e != cudaSuccess) return e;
+    attr[dev] = true;
+  }
+  const int ntiles = (g.M + kTileM - 1) / kTileM;
+  k_mlp_fwd<NC, STORE><<<std::min(ntiles, sm_count(dev)), kMlpThreads, mlp_smem(NC), s>>>(g,
+                                                                                         ntiles);
+  return cudaGetLastError();
+}
+
+template <bool STORE> cudaError_t launch_mlp(const MlpArgs &g, int nc, cudaStream_t s, int dev) {
+  switch (nc) {
+    case 1: return launch_mlp<1, STORE>(g, s, dev);
+    case 2: return launch_mlp<2, STORE>(g, s, dev);
+    case 4: return launch_mlp<4, STORE>(g, s, dev);
+    default: return launch_mlp<6, STORE>(g, s, dev);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Backward through one MLP (k_mlp_bwd): from the gradient dy of its output,
+//   dZ1 = (dy W2) silu'(Z1), dZ0 = (dZ1 W1) silu'(Z0), dx = dZ0 W0
+// in one pass over the row tiles, organised as k_mlp_fwd: the weights stay in
+// shared memory (here as MN-major B operands, so no transposed copy is made),
+// dZ1 and dZ0 go from one product to the next through tensor memory and are
+// also stored, as k_mlp_dw needs them.  dx leaves as FP32 column blocks of 128,
+// each stored or added to what is there, so the sums that follow (dE, dH)
+// need no pass of their own.  The products' and roundings' order is that of the
+// layer-by-layer products.
+struct MlpBwdArgs {
+  int M, nout, kin, nparts;
+  const __nv_bfloat16 *dy;
+  long ldy;
+  const __nv_bfloat16 *W[3];
+  const __nv_bfloat16 *Z0, *Z1;
+  __nv_bfloat16 *d0, *d1;  // dZ0, dZ1 (rows of 128)
+  float *dx[3];
+  long lddx[3];
+  int add[3];  // 1: dx += , 0: dx =
+  int *err;
+};
+
+// rows [0, nrows) of a weight matrix [nrows][ld], columns col0 .. col0 + 127, as
+// MN-major tiles: for every 64 rows two boxes of 64 columns x 64 rows
+__device__ __forceinline__ void load_weights_mn(uint32_t dst, const __nv_bfloat16 *w, int nrows,
+                                                int ld, int col0, int tiles) {
+  for (int i = threadIdx.x; i < tiles * 1024; i += kMlpThreads) {
+    const int t = i >> 10, row = (i >> 4) & 63, c = i & 15, k = t * 64 + row, col = col0 + c * 8;
+    const bool in = k < nrows && col < ld;
+    cp_async16(dst + t * kStageBytes + (c >> 3) * (kStageBytes / 2) + sw128(row, c & 7),
+               in ? w + (long)k * ld + col : w, in);
+  }
+}
+
+// NP: 128-column blocks of dx (0 to 3)
+template <int NP>
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constant__ MlpBwdArgs g,
+                                                            int ntiles) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t *s_w2 = smem, *s_w1 = s_w2 + 2 * kStageBytes, *s_w0 = s_w1 + 2 * kStageBytes;
+  uint8_t *s_ring = s_w0 + 2 * NP * kStageBytes;
+  // full[kRing], empty[kRing], acc_full[2], h_full[2], d_free[2], done
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_ring + kRing * kStageBytes);
+  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 7);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto full = [&](int s) { return smem_u32(&bars[s]); };
+  auto empty = [&](int s) { return smem_u32(&bars[kRing + s]); };
+  auto acc_full = [&](int s) { return smem_u32(&bars[2 * kRing + s]); };
+  auto h_full = [&](int s) { return smem_u32(&bars[2 * kRing + 2 + s]); };
+  auto d_free = [&](int s) { return smem_u32(&bars[2 * kRing + 4 + s]); };
+  const uint32_t done = smem_u32(&bars[2 * kRing + 6]);
+  volatile int *fail = &s_fail;
+  const int nkb = g.nout > 64 ? 2 : 1;  // 64-column blocks of dy
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRing; s++) {
+      mbar_init(full(s), kProducerWarps);
+      mbar_init(empty(s), 1);
+    }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(acc_full(s), 1);
+      mbar_init(h_full(s), kEpiWarps / 2);
+      mbar_init(d_free(s), kEpiWarps / 2);
+    }
+    mbar_init(done, 1);
+    s_fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&s_taddr)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  load_weights_mn(smem_u32(s_w2), g.W[2], g.nout, kW, 0, nkb);
+  load_weights_mn(smem_u32(s_w1), g.W[1], kW, kW, 0, 2);
+  for (int p = 0; p < NP; p++)
+    load_weights_mn(smem_u32(s_w0 + 2 * p * kStageBytes), g.W[0], kW, g.kin, p * kW, 2);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_taddr;
+  const int nloc = ntiles > (int)blockIdx.x
+                       ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1
+                       : 0;
+  const auto acc_of = [&](int s) { return tmem + (uint32_t)s * kW; };
+  const auto hid_of = [&](int s) { return tmem + 3u * kW + (uint32_t)(s * 64); };
+
+  if (warp < kProducerWarps) {
+    const int kc = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const uint32_t place = smem_u32(s_ring) + sw128(r0, kc);
+    int it = 0, handed = 0;
+    bool ok = true;
+    auto hand_on = [&](int upto) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kRing));
+      handed = upto;
+    };
+    for (int j = 0; j < nloc && ok; j++) {
+      const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + r0;
+      for (int c = 0; c < nkb; c++, it++) {
+        const int st = it % kRing;
+        if (it >= kRing) {
+          const uint32_t par = (uint32_t)((it / kRing - 1) & 1);
+          if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
+            if (handed < it) {
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+              hand_on(it);
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), par, fail));
+            if (!ok) {
+              if (lane == 0) atomicExch(&s_fail, 1);
+              break;
+            }
+          }
+        }
+        const int col = c * 64 + kc * 8;
+        const uint32_t dst = place + (uint32_t)st * kStageBytes;
+#pragma unroll
+        for (int i = 0; i < kRowReps; i++) {
+          const bool in = col < g.nout && m0 + 8 * i < g.M;
+          cp_async16(dst + i * 1024, in ? g.dy + (long)(m0 + 8 * i) * g.ldy + col : g.dy, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (it + 1 - handed > kLag) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
+          hand_on(it + 1 - kLag);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    hand_on(it);
+  } else if (warp == kMmaWarp) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc(kW) | 1u << 16;  // B MN-major
+      const uint32_t w2 = smem_u32(s_w2), w1 = smem_u32(s_w1), w0 = smem_u32(s_w0);
+      // a slot's phases: 0 dy W2 (block by block, in tile order over the slots),
+      // 1 dZ1 W1, 2 .. NP + 1 the blocks of dZ0 W0
+      int jn[2] = {0, 1}, ph[2] = {0, 0}, nh[2] = {0, 0}, nd[2] = {0, 0};
+      int jf = 0, cf = 0, it = 0;
+      unsigned long long t0 = 0;
+      while (jn[0] < nloc || jn[1] < nloc) {
+        bool moved = false;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+          if (jn[s] >= nloc) continue;
+          if (ph[s] == 0) {
+            if (jf != jn[s]) continue;  // dy's stages arrive in tile order
+            // the accumulator has been read (the NP or one read of the tile before)
+            if (cf == 0 && jf >= 2 && !mbar_test(d_free(s), (uint32_t)((nd[s] - 1) & 1))) continue;
+            const int st = it % kRing;
+            if (!mbar_test(full(st), (uint32_t)((it / kRing) & 1))) continue;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(s_ring + (size_t)st * kStageBytes);
+            const uint32_t b = w2 + (uint32_t)cf * kStageBytes;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              umma_ss(acc_of(s), umma_desc(a + k * 32), umma_desc_mn(b + k * 2048), idesc,
+                      cf + k > 0);
+            umma_commit(empty(st));
+            it++;
+            if (++cf == nkb) {
+              umma_commit(acc_full(s));
+              cf = 0;
+              jf++;
+              ph[s] = 1;
+            }
+          } else {
+            if (ph[s] <= 2) {
+              if (!mbar_test(h_full(s), (uint32_t)(nh[s] & 1))) continue;
+              nh[s]++;
+            } else if (!mbar_test(d_free(s), (uint32_t)((nd[s] - 1) & 1))) {
+              continue;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t b = ph[s] == 1 ? w1 : w0 + (uint32_t)(2 * (ph[s] - 2)) * kStageBytes;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+              umma_ts(acc_of(s), hid_of(s) + k * 8,
+                      umma_desc_mn(b + (uint32_t)(k >> 2) * kStageBytes + (k & 3) * 2048), idesc,
+                      k > 0);
+            umma_commit(acc_full(s));
+            if (ph[s] >= 2 || NP == 0) nd[s]++;  // this product's accumulator is read to d_free
+            if (++ph[s] == NP + 2) {
+              ph[s] = 0;
+              jn[s] += 2;
+            }
+          }
+          moved = true;
+        }
+        if (moved) {
+          t0 = 0;
+        } else {
+          if (*fail) break;
+          const unsigned long long t = globaltimer();
+          if (t0 == 0) t0 = t;
+          if (t - t0 > kWaitNs) {
+            atomicExch(&s_fail, 1);
+            break;
+          }
+        }
+      }
+      umma_commit(done);
+    }
+  } else if (warp >= kEpiWarp0) {
+    const int s = (warp - kEpiWarp0) >> 3, quarter = warp & 3;
+    const int c0 = (((warp - kEpiWarp0) >> 2) & 1) * 64;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    const uint32_t acc = acc_of(s) + lanes + (uint32_t)c0;
+    const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
+    bool ok = true;
+    int na = 0;
+    auto wait_acc = [&]() {
+      ok = __all_sync(0xffffffffu, mbar_wait_or_fail(acc_full(s), (uint32_t)(na & 1), fail));
+      if (!ok && lane == 0) atomicExch(&s_fail, 1);
+      na++;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return ok;
+    };
+    auto signal = [&](uint32_t bar) {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    for (int j = s; j < nloc && ok; j += 2) {
+      const long row = (long)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + quarter * 32 + lane;
+      const bool live = row < g.M;
+#pragma unroll 1
+      for (int l = 1; l >= 0; l--) {  // dZ1, then dZ0
+        const __nv_bfloat16 *Z = (l ? g.Z1 : g.Z0) + row * kW + c0;
+        __nv_bfloat16 *d = (l ? g.d1 : g.d0) + row * kW + c0;
+        uint32_t z[4][8];
+        if (live) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) ld_sector(Z + k * 16, z[k]);
+        }
+        if (!wait_acc()) break;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          float v[32];
+          tmem_ld32(acc + k * 32, v);
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            float *u = v + 16 * m;
+            uint32_t p[8];
+            if (live) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                const float2 t =
+                    __bfloat1622float2(*reinterpret_cast<__nv_bfloat162 *>(&z[2 * k + m][i]));
+                u[2 * i] *= silu_grad(t.x);
+                u[2 * i + 1] *= silu_grad(t.y);
+              }
+            }
+            pack16(u, p);
+            if (live) st_sector(d + k * 32 + m * 16, p);
+            if (NP > 0 || l == 1) tmem_st8(hid + k * 16 + m * 8, p);
+          }
+        }
+        if (NP > 0 || l == 1) {
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          signal(h_full(s));
+        } else {
+          signal(d_free(s));
+        }
+      }
+      if (!ok) break;
+#pragma unroll 1
+      for (int p = 0; p < NP; p++) {
+        float *dx = g.dx[p] + row * g.lddx[p] + c0;
+        if (!wait_acc()) break;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          float v[32];
+          uint32_t o[4][8];
+          if (g.add[p] && live) {
+#pragma unroll
+            for (int m = 0; m < 4; m++) ld_sector(dx + k * 32 + m * 8, o[m]);
+          }
+          tmem_ld32(acc + k * 32, v);
+          if (k == 1) signal(d_free(s));
+          if (live) {
+            if (g.add[p]) {
+#pragma unroll
+              for (int i = 0; i < 32; i++) v[i] = __uint_as_float(o[i >> 3][i & 7]) + v[i];
+            }
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+              st_sector(dx + k * 32 + m * 8, reinterpret_cast<const uint32_t *>(v + m * 8));
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+  if (threadIdx.x == 0 && s_fail) atomicExch(g.err, 1);
+}
+
+// ---------------------------------------------------------------------------
+// The weight and bias gradients of one MLP's three layers in one launch
+// (k_mlp_dw): dW_l += d_l^T X_l and db_l += column sums of d_l, over all rows.
+// The CTAs are shared out among the layers by the bytes each reads, and a CTA
+// keeps its layer's whole 128 x (up to 384) gradient in tensor memory while it
+// walks its share of the rows, 64 at a time: d is read once for all column
+// blocks of X (the tiled product read it once a block), X's indexed blocks come
+// from their own rows (no gathered copy), and the column sums are one more
+// product, with a block of ones.  Operand tiles (64 rows x 128 columns, MN-major)
+// arrive by cp.async into a ring of 12 x 16 KiB.  The partial results are added
+// to the gradient with 16-byte reductions.
+struct MlpDwJob {
+  const __nv_bfloat16 *d;  // [M][ldd], nout columns
+  long ldd;
+  int nout, kin, nparts;
+  MlpPart part[3];
+  float *gw, *gb;
+  int cta0, ctas;  // the CTAs of the job
+};
+struct MlpDwArgs {
+  int M, njobs;
+  MlpDwJob job[3];
+  int *err;
+};
+constexpr int kDwRing = 12, kDwLag = 8;
+constexpr int kDwProducers = 4;                       // warps
+constexpr int kDwThreads = 32 * (kDwProducers + 4);   // + MMA warp (4) and three idle until the end
+constexpr size_t kDwSmem = (size_t)kDwRing * kStageBytes + 2048 + (2 * kDwRing + 3) * 8 + 1024;
+
+__device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
+               "f"(d)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant__ MlpDwArgs g) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t *s_ring = smem, *s_ones = smem + (size_t)kDwRing * kStageBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_ones + 2048);
+  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kDwRing + 1);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto full = [&](int s) { return smem_u32(&bars[s]); };
+  auto empty = [&](int s) { return smem_u32(&bars[kDwRing + s]); };
+  const uint32_t done = smem_u32(&bars[2 * kDwRing]);
+  volatile int *fail = &s_fail;
+  int q = 0;
+  while (q + 1 < g.njobs && (int)blockIdx.x >= g.job[q + 1].cta0) q++;
+  const MlpDwJob &J = g.job[q];
+  const int P = J.nparts;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kDwRing; s++) {
+      mbar_init(full(s), kDwProducers);
+      mbar_init(empty(s), 1);
+    }
+    mbar_init(done, 1);
+    s_fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kDwProducers) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&s_taddr)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  for (int i = threadIdx.x; i < 512; i += kDwThreads)  // 16 x 64 BF16 ones
+    reinterpret_cast<uint32_t *>(s_ones)[i] = 0x3f803f80u;
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_taddr;
+  // the CTA's blocks of 64 rows
+  const long nblk = ((long)g.M + 63) / 64, me = (int)blockIdx.x - J.cta0;
+  const int b0 = (int)(nblk * me / J.ctas), b1 = (int)(nblk * (me + 1) / J.ctas);
+
+  if (warp < kDwProducers) {
+    // 16 lanes a row of 256 bytes: thread t copies chunk t % 16 of the rows
+    // t / 16 + 8 i, so its place moves by 1024 bytes with i
+    const int c = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+    const uint32_t place = smem_u32(s_ring) + (c >> 3) * (kStageBytes / 2) + sw128(r0, c & 7);
+    int it = 0, handed = 0;
+    bool ok = true;
+    auto hand_on = [&](int upto) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kDwRing));
+      handed = upto;
+    };
+    int rows[2][8];
+    auto load_rows = [&](int p, int b) {
+      const int *idx = J.part[p].rows;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int r = b * 64 + r0 + 8 * i;
+        rows[p - 1][i] = idx && r < g.M ? __ldg(idx + r) : r;
+      }
+    };
+    if (P > 1 && b0 < b1) load_rows(1, b0);
+    if (P > 2 && b0 < b1) load_rows(2, b0);
+    for (int b = b0; b < b1 && ok; b++) {
+#pragma unroll
+      for (int t = 0; t < 4; t++) {  // d, then X's blocks
+        if (t > P) break;
+        const int st = it % kDwRing;
+        if (it >= kDwRing) {
+          const uint32_t par = (uint32_t)((it / kDwRing - 1) & 1);
+          if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
+            if (handed < it) {
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+              hand_on(it);
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), par, fail));
+            if (!ok) {
+              if (lane == 0) atomicExch(&s_fail, 1);
+              break;
+            }
+          }
+        }
+        const __nv_bfloat16 *x = t == 0 ? J.d : J.part[t > 0 ? t - 1 : 0].p;
+        const long ld = t == 0 ? J.ldd : J.part[t > 0 ? t - 1 : 0].ld;
+        const bool incol = c * 8 < (t == 0 ? J.nout : J.part[t > 0 ? t - 1 : 0].cols);
+        const uint32_t dst = place + (uint32_t)st * kStageBytes;
+        const int m0 = b * 64 + r0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const bool in = incol && m0 + 8 * i < g.M;
+          const long r = t >= 2 ? rows[t >= 2 ? t - 2 : 0][i] : m0 + 8 * i;
+          cp_async16(dst + i * 1024, in ? x + r * ld + c * 8 : x, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (t >= 2 && b + 1 < b1) load_rows(t - 1, b + 1);
+        it++;
+        if (it - handed > kDwLag) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kDwLag) : "memory");
+          hand_on(it - kDwLag);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    hand_on(it);
+  } else if (warp == kDwProducers && lane == 0) {
+    const uint32_t mn = 1u << 15 | 1u << 16;  // A and B MN-major
+    const uint32_t idesc = umma_idesc(kW) | mn, idesc1 = umma_idesc(16) | 1u << 15;
+    const uint32_t ones = smem_u32(s_ones);
+    int it = 0;
+    bool ok = true;
+    auto wait = [&](int st, int n) {
+      ok = ok && mbar_wait_or_fail(full(st), (uint32_t)(n & 1), fail);
+      if (!ok) atomicExch(&s_fail, 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    };
+    for (int b = b0; b < b1 && ok; b++) {
+      const int sd = it % kDwRing;
+      wait(sd, it / kDwRing);
+      it++;
+      const uint32_t a = smem_u32(s_ring + (size_t)sd * kStageBytes);
+      for (int p = 0; p < P && ok; p++) {
+        const int st = it % kDwRing;
+        wait(st, it / kDwRing);
+        it++;
+        if (!ok) break;
+        const uint32_t x = smem_u32(s_ring + (size_t)st * kStageBytes);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          umma_ss(tmem + (uint32_t)p * kW, umma_desc_mn(a + k * 2048), umma_desc_mn(x + k * 2048),
+                  idesc, b > b0 || k > 0);
+        umma_commit(empty(st));
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        umma_ss(tmem + 3u * kW, umma_desc_mn(a + k * 2048), umma_desc(ones), idesc1,
+                b > b0 || k > 0);
+      umma_commit(empty(sd));
+    }
+    umma_commit(done);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!s_fail && b1 > b0) {
+    // warps w and w + 4 share a lane quarter: row n of the gradient is a lane
+    const int n = (warp & 3) * 32 + lane;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64) {
+      float v[32];
+      tmem_ld32(tmem + lanes + (uint32_t)cc, v);
+      float *w = J.gw + (long)n * J.kin + cc;
+      if (n < J.nout) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if (cc + 4 * i < J.kin) red_add4(w + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      }
+    }
+    if (warp < 4) {
+      float v[32];
+      tmem_ld32(tmem + lanes + 3u * kW, v);
+      if (n < J.nout) atomicAdd(J.gb + n, v[0]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == kDwProducers) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+  if (threadIdx.x == 0 && s_fail) atomicExch(g.err, 1);
+}
+
+constexpr size_t mlp_bwd_smem(int np) {
+  return (size_t)(4 + 2 * np + kRing) * kStageBytes + (2 * kRing + 8) * sizeof(uint64_t) + 1024;
+}
+
+template <int NP> cudaError_t launch_mlp_bwd(const MlpBwdArgs &g, cudaStream_t s, int dev) {
+  static bool attr[16] = {};  // per device, once
+  if (!attr[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_mlp_bwd<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_bwd_smem(NP));
+    if (e != cudaSuccess) return e;
+    attr[dev] = true;
+  }
+  const int ntiles = (g.M + kTileM - 1) / kTileM;
+  k_mlp_bwd<NP><<<std::min(ntiles, sm_count(dev)), kMlpThreads, mlp_bwd_smem(NP), s>>>(g, ntiles);
+  return cudaGetLastError();
+}
+
+bool aligned(const void *p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
+
+}  // namespace
+}  // namespace op2b
+
+using namespace op2b;
+
+extern "C" int op2b_gnn_mlp(int M, int nparts, const op2b_mlp_part *parts, const void *const *w,
+                            const float *const *b, int nout, const void *R, long ldr, void *y,
+                            long ldy, void *z0, void *a0, void *z1, void *a1, void *stream) {
+  const char *what = "op2b_gnn_mlp";
+  if (M < 0 || nparts < 1 || nparts > 3 || !parts || !w || !b || !y) {
+    set_error("%s: bad sizes or null arguments", what);
+    return -1;
+  }
+  MlpArgs g{};
+  g.M = M;
+  g.nout = nout;
+  for (int i = 0; i < nparts; i++) {
+    const op2b_mlp_part &p = parts[i];
+    if (!p.x || !aligned(p.x, 16) || p.ld % 8 || p.cols % 8 || p.cols < 8 || p.ld < p.cols ||
+        (nparts > 1 ? p.cols != kW : p.cols > 64 && p.cols != kW) || (i == 0 && p.rows)) {
+      set_error("%s: input part %d: 128 columns (8 to 64, or 128, of a single part), 16-byte "
+                "aligned rows; the first part is direct", what, i);
+      return -1;
+    }
+    g.part[i] = MlpPart{(const __nv_bfloat16 *)p.x, p.rows, p.ld, p.cols};
+    g.k0 += p.cols;
+  }
+  if (nout != kW && (nout > 16 || nout < 8 || nout % 8)) {
+    set_error("%s: 128 BF16 outputs, or 8 or 16 FP32 outputs", what);
+    return -1;
+  }
+  for (int l = 0; l < 3; l++) {
+    if (!w[l] || !b[l] || !aligned(w[l], 16)) {
+      set_error("%s: layer %d: null or unaligned weights", what, l);
+      return -1;
+    }
+    g.W[l] = (const __nv_bfloat16 *)w[l];
+    g.b[l] = b[l];
+  }
+  const bool store = z0 != nullptr;
+  if ((a0 != nullptr) != store || (z1 != nullptr) != store || (a1 != nullptr) != store ||
+      !aligned(z0, 32) || !aligned(a0, 32) || !aligned(z1, 32) || !aligned(a1, 32)) {
+    set_error("%s: z0, a0, z1, a1: all or none, 32-byte aligned", what);
+    return -1;
+  }
+  if (nout == kW ? !aligned(y, 32) || ldy % 16 || (R && (!aligned(R, 32) || ldr % 16))
+                 : !aligned(y, 16) || ldy % 4 || R != nullptr) {
+    set_error("%s: rows of the result (and the residual) need 32-byte alignment, FP32 rows 16-byte",
+              what);
+    return -1;
+  }
+  g.Z0 = (__nv_bfloat16 *)z0, g.A0 = (__nv_bfloat16 *)a0;
+  g.Z1 = (__nv_bfloat16 *)z1, g.A1 = (__nv_bfloat16 *)a1;
+  g.R = (const __nv_bfloat16 *)R;
+  g.ldr = ldr;
+  g.Y = y;
+  g.ldy = ldy;
+  if (M == 0) return 0;
+  int dev = 0;
+  g.err = tc_error_flag(what, &dev);
+  if (!g.err) return -1;
+  const int nc = nparts == 1 ? (g.k0 <= 64 ? 1 : 2) : 2 * nparts;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = store ? launch_mlp<true>(g, nc, s, dev) : launch_mlp<false>(g, nc, s, dev);
+  if (rt().initialised) rt().launches++;
+  return cuda_ok(e, what) ? 0 : -1;
+}
+
+extern "C" int op2b_gnn_mlp_backward(int M, const void *dy, long ldy, int nout,
+                                     const void *const *w, int kin, const void *z0,
+                                     const void *z1, void *d0, void *d1, int nparts,
+                                     float *const *dx, const long *lddx, const int *add,
+                                     void *stream) {
+  const char *what = "op2b_gnn_mlp_backward";
+  if (M < 0 || !dy || !w || !z0 || !z1 || !d0 || !d1 || nparts < 0 || nparts > 3 ||
+      (nparts > 0 && (!dx || !lddx || !add))) {
+    set_error("%s: bad sizes or null arguments", what);
+    return -1;
+  }
+  if ((nout != kW && (nout < 8 || nout > 16 || nout % 8)) || ldy % 8 || ldy < nout ||
+      !aligned(dy, 16) || kin % 8 || kin < 8 || (nparts > 0 && kin != nparts * kW)) {
+    set_error("%s: 128 (or 8 or 16) output columns in 16-byte aligned rows, 128 input columns a "
+              "part", what);
+    return -1;
+  }
+  if (!aligned(z0, 32) || !aligned(z1, 32) || !aligned(d0, 32) || !aligned(d1, 32)) {
+    set_error("%s: z0, z1, d0, d1 need 32-byte alignment", what);
+    return -1;
+  }
+  MlpBwdArgs g{};
+  g.M = M;
+  g.nout = nout;
+  g.kin = kin;
+  g.nparts = nparts;
+  g.dy = (const __nv_bfloat16 *)dy;
+  g.ldy = ldy;
+  for (int l = 0; l < 3; l++) {
+    if (!w[l] || !aligned(w[l], 16)) {
+      set_error("%s: layer %d: null or unaligned weights", what, l);
+      return -1;
+    }
+    g.W[l] = (const __nv_bfloat16 *)w[l];
+  }
+  g.Z0 = (const __nv_bfloat16 *)z0, g.Z1 = (const __nv_bfloat16 *)z1;
+  g.d0 = (__nv_bfloat16 *)d0, g.d1 = (__nv_bfloat16 *)d1;
+  for (int p = 0; p < nparts; p++) {
+    if (!dx[p] || !aligned(dx[p], 32) || lddx[p] % 8 || lddx[p] < kW) {
+      set_error("%s: dx part %d: 32-byte aligned rows of at least 128 floats", what, p);
+      return -1;
+    }
+    g.dx[p] = dx[p];
+    g.lddx[p] = lddx[p];
+    g.add[p] = add[p];
+  }
+  if (M == 0) return 0;
+  int dev = 0;
+  g.err = tc_error_flag(what, &dev);
+  if (!g.err) return -1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = nparts == 0   ? launch_mlp_bwd<0>(g, s, dev)
+                        : nparts == 1 ? launch_mlp_bwd<1>(g, s, dev)
+                        : nparts == 2 ? launch_mlp_bwd<2>(g, s, dev)
+                                      : launch_mlp_bwd<3>(g, s, dev);
+  if (rt().initialised) rt().launches++;
+  return cuda_ok(e, what) ? 0 : -1;
+}
+
+extern "C" int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int nout,
+                               int nparts, const op2b_mlp_part *parts, const void *a0,
+                               const void *a1, float *const *gw, float *const *gb,
+                               void *stream) {
+  const char *what = "op2b_gnn_mlp_dw";
+  if (M < 0 || !d || !ldd || nparts < 1 || nparts > 3 || !parts || !a0 || !a1 || !gw || !gb ||
+      (nout != kW && (nout < 8 || nout > 16 || nout % 8))) {
+    set_error("%s: bad sizes or null arguments", what);
+    return -1;
+  }
+  MlpDwArgs g{};
+  g.M = M;
+  g.njobs = 3;
+  const void *act[3] = {nullptr, a0, a1};
+  for (int l = 0; l < 3; l++) {
+    MlpDwJob &J = g.job[l];
+    if (!d[l] || !gw[l] || !gb[l] || !aligned(d[l], 16) || !aligned(gw[l], 16) || ldd[l] % 8 ||
+        (l && !aligned(act[l], 16))) {
+      set_error("%s: layer %d: null or unaligned operands", what, l);
+      return -1;
+    }
+    J.d = (const __nv_bfloat16 *)d[l];
+    J.ldd = ldd[l];
+    J.nout = l == 2 ? nout : kW;
+    J.gw = gw[l];
+    J.gb = gb[l];
+    J.nparts = l ? 1 : nparts;
+    if (l) {
+      J.part[0] = MlpPart{(const __nv_bfloat16 *)act[l], nullptr, kW, kW};
+      J.kin = kW;
+      continue;
+    }
+    for (int i = 0; i < nparts; i++) {
+      const op2b_mlp_part &p = parts[i];
+      if (!p.x || !aligned(p.x, 16) || p.ld % 8 || p.cols % 8 || p.cols < 8 || p.cols > kW ||
+          p.ld < p.cols || (nparts > 1 && p.cols != kW) || (i == 0 && p.rows)) {
+        set_error("%s: input part %d: 128 columns (8 to 128 of a single part), 16-byte aligned "
+                  "rows; the first part is direct", what, i);
+        return -1;
+      }
+      J.part[i] = MlpPart{(const __nv_bfloat16 *)p.x, p.rows, p.ld, p.cols};
+      J.kin += p.cols;
+    }
+  }
+  if (M == 0) return 0;
+  int dev = 0;
+  g.err = tc_error_flag(what, &dev);
+  if (!g.err) return -1;
+  // CTAs by the tiles a job reads per 64 rows, at least four blocks of rows each
+  const int nsm = sm_count(dev), most = std::max(1, ((M + 63) / 64 + 3) / 4);
+  int total = 0, at = 0;
+  for (const MlpDwJob &J : g.job) total += 1 + J.nparts;
+  for (MlpDwJob &J : g.job) {
+    J.cta0 = at;
+    J.ctas = std::max(1, std::min(most, nsm * (1 + J.nparts) / total));
+    at += J.ctas;
+  }
+  static bool attr[16] = {};
+  if (!attr[dev]) {
+    if (!cuda_ok(cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kDwSmem), what))
+      return -1;
+    attr[dev] = true;
+  }
+  k_mlp_dw<<<at, kDwThreads, kDwSmem, static_cast<cudaStream_t>(stream)>>>(g);
+  if (rt().initialised) rt().launches++;
+  return cuda_ok(cudaGetLastError(), what) ? 0 : -1;
+}

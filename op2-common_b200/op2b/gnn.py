@@ -47,6 +47,10 @@ _GNN_SIGS = {
     "op2b_gemm_bf16": (_I, [_I, _I, _I, _P, _L, _L, _P, _L, _L, _P, _L, _I, _P, _P, _P, _L, _I,
                             _I, _P]),
     "op2b_gemm_error": (_I, [_I]),
+    "op2b_gnn_mlp": (_I, [_I, _I, _P, _P, _P, _I, _P, _L, _P, _L, _P, _P, _P, _P, _P]),
+    "op2b_gnn_mlp_backward": (_I, [_I, _P, _L, _I, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _P]),
+    "op2b_gnn_mlp_dw": (_I, [_I, _P, _P, _I, _I, _P, _P, _P, _P, _P, _P]),
+    "op2b_gnn_node_grad": (_I, [_I, _I, _P, _L, _P, _P, _P, _P, _P]),
     "op2b_gnn_gather_pair": (_I, [_I, _I, _P, _P, _P, _L, _P, _L, _I, _P]),
     "op2b_gnn_aggregate": (_I, [_I, _I, _P, _P, _P, _L, _P, _L, _P]),
     "op2b_gnn_to_bf16": (_I, [_I, _I, _P, _L, _P, _L, _P]),
@@ -59,6 +63,10 @@ _GNN_SIGS = {
     "op2b_gnn_memset": (_I, [_P, _I, _L, _P]),
     "op2b_gnn_decode_q": (_I, [_I, _P, _L, _P, _P, _P, _P]),
 }
+
+
+class op2b_mlp_part(ctypes.Structure):
+    _fields_ = [("x", _P), ("rows", _P), ("ld", _L), ("cols", _I)]
 
 
 def _lib():
@@ -204,8 +212,8 @@ def edge_features(mesh: Mesh, g=None):
 
 
 # ---------------------------------------------------------------- the network
-# products with k-contiguous operands (the forward MLP layers) run on the
-# TMA-fed tensor-core kernel; False keeps the register-staged one everywhere
+# one kernel a MLP, forward and backward (op2b_gnn_mlp, ...); False: layer by layer
+# on the register-staged product everywhere
 GEMM_TMA = True
 
 
@@ -248,12 +256,9 @@ class GraphNet:
 
     def _gemm(self, M, N, K, A, a_m, a_k, B, b_n, b_k, C, ldc, epi, bias=None, Z=None, R=None,
               ldr=0, split=1):
-        # every product goes to the TMA-fed persistent kernel (engine 2: k-
-        # contiguous operands as K-major tiles, the others as MN-major tiles)
-        # unless gemm_tma is off (engine 0, operands staged through registers)
-        engine = 2 if self.gemm_tma else 0
+        # layer by layer (gemm_tma off): operands staged through registers
         _call("op2b_gemm_bf16", M, N, K, A, a_m, a_k, B, b_n, b_k, C, ldc, epi, bias, Z, R, ldr,
-              split, engine, self.stream)
+              split, 0, self.stream)
         self.launches += 1
 
     def _split_for(self, rows, ntiles):
@@ -262,7 +267,7 @@ class GraphNet:
         return s
 
     def workspace(self, N, E, train):
-        key = (N, E, train)
+        key = (N, E, train, self.gemm_tma)
         if key in self._ws:
             return self._ws[key]
         torch = self.torch
@@ -271,6 +276,28 @@ class GraphNet:
         z = lambda *shape, dt=bf: torch.zeros(*shape, dtype=dt, device="cuda")
         nb = S + 1 if train else 1
         ws = dict(N=N, E=E, train=train)
+        if self.gemm_tma:
+            # one kernel a MLP: the node and edge states and the aggregates, in
+            # training those of every step and the hidden layers
+            keep = S if train else 0
+            ws["h"] = [z(N, w) for _ in range(keep + 1)]
+            ws["e"] = [z(E, w) for _ in range(keep + 1)]
+            ws["agg"] = [z(N, w) for _ in range(max(keep, 1))]
+            ws["out"] = z(N, OUT, dt=f32)
+            if train:
+                ws["act"] = {}
+                for name, _layers in self.lay:
+                    rows = E if name.startswith("edge") or name == "enc_edge" else N
+                    ws["act"][name] = [z(rows, w) for _ in range(4)]
+                R = max(N, E)
+                ws["dOut"] = z(N, OUT)
+                ws["dH"], ws["dE"] = z(N, w, dt=f32), z(E, w, dt=f32)
+                ws["dAgg"], ws["dX"] = z(N, w, dt=f32), z(E, 2 * w, dt=f32)
+                ws["dyN"], ws["dyE"] = z(N, w), z(E, w)
+                ws["d0"], ws["d1"] = z(R, w), z(R, w)
+                ws["loss"] = z(1, dt=f32)
+            self._ws[key] = ws
+            return ws
         ws["node_in"] = z(N, NODE_IN)
         ws["edge_in"] = z(E, EDGE_IN)
         ws["CE"] = [z(E, 3 * w) for _ in range(S if train else 1)]
@@ -320,6 +347,93 @@ class GraphNet:
         self._gemm(M, nout, kin, A1.data_ptr(), w, 1, Wp, kin, 1, out, ldo, last, bias=bp,
                    R=resid, ldr=ldr)
 
+    def _mlp(self, name, M, parts, y, ldy, resid=None, ldr=0, keep=(None,) * 4):
+        """One MLP in one kernel; parts: (pointer, rows pointer or None, leading
+        dimension, columns) of its input's column blocks."""
+        arr = (op2b_mlp_part * len(parts))(*parts)
+        layers = [self._w(name, i) for i in range(3)]
+        W = (_P * 3)(*[l[0] for l in layers])
+        b = (_P * 3)(*[l[1] for l in layers])
+        _call("op2b_gnn_mlp", M, len(parts), arr, W, b, layers[2][5], resid, ldr, y, ldy, *keep,
+              self.stream)
+        self.launches += 1
+
+    def _mlp_grad(self, name, M, dy, ldy, parts, dx, ws):
+        """Backward of one MLP in two kernels: dx: (pointer, leading dimension,
+        1 to add to it / 0 to store) per 128-column block of its input; the
+        weight and bias gradients are added to self.g."""
+        z0, a0, z1, a1 = (t.data_ptr() for t in ws["act"][name])
+        d0, d1 = ws["d0"].data_ptr(), ws["d1"].data_ptr()
+        layers = [self._w(name, i) for i in range(3)]
+        W = (_P * 3)(*[l[0] for l in layers])
+        n, nout = len(dx), layers[2][5]
+        _call("op2b_gnn_mlp_backward", M, dy, ldy, nout, W, layers[0][4], z0, z1, d0, d1, n,
+              (_P * 3)(*[d[0] for d in dx]), (_L * 3)(*[d[1] for d in dx]),
+              (_I * 3)(*[d[2] for d in dx]), self.stream)
+        _call("op2b_gnn_mlp_dw", M, (_P * 3)(d0, d1, dy), (_L * 3)(WIDTH, WIDTH, ldy), nout,
+              len(parts), (op2b_mlp_part * len(parts))(*parts), a0, a1,
+              (_P * 3)(*[l[2] for l in layers]), (_P * 3)(*[l[3] for l in layers]), self.stream)
+        self.launches += 2
+
+    def _parts(self, dg, ws, l):
+        """The input blocks of step l's edge and node MLPs."""
+        w, k = WIDTH, l if ws["train"] else 0
+        h, e, agg = ws["h"][k].data_ptr(), ws["e"][k].data_ptr(), ws["agg"][k].data_ptr()
+        src, dst = dg["src"].data_ptr(), dg["dst"].data_ptr()
+        return ([(e, None, w, w), (h, src, w, w), (h, dst, w, w)],
+                [(h, None, w, w), (agg, None, w, w)])
+
+    def _forward_fused(self, dg, ni, ei, ws):
+        """The forward pass with one kernel a MLP.  Without a backward pass to
+        come the states are updated in place: a row tile is read before it is
+        written, and no other tile reads its direct rows."""
+        N, E = dg["N"], dg["E"]
+        w, st, train = WIDTH, self.stream, ws["train"]
+        off, idx = dg["off"].data_ptr(), dg["idx"].data_ptr()
+        kept = lambda name: tuple(t.data_ptr() for t in ws["act"][name]) if train else (None,) * 4
+        ptr = lambda k, l: ws[k][l if train else 0].data_ptr()
+        self._mlp("enc_node", N, [(ni.data_ptr(), None, NODE_IN, NODE_IN)], ptr("h", 0), w,
+                  keep=kept("enc_node"))
+        self._mlp("enc_edge", E, [(ei.data_ptr(), None, EDGE_IN, EDGE_IN)], ptr("e", 0), w,
+                  keep=kept("enc_edge"))
+        for l in range(self.steps):
+            pe, pn = self._parts(dg, ws, l)
+            e1 = ptr("e", l + 1)
+            self._mlp(f"edge{l}", E, pe, e1, w, resid=pe[0][0], ldr=w, keep=kept(f"edge{l}"))
+            _call("op2b_gnn_aggregate", N, w, off, idx, e1, w, pn[1][0], w, st)
+            self._mlp(f"node{l}", N, pn, ptr("h", l + 1), w, resid=pn[0][0], ldr=w,
+                      keep=kept(f"node{l}"))
+            self.launches += 1
+        self._mlp("dec", N, [(ptr("h", self.steps), None, w, w)], ws["out"].data_ptr(), OUT,
+                  keep=kept("dec"))
+        return ws["out"]
+
+    def _backward_fused(self, dg, ws, dO):
+        N, E = dg["N"], dg["E"]
+        w, st = WIDTH, self.stream
+        dH, dE, dAgg, dX, dyN, dyE = (ws[k].data_ptr() for k in ("dH", "dE", "dAgg", "dX", "dyN",
+                                                                 "dyE"))
+        dst, off, idx, rev = (dg[k].data_ptr() for k in ("dst", "off", "idx", "rev"))
+        self._mlp_grad("dec", N, dO, OUT, [(ws["h"][self.steps].data_ptr(), None, w, w)],
+                       [(dH, w, 0)], ws)
+        _call("op2b_gnn_memset", dE, 0, ws["dE"].numel() * 4, st)
+        for l in reversed(range(self.steps)):
+            pe, pn = self._parts(dg, ws, l)
+            _call("op2b_gnn_to_bf16", N, w, dH, w, dyN, w, st)
+            self._mlp_grad(f"node{l}", N, dyN, w, pn, [(dH, w, 1), (dAgg, w, 0)], ws)
+            _call("op2b_gnn_edge_grad", E, w, dst, dE, dAgg, w, dyE, st)
+            self._mlp_grad(f"edge{l}", E, dyE, w, pe,
+                           [(dE, w, 1), (dX, 2 * w, 0), (dX + 4 * w, 2 * w, 0)], ws)
+            _call("op2b_gnn_node_grad", N, w, dX, 2 * w, off, idx, rev, dH, st)
+            self.launches += 3
+        _call("op2b_gnn_to_bf16", N, w, dH, w, dyN, w, st)
+        self._mlp_grad("enc_node", N, dyN, w, [(ws["_node_in"].data_ptr(), None, NODE_IN,
+                                                NODE_IN)], [], ws)
+        _call("op2b_gnn_to_bf16", E, w, dE, w, dyE, w, st)
+        self._mlp_grad("enc_edge", E, dyE, w, [(ws["_edge_in"].data_ptr(), None, EDGE_IN,
+                                                EDGE_IN)], [], ws)
+        self.launches += 2
+
     def upload_graph(self, g):
         t = self.torch
         dev = lambda a: t.from_numpy(np.ascontiguousarray(a, np.int32)).to("cuda")
@@ -336,6 +450,8 @@ class GraphNet:
         ni = node_in if node_in.dtype == torch.bfloat16 else node_in.to(torch.bfloat16)
         ei = edge_in if edge_in.dtype == torch.bfloat16 else edge_in.to(torch.bfloat16)
         ws["_node_in"], ws["_edge_in"] = ni, ei
+        if "h" in ws:
+            return self._forward_fused(dg, ni, ei, ws)
         CN0 = ws["CN"][0]
         CE0 = ws["CE"][0]
         self._mlp_fwd("enc_node", N, ni.data_ptr(), NODE_IN, CN0.data_ptr(), 2 * w, ws=ws)
@@ -396,6 +512,9 @@ class GraphNet:
     def backward(self, dg, ws, dOut=None):
         """Backpropagate the gradient in ws['dOut'] (bf16, N x 8) through the
         network of the last forward(train=True); accumulates into self.g."""
+        if "h" in ws:
+            self._backward_fused(dg, ws, ws["dOut"].data_ptr() if dOut is None else dOut)
+            return
         N, E = dg["N"], dg["E"]
         w, S, st = WIDTH, self.steps, self.stream
         dH, dE, dCat = ws["dH"], ws["dE"], ws["dCat"]

@@ -344,8 +344,8 @@ def main(argv=None):
                     help="under torchrun (WORLD_SIZE > 1) training is data parallel; the "
                          "gradient all-reduce's backend (gloo: ranks may share a GPU)")
     ap.add_argument("--gemm-tma", type=int, default=1,
-                    help="1: forward products on the TMA-fed tensor-core GEMM; 0: all on the "
-                         "register-staged one")
+                    help="1: one tensor-core kernel a MLP; 0: layer by layer on the "
+                         "register-staged product")
     a = ap.parse_args(argv)
     G.GEMM_TMA = bool(a.gemm_tma)
     log = lambda s: print(s, flush=True)

@@ -934,18 +934,34 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
         for (int s = handed; s < upto; s++) mbar_arrive(full(s % kDwRing));
       handed = upto;
     };
+    // the four operands' first chunk, row stride in bytes and whether the
+    // thread's chunk lies inside the columns, in registers for the whole loop
+    const char *x[4];
+    long ld[4];
+    bool incol[4];
+    const int *idx[2];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const MlpPart &X = J.part[t > 0 ? t - 1 : 0];
+      x[t] = reinterpret_cast<const char *>(t ? X.p : J.d);
+      ld[t] = 2 * (t ? X.ld : J.ldd);
+      incol[t] = t <= P && c * 8 < (t ? X.cols : J.nout);
+      if (t >= 2) idx[t - 2] = X.rows;
+    }
+    const int M = g.M;
     int rows[2][8];
-    auto load_rows = [&](int p, int b) {
-      const int *idx = J.part[p].rows;
+    auto load_rows = [&](int q, int b) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const int r = b * 64 + r0 + 8 * i;
-        rows[p - 1][i] = idx && r < g.M ? __ldg(idx + r) : r;
+        rows[q][i] = idx[q] && r < M ? __ldg(idx[q] + r) : r;
       }
     };
-    if (P > 1 && b0 < b1) load_rows(1, b0);
-    if (P > 2 && b0 < b1) load_rows(2, b0);
+    if (P > 1 && b0 < b1) load_rows(0, b0);
+    if (P > 2 && b0 < b1) load_rows(1, b0);
     for (int b = b0; b < b1 && ok; b++) {
+      const int m0 = b * 64 + r0;
+      const bool whole = b * 64 + 64 <= M;
 #pragma unroll
       for (int t = 0; t < 4; t++) {  // d, then X's blocks
         if (t > P) break;
@@ -964,19 +980,23 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
             }
           }
         }
-        const __nv_bfloat16 *x = t == 0 ? J.d : J.part[t > 0 ? t - 1 : 0].p;
-        const long ld = t == 0 ? J.ldd : J.part[t > 0 ? t - 1 : 0].ld;
-        const bool incol = c * 8 < (t == 0 ? J.nout : J.part[t > 0 ? t - 1 : 0].cols);
         const uint32_t dst = place + (uint32_t)st * kStageBytes;
-        const int m0 = b * 64 + r0;
+        const char *src = x[t] + c * 16;
+        if (whole && incol[t]) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const bool in = incol && m0 + 8 * i < g.M;
-          const long r = t >= 2 ? rows[t >= 2 ? t - 2 : 0][i] : m0 + 8 * i;
-          cp_async16(dst + i * 1024, in ? x + r * ld + c * 8 : x, in);
+          for (int i = 0; i < 8; i++)
+            cp_async16(dst + i * 1024, src + (t >= 2 ? rows[t >= 2 ? t - 2 : 0][i] : m0 + 8 * i) * ld[t]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const bool in = incol[t] && m0 + 8 * i < M;
+            cp_async16(dst + i * 1024,
+                       in ? src + (t >= 2 ? rows[t >= 2 ? t - 2 : 0][i] : m0 + 8 * i) * ld[t] : x[t],
+                       in);
+          }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (t >= 2 && b + 1 < b1) load_rows(t - 1, b + 1);
+        if (t >= 2 && b + 1 < b1) load_rows(t - 2, b + 1);
         it++;
         if (it - handed > kDwLag) {
           asm volatile("cp.async.wait_group %0;" ::"n"(kDwLag) : "memory");

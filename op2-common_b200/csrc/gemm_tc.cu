@@ -957,6 +957,19 @@ cudaError_t launch_ws(const GemmArgs &g, const CUtensorMap &ta, const CUtensorMa
 
 }  // namespace
 
+bool tc_store_map(CUtensorMap *m, void *base, bool f32, int cols, int rows, long ld) {
+  EncodeTiled enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint32_t esize = f32 ? 4 : 2;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * esize};
+  const cuuint32_t box[2] = {64 / esize, 32};
+  const cuuint32_t estr[2] = {1, 1};
+  return enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base,
+             dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int *tc_error_flag(const char *what, int *device) {
   int dev = 0;
   cudaGetDevice(&dev);

@@ -537,7 +537,10 @@ template <bool STORE> cudaError_t launch_mlp(const MlpArgs &g, int nc, cudaStrea
 // dZ1 and dZ0 go from one product to the next through tensor memory and are
 // also stored, as k_mlp_dw needs them.  dx leaves as FP32 column blocks of 128,
 // each stored or added to what is there, so the sums that follow (dE, dH)
-// need no pass of their own.  The products' and roundings' order is that of the
+// need no pass of their own.  The results leave by TMA from 2 KiB a warp of
+// shared memory (stores, and reductions for what is added): a lane's own row
+// segments cost a shared-memory/L1 cycle a row and instruction, and the stores'
+// bursts were what the kernel waited for.  The products' and roundings' order is that of the
 // layer-by-layer products.
 struct MlpBwdArgs {
   int M, nout, kin, nparts;
@@ -545,12 +548,13 @@ struct MlpBwdArgs {
   long ldy;
   const __nv_bfloat16 *W[3];
   const __nv_bfloat16 *Z0, *Z1;
-  __nv_bfloat16 *d0, *d1;  // dZ0, dZ1 (rows of 128)
-  float *dx[3];
-  long lddx[3];
-  int add[3];  // 1: dx += , 0: dx =
+  CUtensorMap md[2];   // dZ0, dZ1 (rows of 128)
+  CUtensorMap mdx[3];  // dx
+  int add[3];          // 1: dx += , 0: dx =
   int *err;
 };
+constexpr int kBwdRing = 2;            // stages of dy
+constexpr int kOutBytes = 32 * 64;     // a warp's staged box: 64 bytes of 32 rows
 
 // rows [0, nrows) of a weight matrix [nrows][ld], columns col0 .. col0 + 127, as
 // MN-major tiles: for every 64 rows two boxes of 64 columns x 64 rows
@@ -572,22 +576,23 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *s_w2 = smem, *s_w1 = s_w2 + 2 * kStageBytes, *s_w0 = s_w1 + 2 * kStageBytes;
   uint8_t *s_ring = s_w0 + 2 * NP * kStageBytes;
-  // full[kRing], empty[kRing], acc_full[2], h_full[2], d_free[2], done
-  uint64_t *bars = reinterpret_cast<uint64_t *>(s_ring + kRing * kStageBytes);
-  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 7);
+  uint8_t *s_out = s_ring + kBwdRing * kStageBytes;
+  // full[kBwdRing], empty[kBwdRing], acc_full[2], h_full[2], d_free[2], done
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_out + kEpiWarps * kOutBytes);
+  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kBwdRing + 7);
   int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int s) { return smem_u32(&bars[s]); };
-  auto empty = [&](int s) { return smem_u32(&bars[kRing + s]); };
-  auto acc_full = [&](int s) { return smem_u32(&bars[2 * kRing + s]); };
-  auto h_full = [&](int s) { return smem_u32(&bars[2 * kRing + 2 + s]); };
-  auto d_free = [&](int s) { return smem_u32(&bars[2 * kRing + 4 + s]); };
-  const uint32_t done = smem_u32(&bars[2 * kRing + 6]);
+  auto empty = [&](int s) { return smem_u32(&bars[kBwdRing + s]); };
+  auto acc_full = [&](int s) { return smem_u32(&bars[2 * kBwdRing + s]); };
+  auto h_full = [&](int s) { return smem_u32(&bars[2 * kBwdRing + 2 + s]); };
+  auto d_free = [&](int s) { return smem_u32(&bars[2 * kBwdRing + 4 + s]); };
+  const uint32_t done = smem_u32(&bars[2 * kBwdRing + 6]);
   volatile int *fail = &s_fail;
   const int nkb = g.nout > 64 ? 2 : 1;  // 64-column blocks of dy
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kRing; s++) {
+    for (int s = 0; s < kBwdRing; s++) {
       mbar_init(full(s), kProducerWarps);
       mbar_init(empty(s), 1);
     }
@@ -632,15 +637,15 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0)
-        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kRing));
+        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kBwdRing));
       handed = upto;
     };
     for (int j = 0; j < nloc && ok; j++) {
       const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + r0;
       for (int c = 0; c < nkb; c++, it++) {
-        const int st = it % kRing;
-        if (it >= kRing) {
-          const uint32_t par = (uint32_t)((it / kRing - 1) & 1);
+        const int st = it % kBwdRing;
+        if (it >= kBwdRing) {
+          const uint32_t par = (uint32_t)((it / kBwdRing - 1) & 1);
           if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
             if (handed < it) {
               asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -661,9 +666,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
           cp_async16(dst + i * 1024, in ? g.dy + (long)(m0 + 8 * i) * g.ldy + col : g.dy, in);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (it + 1 - handed > kLag) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
-          hand_on(it + 1 - kLag);
+        if (it + 1 - handed > 1) {
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          hand_on(it);
         }
       }
     }
@@ -687,8 +692,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
             if (jf != jn[s]) continue;  // dy's stages arrive in tile order
             // the accumulator has been read (the NP or one read of the tile before)
             if (cf == 0 && jf >= 2 && !mbar_test(d_free(s), (uint32_t)((nd[s] - 1) & 1))) continue;
-            const int st = it % kRing;
-            if (!mbar_test(full(st), (uint32_t)((it / kRing) & 1))) continue;
+            const int st = it % kBwdRing;
+            if (!mbar_test(full(st), (uint32_t)((it / kBwdRing) & 1))) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(s_ring + (size_t)st * kStageBytes);
             const uint32_t b = w2 + (uint32_t)cf * kStageBytes;
@@ -747,6 +752,33 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
     const uint32_t acc = acc_of(s) + lanes + (uint32_t)c0;
     const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
+    uint8_t *out = s_out + (warp - kEpiWarp0) * kOutBytes;
+    // 64 bytes of each lane's row to column x of the rows from y on
+    auto put = [&](const CUtensorMap *m, int x, int y, const uint32_t *v, bool add) {
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+            make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0 && y < g.M) {  // rows past M are clipped
+        if (add)
+          asm volatile(
+              "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group "
+              "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+              "r"(x), "r"(y), "r"(smem_u32(out))
+              : "memory");
+        else
+          asm volatile(
+              "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group "
+              "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+              "r"(x), "r"(y), "r"(smem_u32(out))
+              : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+    };
     bool ok = true;
     int na = 0;
     auto wait_acc = [&]() {
@@ -764,10 +796,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
     for (int j = s; j < nloc && ok; j += 2) {
       const long row = (long)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + quarter * 32 + lane;
       const bool live = row < g.M;
+      const int y = (int)row - lane;
 #pragma unroll 1
       for (int l = 1; l >= 0; l--) {  // dZ1, then dZ0
         const __nv_bfloat16 *Z = (l ? g.Z1 : g.Z0) + row * kW + c0;
-        __nv_bfloat16 *d = (l ? g.d1 : g.d0) + row * kW + c0;
         uint32_t z[4][8];
         if (live) {
 #pragma unroll
@@ -778,10 +810,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
         for (int k = 0; k < 2; k++) {
           float v[32];
           tmem_ld32(acc + k * 32, v);
+          uint32_t p[16];
 #pragma unroll
           for (int m = 0; m < 2; m++) {
             float *u = v + 16 * m;
-            uint32_t p[8];
             if (live) {
 #pragma unroll
               for (int i = 0; i < 8; i++) {
@@ -791,10 +823,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
                 u[2 * i + 1] *= silu_grad(t.y);
               }
             }
-            pack16(u, p);
-            if (live) st_sector(d + k * 32 + m * 16, p);
-            if (NP > 0 || l == 1) tmem_st8(hid + k * 16 + m * 8, p);
+            pack16(u, p + 8 * m);
+            if (NP > 0 || l == 1) tmem_st8(hid + k * 16 + m * 8, p + 8 * m);
           }
+          put(&g.md[l], c0 + k * 32, y, p, false);
         }
         if (NP > 0 || l == 1) {
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -806,30 +838,20 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
       if (!ok) break;
 #pragma unroll 1
       for (int p = 0; p < NP; p++) {
-        float *dx = g.dx[p] + row * g.lddx[p] + c0;
         if (!wait_acc()) break;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
           float v[32];
-          uint32_t o[4][8];
-          if (g.add[p] && live) {
-#pragma unroll
-            for (int m = 0; m < 4; m++) ld_sector(dx + k * 32 + m * 8, o[m]);
-          }
           tmem_ld32(acc + k * 32, v);
           if (k == 1) signal(d_free(s));
-          if (live) {
-            if (g.add[p]) {
 #pragma unroll
-              for (int i = 0; i < 32; i++) v[i] = __uint_as_float(o[i >> 3][i & 7]) + v[i];
-            }
-#pragma unroll
-            for (int m = 0; m < 4; m++)
-              st_sector(dx + k * 32 + m * 8, reinterpret_cast<const uint32_t *>(v + m * 8));
-          }
+          for (int m = 0; m < 2; m++)
+            put(&g.mdx[p], c0 + k * 32 + m * 16, y, reinterpret_cast<const uint32_t *>(v + 16 * m),
+                g.add[p] != 0);
         }
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
@@ -1077,7 +1099,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
 }
 
 constexpr size_t mlp_bwd_smem(int np) {
-  return (size_t)(4 + 2 * np + kRing) * kStageBytes + (2 * kRing + 8) * sizeof(uint64_t) + 1024;
+  return (size_t)(4 + 2 * np + kBwdRing) * kStageBytes + kEpiWarps * kOutBytes +
+         (2 * kBwdRing + 8) * sizeof(uint64_t) + 1024;
 }
 
 template <int NP> cudaError_t launch_mlp_bwd(const MlpBwdArgs &g, cudaStream_t s, int dev) {
@@ -1199,20 +1222,24 @@ extern "C" int op2b_gnn_mlp_backward(int M, const void *dy, long ldy, int nout,
     g.W[l] = (const __nv_bfloat16 *)w[l];
   }
   g.Z0 = (const __nv_bfloat16 *)z0, g.Z1 = (const __nv_bfloat16 *)z1;
-  g.d0 = (__nv_bfloat16 *)d0, g.d1 = (__nv_bfloat16 *)d1;
   for (int p = 0; p < nparts; p++) {
     if (!dx[p] || !aligned(dx[p], 32) || lddx[p] % 8 || lddx[p] < kW) {
       set_error("%s: dx part %d: 32-byte aligned rows of at least 128 floats", what, p);
       return -1;
     }
-    g.dx[p] = dx[p];
-    g.lddx[p] = lddx[p];
     g.add[p] = add[p];
   }
   if (M == 0) return 0;
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
+  bool mapped = tc_store_map(&g.md[0], d0, false, kW, M, kW) &&
+                tc_store_map(&g.md[1], d1, false, kW, M, kW);
+  for (int p = 0; p < nparts; p++) mapped = mapped && tc_store_map(&g.mdx[p], dx[p], true, kW, M, lddx[p]);
+  if (!mapped) {
+    set_error("%s: the results cannot be described as tensor maps", what);
+    return -1;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = nparts == 0   ? launch_mlp_bwd<0>(g, s, dev)
                         : nparts == 1 ? launch_mlp_bwd<1>(g, s, dev)

@@ -957,6 +957,10 @@ cudaError_t launch_ws(const GemmArgs &g, const CUtensorMap &ta, const CUtensorMa
 
 }  // namespace
 
+bool tc_operand_map(CUtensorMap *m, const void *base, int rows, int K, long ld) {
+  return operand_map(m, base, rows, K, ld);
+}
+
 bool tc_store_map(CUtensorMap *m, void *base, bool f32, int cols, int rows, long ld) {
   EncodeTiled enc = encode_tiled();
   if (!enc) return false;

@@ -5,10 +5,10 @@
 // be gathered into a 384-wide array first; here
 //   * the three weight matrices stay in shared memory (K-major, 128-byte
 //     swizzle) for the whole kernel: 160 KiB for the edge MLP (K = 384);
-//   * warps 0-1 load the 128-row input tile in 64-column blocks by cp.async
-//     into a ring of four 16 KiB stages, each row from its own address: a
-//     direct row, or the row of h an index names, so no gathered copy exists;
-//   * warp 2 issues the MMAs: layer 0 of a tile runs two tiles ahead, layers 1
+//   * warps 0-2 load the 128-row input tile in 64-column blocks into a ring of
+//     16 KiB stages: direct rows by TMA, rows of h that an index names by
+//     cp.async, each from its own address, so no gathered copy exists;
+//   * warp 3 issues the MMAs: layer 0 of a tile runs two tiles ahead, layers 1
 //     and 2 as their operands appear, so the tensor core and the activations
 //     of two tiles overlap;
 //   * warps 4-19 are the epilogues, eight for even and eight for odd tiles (two
@@ -37,11 +37,8 @@ namespace op2b {
 namespace {
 
 constexpr int kW = 128;                 // hidden width
-constexpr int kRing = 4;                // input stages of 128 rows x 64 columns
-constexpr int kLag = 2;                 // cp.async groups left in flight before a stage is handed on
-constexpr int kProducerWarps = 2, kRowReps = kTileM / (4 * kProducerWarps);
-constexpr int kMmaWarp = 2, kEpiWarp0 = 4, kEpiWarps = 16;
-// 20 warps (one idle): five a scheduler, whose 16K registers allow 96 a thread
+constexpr int kProducerWarps = 3, kMmaWarp = 3, kEpiWarp0 = 4, kEpiWarps = 16;
+// 20 warps: five a scheduler, whose 16K registers allow 96 a thread
 constexpr int kMlpThreads = 32 * (kEpiWarp0 + kEpiWarps);
 
 struct MlpPart {
@@ -56,7 +53,8 @@ struct MlpArgs {
   MlpPart part[3];
   const __nv_bfloat16 *W[3];
   const float *b[3];
-  __nv_bfloat16 *Z0, *A0, *Z1, *A1;  // training: pre-activations and activations (rows of 128)
+  CUtensorMap mx[3];                 // the parts without rows
+  CUtensorMap mz[2], ma[2], my;      // training: Z0, Z1, A0, A1 (rows of 128) and Y
   const __nv_bfloat16 *R;            // residual added to the result, or null
   long ldr;
   void *Y;
@@ -153,6 +151,38 @@ __device__ __forceinline__ void ld_sector(const void *p, uint32_t *r) {
                : "memory");
 }
 
+// A warp's 32 rows x 64 bytes out to global memory by TMA: 16 words of each
+// lane's row, to column x (in elements of the map) of the rows from y on.  `out`:
+// the warp's 2 KiB of shared memory, in the 64-byte swizzle; rows past the
+// matrix are clipped.  `add`: an FP32 reduction instead of a store.
+constexpr int kOutBytes = 32 * 64;
+__device__ __forceinline__ void put_rows(uint8_t *out, int lane, const CUtensorMap *m, int x, int y,
+                                         bool inside, const uint32_t *v, bool add) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    *reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+        make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0 && inside) {
+    if (add)
+      asm volatile(
+          "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group "
+          "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+          "r"(x), "r"(y), "r"(smem_u32(out))
+          : "memory");
+    else
+      asm volatile(
+          "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group "
+          "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+          "r"(x), "r"(y), "r"(smem_u32(out))
+          : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+
 // 16 floats to 16 BF16 (element 2i in the low half of word i)
 __device__ __forceinline__ void pack16(const float *v, uint32_t *r) {
 #pragma unroll
@@ -182,15 +212,23 @@ __device__ __forceinline__ void load_weights(uint32_t dst, const __nv_bfloat16 *
   }
 }
 
+// Input stages of 128 rows x 64 columns.  With the hidden layers kept, two of
+// the four give way to the epilogue warps' 2 KiB each, from which Z, A and y leave
+// by TMA (a lane's own row segments would cost an L1 cycle a row and
+// instruction); without, only y is written, and the deeper ring is worth more.
+__host__ __device__ constexpr int mlp_ring(bool store) { return store ? 2 : 4; }
+
 // NC: 64-column blocks of the input (1, 2, 4 or 6); STORE: keep Z0, A0, Z1, A1
 template <int NC, bool STORE>
 __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constant__ MlpArgs g,
                                                             int ntiles) {
+  constexpr int kRing = mlp_ring(STORE);
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *s_w0 = smem, *s_w1 = s_w0 + NC * kStageBytes, *s_w2 = s_w1 + 2 * kStageBytes;
   uint8_t *s_ring = s_w2 + 2 * kStageBytes;
-  float *s_bias = reinterpret_cast<float *>(s_ring + kRing * kStageBytes);  // 3 x 128
+  uint8_t *s_out = s_ring + kRing * kStageBytes;  // STORE: kOutBytes a warp
+  float *s_bias = reinterpret_cast<float *>(s_out + (STORE ? kEpiWarps * kOutBytes : 0));  // 3 x 128
   // full[kRing], empty[kRing], first_full[2], acc_full[2], h_full[2], d_free[3], done
   uint64_t *bars = reinterpret_cast<uint64_t *>(s_bias + 3 * kW);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 10);
@@ -207,7 +245,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kRing; s++) {
-      mbar_init(full(s), kProducerWarps);
+      mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
     }
     for (int s = 0; s < 2; s++) {
@@ -248,81 +286,70 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
   const auto hid_of = [&](int s) { return tmem + 3u * kW + (uint32_t)(s * 64); };
 
   if (warp < kProducerWarps) {
-    // a stage is 1024 chunks of 16 bytes: thread t copies chunk t % 8 of the
-    // rows t / 8 + 8 i, eight lanes a row, so its place in the swizzled tile
-    // moves by 1024 bytes with i
-    const int kc = threadIdx.x & 7, r0 = threadIdx.x >> 3;
-    const uint32_t place = smem_u32(s_ring) + sw128(r0, kc);
-    int it = 0, handed = 0;  // stages issued, stages handed to the MMAs
-    bool ok = true;
-    auto hand_on = [&](int upto) {  // the copies of stages [handed, upto) have landed
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0)
-        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kRing));
-      handed = upto;
-    };
-    int rows[2][kRowReps];  // the indexed parts' rows; loaded a tile ahead
-    auto load_rows = [&](int p, int j) {
-      const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + r0;
-      const int *idx = g.part[p + 1].rows;
+    // stage n is one warp's (n % kTurns): the warps' latencies overlap, and each
+    // waits only for its own copies.  No more warps than stages: the wait for a
+    // stage's last use then follows, in the same warp, one that implies the use before.  Direct rows (zeros outside the rows and columns)
+    // come by TMA; of indexed ones lane l copies chunk l % 8 of rows
+    // l / 8 + 4 i, eight lanes a row, each lane holding four rows' indices.
+    const int kc = lane & 7, r0 = lane >> 3;
+    const uint32_t place0 = sw128(r0, kc), place1 = sw128(r0 + 4, kc);  // even, odd i
+    constexpr int kTurns = kProducerWarps < kRing ? kProducerWarps : kRing;
+    const int total = warp < kTurns ? nloc * NC : 0;
+    int n = warp, j = warp / NC, c = warp % NC;  // stage, local tile, block
+    int idx[4] = {0, 0, 0, 0}, next[4] = {0, 0, 0, 0};
+    auto load_rows = [&](int jn, int cn, int *to) {
+      const int *rows = NC == 1 ? nullptr : g.part[cn >> 1].rows;
+      if (!rows) return;
+      const int m = (int)(blockIdx.x + (unsigned)jn * gridDim.x) * kTileM + lane;
 #pragma unroll
-      for (int i = 0; i < kRowReps; i++) {
-        const int r = m0 + 8 * i;
-        rows[p][i] = idx && r < g.M ? __ldg(idx + r) : r;
-      }
+      for (int i = 0; i < 4; i++) to[i] = m + 32 * i < g.M ? __ldg(rows + m + 32 * i) : 0;
     };
-    if (NC > 2 && nloc > 0) load_rows(0, 0);
-    if (NC > 4 && nloc > 0) load_rows(1, 0);
-    for (int j = 0; j < nloc && ok; j++) {
+    if (n < total) load_rows(j, c, idx);
+    int tma = -1;  // the last stage this warp loaded by TMA
+    for (; n < total; n += kTurns) {
+      const int st = n % kRing;
+      const int jn = c + kTurns >= NC ? j + (c + kTurns) / NC : j;
+      const int cn = (c + kTurns) % NC;
+      if (n + kTurns < total) load_rows(jn, cn, next);
+      if (n >= kRing &&
+          !__all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), (uint32_t)((n / kRing - 1) & 1),
+                                                     fail))) {
+        if (lane == 0) atomicExch(&s_fail, 1);
+        break;
+      }
       const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM;
-      const bool whole = m0 + kTileM <= g.M;
-#pragma unroll
-      for (int c = 0; c < NC; c++, it++) {
-        const int st = it % kRing;
-        if (it >= kRing) {
-          const uint32_t par = (uint32_t)((it / kRing - 1) & 1);
-          if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
-            if (handed < it) {  // nothing to overlap with: hand on what is in flight
-              asm volatile("cp.async.wait_group 0;" ::: "memory");
-              hand_on(it);
-            }
-            ok = __all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), par, fail));
-            if (!ok) {
-              if (lane == 0) atomicExch(&s_fail, 1);
-              break;
-            }
-          }
+      const MlpPart &P = g.part[NC == 1 ? 0 : c >> 1];
+      const int cb = NC == 1 ? 0 : (c & 1) * 64;
+      const uint32_t dst = smem_u32(s_ring + (size_t)st * kStageBytes);
+      if (!P.rows) {
+        if (lane == 0) {
+          mbar_expect_tx(full(st), kStageBytes);
+          tma_load_2d(dst, &g.mx[NC == 1 ? 0 : c >> 1], cb, m0, full(st));
         }
-        const int part = NC == 1 ? 0 : c / 2, col = (NC == 1 ? 0 : (c & 1) * 64) + kc * 8;
-        const MlpPart &P = g.part[part];
-        const __nv_bfloat16 *base = P.p + col;
-        const uint32_t dst = place + (uint32_t)st * kStageBytes;
-        const bool incol = NC > 1 || col < P.cols;
-        if (whole && incol) {
+        tma = n;
+      } else {
+        const char *base = reinterpret_cast<const char *>(P.p + cb + kc * 8);
+        const long ld = 2 * P.ld;
+        const bool whole = m0 + kTileM <= g.M;
 #pragma unroll
-          for (int i = 0; i < kRowReps; i++)
-            cp_async16(dst + i * 1024,
-                       base + (part > 0 ? rows[part > 0 ? part - 1 : 0][i] : m0 + r0 + 8 * i) * P.ld);
-        } else {
-#pragma unroll
-          for (int i = 0; i < kRowReps; i++) {
-            const bool in = incol && m0 + r0 + 8 * i < g.M;
-            cp_async16(dst + i * 1024,
-                       in ? base + (part > 0 ? rows[part > 0 ? part - 1 : 0][i] : m0 + r0 + 8 * i) * P.ld
-                          : P.p, in);
-          }
+        for (int i = 0; i < 32; i++) {
+          const int r = __shfl_sync(0xffffffffu, idx[i >> 3], (4 * i & 31) + r0);
+          const uint32_t to = dst + (i & 1 ? place1 : place0) + (i >> 1) * 1024;
+          if (whole) cp_async16(to, base + r * ld);
+          else cp_async16(to, base + r * ld, m0 + 4 * i + r0 < g.M);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (part > 0 && (c & 1) && j + 1 < nloc) load_rows(part - 1, j + 1);
-        if (it + 1 - handed > kLag) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(kLag) : "memory");
-          hand_on(it + 1 - kLag);
-        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full(st));
       }
+#pragma unroll
+      for (int i = 0; i < 4; i++) idx[i] = next[i];
+      j = jn;
+      c = cn;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    hand_on(it);
+    // after a failure, a load that nobody waits for any more
+    if (lane == 0 && *fail && tma >= 0) mbar_wait(full(tma % kRing), (uint32_t)((tma / kRing) & 1));
   } else if (warp == kMmaWarp) {
     if (lane == 0) {  // MMA issuer: whatever has its operands next
       const uint32_t idesc = umma_idesc(kW), idesc2 = umma_idesc((g.nout + 15) & ~15);
@@ -390,6 +417,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
     const int c0 = (((warp - kEpiWarp0) >> 2) & 1) * 64;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
     const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
+    uint8_t *out = s_out + (warp - kEpiWarp0) * kOutBytes;
     bool ok = true;
     auto wait_for = [&](uint32_t bar, int n) {  // the n-th completion (from 0) of bar
       ok = __all_sync(0xffffffffu, mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail));
@@ -406,30 +434,31 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
       const long row = (long)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + quarter * 32 + lane;
       const bool live = row < g.M;
       const uint32_t acc = acc_of(j) + lanes + (uint32_t)c0;
+      const int y0 = (int)row - lane;
 #pragma unroll 1
       for (int l = 0; l < 2; l++) {
         if (!(l == 0 ? wait_for(first_full(s), jj) : wait_for(acc_full(s), 2 * jj))) break;
-        __nv_bfloat16 *Z = l == 0 ? g.Z0 : g.Z1, *A = l == 0 ? g.A0 : g.A1;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
           float v[32];
           tmem_ld32(acc + k * 32, v);
+          uint32_t p[16];
 #pragma unroll
           for (int m = 0; m < 2; m++) {
             float *u = v + 16 * m;
-            const int c = c0 + k * 32 + m * 16;
-            uint32_t p[8];
-            add_smem16(u, s_bias + l * kW + c);
-            if (STORE) {
-              pack16(u, p);
-              if (live) st_sector(Z + row * kW + c, p);
-            }
+            add_smem16(u, s_bias + l * kW + c0 + k * 32 + m * 16);
+            if (STORE) pack16(u, p + 8 * m);
+          }
+          if (STORE) put_rows(out, lane, &g.mz[l], c0 + k * 32, y0, y0 < g.M, p, false);
+#pragma unroll
+          for (int m = 0; m < 2; m++) {
+            float *u = v + 16 * m;
 #pragma unroll
             for (int i = 0; i < 16; i++) u[i] = silu(u[i]);
-            pack16(u, p);
-            if (STORE && live) st_sector(A + row * kW + c, p);
-            tmem_st8(hid + k * 16 + m * 8, p);
+            pack16(u, p + 8 * m);
+            tmem_st8(hid + k * 16 + m * 8, p + 8 * m);
           }
+          if (STORE) put_rows(out, lane, &g.ma[l], c0 + k * 32, y0, y0 < g.M, p, false);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         signal(h_full(s));
@@ -448,10 +477,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
           float v[32];
           tmem_ld32(acc + k * 32, v);
           if (k == 1) signal(d_free(j % 3));  // the accumulator has been read
+          uint32_t p[16];
 #pragma unroll
           for (int m = 0; m < 2; m++) {
             float *u = v + 16 * m;
-            uint32_t p[8];
             add_smem16(u, s_bias + 2 * kW + c0 + k * 32 + m * 16);
             if (g.R && live) {
 #pragma unroll
@@ -462,9 +491,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
                 u[2 * i + 1] += t.y;
               }
             }
-            pack16(u, p);
-            if (live) st_sector(y + k * 32 + m * 16, p);
+            pack16(u, p + 8 * m);
+            if (!STORE && live) st_sector(y + k * 32 + m * 16, p + 8 * m);
           }
+          if (STORE) put_rows(out, lane, &g.my, c0 + k * 32, y0, y0 < g.M, p, false);
         }
       } else {  // the decoder: nout <= 16 FP32 columns
         if (!wait_for(acc_full(s), 2 * jj + 1)) break;
@@ -481,6 +511,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
         }
       }
     }
+    if (STORE && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   // every issued MMA has finished once "done" has arrived
@@ -500,9 +531,9 @@ int sm_count(int dev) {
   return nsm > 0 ? nsm : 148;
 }
 
-constexpr size_t mlp_smem(int nc) {
-  return (size_t)(nc + 4 + kRing) * kStageBytes + 3 * kW * sizeof(float) +
-         (2 * kRing + 11) * sizeof(uint64_t) + 1024;
+constexpr size_t mlp_smem(int nc, bool store) {
+  return (size_t)(nc + 4 + mlp_ring(store)) * kStageBytes + (store ? kEpiWarps * kOutBytes : 0) +
+         3 * kW * sizeof(float) + (2 * mlp_ring(store) + 11) * sizeof(uint64_t) + 1024;
 }
 
 template <int NC, bool STORE>
@@ -510,12 +541,12 @@ cudaError_t launch_mlp(const MlpArgs &g, cudaStream_t s, int dev) {
   static bool attr[16] = {};  // per device, once
   if (!attr[dev]) {
     const cudaError_t e = cudaFuncSetAttribute(
-        k_mlp_fwd<NC, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem(NC));
+        k_mlp_fwd<NC, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem(NC, STORE));
     if (e != cudaSuccess) return e;
     attr[dev] = true;
   }
   const int ntiles = (g.M + kTileM - 1) / kTileM;
-  k_mlp_fwd<NC, STORE><<<std::min(ntiles, sm_count(dev)), kMlpThreads, mlp_smem(NC), s>>>(g,
+  k_mlp_fwd<NC, STORE><<<std::min(ntiles, sm_count(dev)), kMlpThreads, mlp_smem(NC, STORE), s>>>(g,
                                                                                          ntiles);
   return cudaGetLastError();
 }
@@ -544,8 +575,7 @@ template <bool STORE> cudaError_t launch_mlp(const MlpArgs &g, int nc, cudaStrea
 // layer-by-layer products.
 struct MlpBwdArgs {
   int M, nout, kin, nparts;
-  const __nv_bfloat16 *dy;
-  long ldy;
+  CUtensorMap mdy;
   const __nv_bfloat16 *W[3];
   const __nv_bfloat16 *Z0, *Z1;
   CUtensorMap md[2];   // dZ0, dZ1 (rows of 128)
@@ -554,7 +584,6 @@ struct MlpBwdArgs {
   int *err;
 };
 constexpr int kBwdRing = 2;            // stages of dy
-constexpr int kOutBytes = 32 * 64;     // a warp's staged box: 64 bytes of 32 rows
 
 // rows [0, nrows) of a weight matrix [nrows][ld], columns col0 .. col0 + 127, as
 // MN-major tiles: for every 64 rows two boxes of 64 columns x 64 rows
@@ -593,7 +622,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kBwdRing; s++) {
-      mbar_init(full(s), kProducerWarps);
+      mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
     }
     for (int s = 0; s < 2; s++) {
@@ -629,51 +658,25 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
   const auto hid_of = [&](int s) { return tmem + 3u * kW + (uint32_t)(s * 64); };
 
   if (warp < kProducerWarps) {
-    const int kc = threadIdx.x & 7, r0 = threadIdx.x >> 3;
-    const uint32_t place = smem_u32(s_ring) + sw128(r0, kc);
-    int it = 0, handed = 0;
-    bool ok = true;
-    auto hand_on = [&](int upto) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0)
-        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kBwdRing));
-      handed = upto;
-    };
-    for (int j = 0; j < nloc && ok; j++) {
-      const int m0 = (int)(blockIdx.x + (unsigned)j * gridDim.x) * kTileM + r0;
-      for (int c = 0; c < nkb; c++, it++) {
-        const int st = it % kBwdRing;
-        if (it >= kBwdRing) {
-          const uint32_t par = (uint32_t)((it / kBwdRing - 1) & 1);
-          if (!__all_sync(0xffffffffu, mbar_try(empty(st), par))) {
-            if (handed < it) {
-              asm volatile("cp.async.wait_group 0;" ::: "memory");
-              hand_on(it);
-            }
-            ok = __all_sync(0xffffffffu, mbar_wait_or_fail(empty(st), par, fail));
-            if (!ok) {
-              if (lane == 0) atomicExch(&s_fail, 1);
-              break;
-            }
-          }
+    if (threadIdx.x == 0) {  // dy's blocks, zeros outside its rows and columns
+      const int total = nloc * nkb;
+      int n = 0;
+      for (; n < total; n++) {
+        const int st = n % kBwdRing;
+        if (n >= kBwdRing &&
+            !mbar_wait_or_fail(empty(st), (uint32_t)((n / kBwdRing - 1) & 1), fail)) {
+          atomicExch(&s_fail, 1);
+          break;
         }
-        const int col = c * 64 + kc * 8;
-        const uint32_t dst = place + (uint32_t)st * kStageBytes;
-#pragma unroll
-        for (int i = 0; i < kRowReps; i++) {
-          const bool in = col < g.nout && m0 + 8 * i < g.M;
-          cp_async16(dst + i * 1024, in ? g.dy + (long)(m0 + 8 * i) * g.ldy + col : g.dy, in);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (it + 1 - handed > 1) {
-          asm volatile("cp.async.wait_group 1;" ::: "memory");
-          hand_on(it);
-        }
+        const int m0 = (int)(blockIdx.x + (unsigned)(n / nkb) * gridDim.x) * kTileM;
+        mbar_expect_tx(full(st), kStageBytes);
+        tma_load_2d(smem_u32(s_ring + (size_t)st * kStageBytes), &g.mdy, n % nkb * 64, m0,
+                    full(st));
       }
+      if (*fail)  // the loads that nobody waits for any more
+        for (int i = max(0, n - kBwdRing); i < n; i++)
+          mbar_wait(full(i % kBwdRing), (uint32_t)((i / kBwdRing) & 1));
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    hand_on(it);
   } else if (warp == kMmaWarp) {
     if (lane == 0) {
       const uint32_t idesc = umma_idesc(kW) | 1u << 16;  // B MN-major
@@ -753,31 +756,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
     const uint32_t acc = acc_of(s) + lanes + (uint32_t)c0;
     const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
     uint8_t *out = s_out + (warp - kEpiWarp0) * kOutBytes;
-    // 64 bytes of each lane's row to column x of the rows from y on
     auto put = [&](const CUtensorMap *m, int x, int y, const uint32_t *v, bool add) {
-      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        *reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
-            make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0 && y < g.M) {  // rows past M are clipped
-        if (add)
-          asm volatile(
-              "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group "
-              "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
-              "r"(x), "r"(y), "r"(smem_u32(out))
-              : "memory");
-        else
-          asm volatile(
-              "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group "
-              "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
-              "r"(x), "r"(y), "r"(smem_u32(out))
-              : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      }
+      put_rows(out, lane, m, x, y, y < g.M, v, add);
     };
     bool ok = true;
     int na = 0;
@@ -1169,8 +1149,6 @@ extern "C" int op2b_gnn_mlp(int M, int nparts, const op2b_mlp_part *parts, const
               what);
     return -1;
   }
-  g.Z0 = (__nv_bfloat16 *)z0, g.A0 = (__nv_bfloat16 *)a0;
-  g.Z1 = (__nv_bfloat16 *)z1, g.A1 = (__nv_bfloat16 *)a1;
   g.R = (const __nv_bfloat16 *)R;
   g.ldr = ldr;
   g.Y = y;
@@ -1179,6 +1157,20 @@ extern "C" int op2b_gnn_mlp(int M, int nparts, const op2b_mlp_part *parts, const
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
+  for (int i = 0; i < nparts; i++)
+    if (!parts[i].rows &&
+        !tc_operand_map(&g.mx[i], parts[i].x, M, parts[i].cols, parts[i].ld)) {
+      set_error("%s: input part %d cannot be described as a tensor map", what, i);
+      return -1;
+    }
+  if (store && !(tc_store_map(&g.mz[0], z0, false, kW, M, kW) &&
+                 tc_store_map(&g.mz[1], z1, false, kW, M, kW) &&
+                 tc_store_map(&g.ma[0], a0, false, kW, M, kW) &&
+                 tc_store_map(&g.ma[1], a1, false, kW, M, kW) &&
+                 (nout != kW || tc_store_map(&g.my, y, false, kW, M, ldy)))) {
+    set_error("%s: the results cannot be described as tensor maps", what);
+    return -1;
+  }
   const int nc = nparts == 1 ? (g.k0 <= 64 ? 1 : 2) : 2 * nparts;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = store ? launch_mlp<true>(g, nc, s, dev) : launch_mlp<false>(g, nc, s, dev);
@@ -1212,8 +1204,6 @@ extern "C" int op2b_gnn_mlp_backward(int M, const void *dy, long ldy, int nout,
   g.nout = nout;
   g.kin = kin;
   g.nparts = nparts;
-  g.dy = (const __nv_bfloat16 *)dy;
-  g.ldy = ldy;
   for (int l = 0; l < 3; l++) {
     if (!w[l] || !aligned(w[l], 16)) {
       set_error("%s: layer %d: null or unaligned weights", what, l);
@@ -1233,11 +1223,11 @@ extern "C" int op2b_gnn_mlp_backward(int M, const void *dy, long ldy, int nout,
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
-  bool mapped = tc_store_map(&g.md[0], d0, false, kW, M, kW) &&
+  bool mapped = tc_operand_map(&g.mdy, dy, M, nout, ldy) && tc_store_map(&g.md[0], d0, false, kW, M, kW) &&
                 tc_store_map(&g.md[1], d1, false, kW, M, kW);
   for (int p = 0; p < nparts; p++) mapped = mapped && tc_store_map(&g.mdx[p], dx[p], true, kW, M, lddx[p]);
   if (!mapped) {
-    set_error("%s: the results cannot be described as tensor maps", what);
+    set_error("%s: dy or the results cannot be described as tensor maps", what);
     return -1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -79,7 +79,11 @@ static std::vector<std::unique_ptr<InvMapCache>> &inv_cache() {
   return v;
 }
 
+static long g_generation = 0;
+long gather_generation() { return g_generation; }
+
 void release_inverse_maps() {
+  g_generation++;
   release_slot_records();
   inv_cache().clear();
 }

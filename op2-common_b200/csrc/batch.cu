@@ -13,9 +13,16 @@
 //    rms < tol * rms0.  rms0 is an instance's rms after its first iteration.
 //  * A single-CTA convergence kernel ends each iteration: per-instance rms,
 //    phase changes, and the rebuilt work lists; it publishes the number of
-//    active instances to mapped host memory.  The whole iteration (promote,
-//    save_soln, 2 x {adt_calc, res_calc, bres_calc, update} for both
-//    precisions, convergence) is captured once in a CUDA graph and replayed.
+//    active instances to mapped host memory.  The whole iteration
+//    (promotion, 2 x {res_calc + bres_calc, update} for both precisions,
+//    convergence) is captured once in a CUDA graph and replayed, the two
+//    precisions' stages on two branches (the one without instances then costs
+//    no time).
+//  * As in the runtime's own Airfoil loops, adt_calc is computed by the update
+//    before it (into a second array for the next iteration's first, so the adt
+//    dat keeps the last one), save_soln by the first update (which reads q
+//    itself and stores it to qold), and bres_calc by res_calc's kernel over
+//    the linked corner records: per step two kernels instead of five.
 //  * The res_calc strategy and the block size are chosen by a project-written
 //    autotuner (op2b_batch_tune) that times each candidate on the batch.
 #include <cuda_runtime.h>
@@ -30,6 +37,7 @@
 
 #include "airfoil_math.cuh"
 #include "batch.h"
+#include "corner.cuh"
 #include "gather.h"
 #include "op2b_batch.h"
 #include "op2b_runtime.h"
@@ -45,18 +53,6 @@ constexpr int kMinChunk = 256;  // smallest partition size (elements per work it
 #define FOR_ITEMS(list, count)                                   \
   const int nitems = *(count);                                   \
   for (int w = blockIdx.x; w < nitems; w += gridDim.x)
-
-template <typename T>
-__global__ void k_b_save(const WorkItem *items, const int *count, const T *q, T *qold) {
-  FOR_ITEMS(items, count) {
-    WorkItem it = items[w];
-    for (int c = it.begin + threadIdx.x; c < it.end; c += blockDim.x) {
-      T v[4];
-      Vec<T>::ld4(q + 4 * (size_t)c, v);
-      Vec<T>::st4(qold + 4 * (size_t)c, v);
-    }
-  }
-}
 
 template <typename T>
 __global__ void k_b_adt(const WorkItem *items, const int *count, const int4 *pcell, const T *x,
@@ -115,6 +111,28 @@ __global__ void k_b_res_gather(const WorkItem *items, const int *count, const in
         }
       }
       Vec<T>::st4(res + 4 * (size_t)c, acc);
+    }
+  }
+}
+
+// owner-computes res_calc and bres_calc in one pass over the cell items (corner
+// records with the boundary edges linked in, corner.cuh), each instance's
+// freestream at its far-field edges: both loops' increments in their order
+template <typename T>
+__global__ void k_b_pair(const WorkItem *items, const int *count, const int4 *rec_o,
+                         const int4 *rec_cn, const unsigned *rec_meta, const int *bound,
+                         const T *x, const T *q, const T *adt, T *res, const double *qinf,
+                         int ncell, AirConst<T> k) {
+  FOR_ITEMS(items, count) {
+    const WorkItem it = items[w];
+    AirConst<T> kk = k;
+#pragma unroll
+    for (int m = 0; m < 4; m++) kk.qinf[m] = (T)__ldg(qinf + 4 * it.inst + m);
+    for (int c = it.begin + threadIdx.x; c < it.end; c += blockDim.x) {
+      CornerOps<T> d;
+      const CornerRec r = load_crec(rec_o, rec_cn, rec_meta, c, ncell);
+      load_corner_cell<T, true>(d, c, r, x, q, adt, res, BresLink{bound});
+      compute_corner<T, true>(d, c, res, kk);
     }
   }
 }
@@ -217,19 +235,29 @@ __global__ void k_b_bres(const WorkItem *items, const int *count, InvMap inv,
   }
 }
 
-// update (q = qold - res/adt in FP64, res = 0) and the instance's sum of del^2
-template <typename T>
-__global__ void k_b_update(const WorkItem *items, const int *count, const T *qold, T *q, T *res,
-                           const T *adt, double *rms_sum) {
+// update (q = qold - res/adt in FP64, res = 0), the adt_calc of the new q, and
+// the instance's sum of del^2 (rms_sum: of an iteration's second update).  FIRST:
+// the iteration's first update, whose qold is q itself: it is stored to qold
+// (save_soln) on the way.
+template <typename T, bool FIRST>
+__global__ void k_b_update(const WorkItem *items, const int *count, T *qold, T *q, T *res,
+                           const T *adt, double *rms_sum, const int4 *pcell, const T *x,
+                           T *adt_next, AirConst<T> k) {
   __shared__ double s_part[32];
   FOR_ITEMS(items, count) {
     WorkItem it = items[w];
     double sum = 0.0;
     for (int c = it.begin + threadIdx.x; c < it.end; c += blockDim.x) {
-      T qo[4], r[4], qn[4];
-      Vec<T>::ld4(qold + 4 * (size_t)c, qo);
+      T qo[4], r[4], qn[4], a[8];
+      const int4 p = __ldg(pcell + c);
+      Vec<T>::ld2(x + 2 * (size_t)p.x, a[0], a[1]);
+      Vec<T>::ld2(x + 2 * (size_t)p.y, a[2], a[3]);
+      Vec<T>::ld2(x + 2 * (size_t)p.z, a[4], a[5]);
+      Vec<T>::ld2(x + 2 * (size_t)p.w, a[6], a[7]);
+      Vec<T>::ld4_rw((FIRST ? q : qold) + 4 * (size_t)c, qo);
       Vec<T>::ld4_rw(res + 4 * (size_t)c, r);
       double adti = 1.0f / (double)__ldg(adt + c);
+      if (FIRST) Vec<T>::st4(qold + 4 * (size_t)c, qo);
 #pragma unroll
       for (int m = 0; m < 4; m++) {
         double del = adti * (double)r[m];
@@ -239,71 +267,105 @@ __global__ void k_b_update(const WorkItem *items, const int *count, const T *qol
       Vec<T>::st4(q + 4 * (size_t)c, qn);
       T z[4] = {(T)0, (T)0, (T)0, (T)0};
       Vec<T>::st4(res + 4 * (size_t)c, z);
+      adt_next[c] = air_adt<T>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], qn[0], qn[1],
+                               qn[2], qn[3], k);
     }
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0 && rms_sum) {  // only the second update of an iteration counts
-      double t = 0.0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += s_part[i];
-      atomicAdd(rms_sum + it.inst, t);
+    if (rms_sum) {  // only the second update of an iteration counts
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+      if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += s_part[i];
+        atomicAdd(rms_sum + it.inst, t);
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
-// FP32 -> FP64 storage for instances entering the FP64 phase
+// FP32 -> FP64 storage for instances entering the FP64 phase, and the adt_calc
+// of the promoted q that their first FP64 step reads
 __global__ void k_b_promote(const WorkItem *items, const int *count, const float *q32,
-                            double *q64) {
+                            double *q64, const int4 *pcell, const double *x, double *adt,
+                            AirConst<double> k) {
   FOR_ITEMS(items, count) {
     WorkItem it = items[w];
-    for (int c = it.begin + threadIdx.x; c < it.end; c += blockDim.x)
-      for (int m = 0; m < 4; m++) q64[4 * (size_t)c + m] = (double)q32[4 * (size_t)c + m];
+    for (int c = it.begin + threadIdx.x; c < it.end; c += blockDim.x) {
+      const int4 p = __ldg(pcell + c);
+      double q[4], a[8];
+#pragma unroll
+      for (int m = 0; m < 4; m++) q[m] = (double)q32[4 * (size_t)c + m];
+      Vec<double>::st4(q64 + 4 * (size_t)c, q);
+      Vec<double>::ld2(x + 2 * (size_t)p.x, a[0], a[1]);
+      Vec<double>::ld2(x + 2 * (size_t)p.y, a[2], a[3]);
+      Vec<double>::ld2(x + 2 * (size_t)p.z, a[4], a[5]);
+      Vec<double>::ld2(x + 2 * (size_t)p.w, a[6], a[7]);
+      adt[c] = air_adt<double>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], q[0], q[1], q[2],
+                               q[3], k);
+    }
   }
 }
 
 // ------------------------------------------------------------------ convergence + lists
 
-__device__ void build_list(const BatchDev &b, const int *off, int ninst, const int *sel,
-                           WorkItem *out, int *count, int *s_scan) {
-  // sel[i] != 0: instance i belongs to this list; items of b.chunk elements
-  int i = threadIdx.x;
-  int n = 0;
-  if (i < ninst && sel[i]) n = (off[i + 1] - off[i] + b.chunk - 1) / b.chunk;
-  s_scan[i] = n;
+// the items of the instances with sel[i] != 0 (off: their element ranges), `chunk`
+// elements each: a scan of the instances' item counts, then every thread writes
+// items of the whole list (a thread an instance would leave a large one's
+// items to one thread)
+__device__ void build_list(const BatchDev &b, const int *off, const int *sel, WorkItem *out,
+                           int *count, int *s_scan, int *s_warp) {
+  const int i = threadIdx.x, lane = i & 31;
+  const int n = i < b.ninst && sel[i] ? (off[i + 1] - off[i] + b.chunk - 1) / b.chunk : 0;
+  int inc = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) s_warp[i >> 5] = inc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int j = 0; j < ninst; j++) {
-      int t = s_scan[j];
-      s_scan[j] = acc;
-      acc += t;
+  if (i < 32) {
+    int t = s_warp[i];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, t, o);
+      if (i >= o) t += u;
     }
-    *count = acc;
+    s_warp[i] = t;
   }
   __syncthreads();
-  if (i < ninst && sel[i]) {
-    int base = s_scan[i];
-    for (int k = 0; k < n; k++) {
-      int beg = off[i] + k * b.chunk;
-      out[base + k] = WorkItem{i, beg, min(beg + b.chunk, off[i + 1]), 0};
+  s_scan[i] = inc - n + (i >= 32 ? s_warp[(i >> 5) - 1] : 0);
+  const int total = s_warp[31];
+  if (i == 0) *count = total;
+  __syncthreads();
+  for (int w = i; w < total; w += 1024) {
+    int lo = 0, hi = b.ninst - 1;  // the last instance whose items start at or before w
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (s_scan[mid] <= w) lo = mid;
+      else hi = mid - 1;
     }
+    const int beg = off[lo] + (w - s_scan[lo]) * b.chunk;
+    out[w] = WorkItem{lo, beg, min(beg + b.chunk, off[lo + 1]), 0};
   }
   __syncthreads();
 }
 
+// One CTA of 1024 threads.  The lists depend on the phases and the item size
+// alone: they are rebuilt when one of them changed.
 __global__ void k_b_converge(BatchDev b, int init) {
-  __shared__ int s_sel32[1024], s_sel64[1024], s_selp[1024], s_scan[1024];
-  __shared__ int s_active, s_iter;
+  __shared__ int s_sel32[1024], s_sel64[1024], s_selp[1024], s_scan[1024], s_warp[32];
+  __shared__ int s_active, s_iter, s_changed;
   int i = threadIdx.x;
   if (i == 0) {
     s_active = 0;
     s_iter = 0;
+    s_changed = init || *b.built != b.chunk;
   }
   __syncthreads();
   if (i < b.ninst) {
     int p = b.phase[i];
     if (!init) {
+      const int before = p;
       if (p == 3) p = 1;  // promoted during the iteration just finished
       if (p == 0 || p == 1) {
         int it = ++b.iters[i];
@@ -330,24 +392,26 @@ __global__ void k_b_converge(BatchDev b, int init) {
         }
       }
       b.phase[i] = p;
+      if (p != before) s_changed = 1;
       atomicMax(&s_iter, b.iters[i]);
     }
     s_sel32[i] = p == 0;
     s_sel64[i] = p == 1 || p == 3;
     s_selp[i] = p == 3;
     if (p != 2) atomicAdd(&s_active, 1);
-  } else if (i < 1024) {
-    s_sel32[i] = s_sel64[i] = s_selp[i] = 0;
   }
   __syncthreads();
-  build_list(b, b.cell_off, b.ninst, s_sel32, b.w32.cells, b.w32.count + 0, s_scan);
-  build_list(b, b.brow_off, b.ninst, s_sel32, b.w32.brows, b.w32.count + 1, s_scan);
-  build_list(b, b.edge_off, b.ninst, s_sel32, b.w32.edges, b.w32.count + 2, s_scan);
-  build_list(b, b.cell_off, b.ninst, s_sel64, b.w64.cells, b.w64.count + 0, s_scan);
-  build_list(b, b.brow_off, b.ninst, s_sel64, b.w64.brows, b.w64.count + 1, s_scan);
-  build_list(b, b.edge_off, b.ninst, s_sel64, b.w64.edges, b.w64.count + 2, s_scan);
-  build_list(b, b.cell_off, b.ninst, s_selp, b.promote, b.npromote, s_scan);
+  if (s_changed) {
+    build_list(b, b.cell_off, s_sel32, b.w32.cells, b.w32.count + 0, s_scan, s_warp);
+    build_list(b, b.brow_off, s_sel32, b.w32.brows, b.w32.count + 1, s_scan, s_warp);
+    build_list(b, b.edge_off, s_sel32, b.w32.edges, b.w32.count + 2, s_scan, s_warp);
+    build_list(b, b.cell_off, s_sel64, b.w64.cells, b.w64.count + 0, s_scan, s_warp);
+    build_list(b, b.brow_off, s_sel64, b.w64.brows, b.w64.count + 1, s_scan, s_warp);
+    build_list(b, b.edge_off, s_sel64, b.w64.edges, b.w64.count + 2, s_scan, s_warp);
+    build_list(b, b.cell_off, s_selp, b.promote, b.npromote, s_scan, s_warp);
+  }
   if (threadIdx.x == 0) {
+    *b.built = b.chunk;
     volatile int *m = b.mapped;
     m[1] = s_iter;
     __threadfence_system();
@@ -366,6 +430,7 @@ struct PrecisionDats {
   const int *pcell = nullptr, *pedge = nullptr, *pecell = nullptr, *pbedge = nullptr,
             *bound = nullptr;
   void *x = nullptr, *q = nullptr, *qold = nullptr, *adt = nullptr, *res = nullptr;
+  void *adt0 = nullptr;  // the batch's own: adt of the coming iteration's first step
 };
 
 struct op2b_batch_s {
@@ -373,10 +438,15 @@ struct op2b_batch_s {
   std::vector<void *> owned;
   PrecisionDats p32, p64;
   const SlotRecords *slots = nullptr;
-  const InvMap *inv_cells = nullptr, *inv_bound = nullptr;
+  const InvMap *inv_bound = nullptr;
+  bool linked = false;   // the boundary edges are in the corner records (k_b_pair)
+  long generation = -1;  // of the records (gather_generation)
   op2b_airfoil_dats h32{}, h64{};
   int ninst = 0, ncells = 0;
-  int block = 256, blocks_per_sm = 4;
+  int block = 256, blocks_per_sm = 0;  // 0: by the number of items
+  int part_size = 0;                   // elements per item; 0: by the number of cells
+  cudaStream_t side = nullptr;         // the FP64 branch of the captured iteration
+  cudaEvent_t fork = nullptr, join = nullptr;
   int res_kernel = OP2B_BATCH_RES_GATHER;
   // OP2B_BATCH_RES_COLOUR: the edges grouped by colour (device) and each
   // colour's first element (host, ncolours + 1 entries), from a parallel
@@ -404,56 +474,147 @@ template <typename T> static AirConst<T> consts_or(bool &ok) {
   return k;
 }
 
+// A launch's CTAs: one an item of a full list up to 16 an SM, whose scheduler
+// then evens out the items (a list shrinks as instances converge; a CTA
+// without an item ends at once), or the caller's blocks_per_sm.
+static int item_grid(const op2b_batch_s *b, long long elements) {
+  const long long items = elements / b->dev.chunk + b->ninst;
+  const long long cap = (long long)rt().nsm * (b->blocks_per_sm > 0 ? b->blocks_per_sm : 16);
+  return (int)std::max(1LL, std::min(items, cap));
+}
+
 template <typename T>
 static void enqueue_stage(op2b_batch_s *b, const PrecisionDats &d, const WorkLists &w,
-                          cudaStream_t s, bool second_half_only) {
-  (void)second_half_only;
+                          cudaStream_t s) {
   bool ok;
   AirConst<T> k = consts_or<T>(ok);
-  int grid = rt().nsm * b->blocks_per_sm, th = b->block;
+  const int th = b->block, gc = item_grid(b, b->ncells);
   const T *x = (const T *)d.x;
-  T *q = (T *)d.q, *qold = (T *)d.qold, *adt = (T *)d.adt, *res = (T *)d.res;
-  k_b_save<T><<<grid, th, 0, s>>>(w.cells, w.count, q, qold);
+  T *q = (T *)d.q, *qold = (T *)d.qold, *adt = (T *)d.adt, *res = (T *)d.res, *adt0 = (T *)d.adt0;
+  const int4 *pcell = reinterpret_cast<const int4 *>(d.pcell);
   for (int step = 0; step < 2; step++) {
-    k_b_adt<T><<<grid, th, 0, s>>>(w.cells, w.count, reinterpret_cast<const int4 *>(d.pcell), x,
-                                   q, adt, k);
-    if (b->res_kernel == OP2B_BATCH_RES_ATOMIC)
-      k_b_res_atomic<T><<<grid, th, 0, s>>>(w.edges, w.count + 2,
-                                            reinterpret_cast<const int2 *>(d.pedge),
-                                            reinterpret_cast<const int2 *>(d.pecell), x, q, adt,
-                                            res, k);
-    else if (b->res_kernel == OP2B_BATCH_RES_COLOUR)
-      for (size_t c = 0; c + 1 < b->colour_off.size(); c++) {
-        const int n = b->colour_off[c + 1] - b->colour_off[c];
-        if (n <= 0) continue;
-        k_b_res_colour<T><<<std::min(grid, (n + th - 1) / th), th, 0, s>>>(
-            b->colour_elems + b->colour_off[c], n, b->dev.edge_off, b->ninst, b->dev.phase,
-            sizeof(T) == 8, reinterpret_cast<const int2 *>(d.pedge),
-            reinterpret_cast<const int2 *>(d.pecell), x, q, adt, res, k);
-      }
-    else
-      k_b_res_gather<T><<<grid, th, 0, s>>>(w.cells, w.count,
+    const T *a = step == 0 ? adt0 : adt;  // this step's adt_calc
+    if (b->res_kernel == OP2B_BATCH_RES_GATHER && b->linked) {
+      k_b_pair<T><<<gc, th, 0, s>>>(w.cells, w.count, reinterpret_cast<const int4 *>(b->slots->o),
+                                    reinterpret_cast<const int4 *>(b->slots->cn), b->slots->meta,
+                                    d.bound, x, q, a, res, b->dev.qinf, b->ncells, k);
+    } else {
+      if (b->res_kernel == OP2B_BATCH_RES_ATOMIC)
+        k_b_res_atomic<T><<<item_grid(b, b->h64.pecell->from->size), th, 0, s>>>(
+            w.edges, w.count + 2, reinterpret_cast<const int2 *>(d.pedge),
+            reinterpret_cast<const int2 *>(d.pecell), x, q, a, res, k);
+      else if (b->res_kernel == OP2B_BATCH_RES_COLOUR)
+        for (size_t c = 0; c + 1 < b->colour_off.size(); c++) {
+          const int n = b->colour_off[c + 1] - b->colour_off[c];
+          if (n <= 0) continue;
+          k_b_res_colour<T><<<std::min(rt().nsm * 16, (n + th - 1) / th), th, 0, s>>>(
+              b->colour_elems + b->colour_off[c], n, b->dev.edge_off, b->ninst, b->dev.phase,
+              sizeof(T) == 8, reinterpret_cast<const int2 *>(d.pedge),
+              reinterpret_cast<const int2 *>(d.pecell), x, q, a, res, k);
+        }
+      else
+        k_b_res_gather<T><<<gc, th, 0, s>>>(w.cells, w.count,
                                             reinterpret_cast<const int4 *>(b->slots->o),
                                             reinterpret_cast<const int4 *>(b->slots->n1),
                                             reinterpret_cast<const uint4 *>(b->slots->n2), x, q,
-                                            adt, res, k);
-    k_b_bres<T><<<grid, th, 0, s>>>(w.brows, w.count + 1, *b->inv_bound,
-                                    reinterpret_cast<const int2 *>(d.pbedge), d.bound, x, q, adt,
-                                    res, b->dev.qinf, k);
+                                            a, res, k);
+      k_b_bres<T><<<item_grid(b, b->inv_bound->nrows), th, 0, s>>>(
+          w.brows, w.count + 1, *b->inv_bound, reinterpret_cast<const int2 *>(d.pbedge), d.bound,
+          x, q, a, res, b->dev.qinf, k);
+    }
     // rms is that of the second update (airfoil.cpp:265, :281)
-    k_b_update<T><<<grid, th, 0, s>>>(w.cells, w.count, qold, q, res, adt,
-                                      step == 1 ? b->dev.rms_sum : nullptr);
+    if (step == 0)
+      k_b_update<T, true><<<gc, th, 0, s>>>(w.cells, w.count, qold, q, res, a, nullptr, pcell, x,
+                                            adt, k);
+    else
+      k_b_update<T, false><<<gc, th, 0, s>>>(w.cells, w.count, qold, q, res, a, b->dev.rms_sum,
+                                             pcell, x, adt0, k);
   }
 }
 
-static void enqueue_iteration(op2b_batch_s *b, cudaStream_t s) {
-  int grid = rt().nsm * b->blocks_per_sm;
-  if (b->p32.bytes && b->p64.bytes)
-    k_b_promote<<<grid, b->block, 0, s>>>(b->dev.promote, b->dev.npromote,
-                                          (const float *)b->p32.q, (double *)b->p64.q);
-  if (b->p32.bytes) enqueue_stage<float>(b, b->p32, b->dev.w32, s, false);
-  if (b->p64.bytes) enqueue_stage<double>(b, b->p64, b->dev.w64, s, false);
+// One iteration.  `fork`: the FP64 stage on the batch's second stream (the two
+// precisions share no dat once the promotion is done).
+static void enqueue_iteration(op2b_batch_s *b, cudaStream_t s, bool fork) {
+  const bool both = b->p32.bytes && b->p64.bytes;
+  bool ok;
+  if (both)
+    k_b_promote<<<item_grid(b, b->ncells), b->block, 0, s>>>(
+        b->dev.promote, b->dev.npromote, (const float *)b->p32.q, (double *)b->p64.q,
+        reinterpret_cast<const int4 *>(b->p64.pcell), (const double *)b->p64.x,
+        (double *)b->p64.adt0, consts_or<double>(ok));
+  cudaStream_t s64 = s;
+  if (both && fork) {
+    cudaEventRecord(b->fork, s);
+    cudaStreamWaitEvent(b->side, b->fork, 0);
+    s64 = b->side;
+  }
+  if (b->p32.bytes) enqueue_stage<float>(b, b->p32, b->dev.w32, s);
+  if (b->p64.bytes) enqueue_stage<double>(b, b->p64, b->dev.w64, s64);
+  if (s64 != s) {
+    cudaEventRecord(b->join, s64);
+    cudaStreamWaitEvent(s, b->join, 0);
+  }
   k_b_converge<<<1, 1024, 0, s>>>(b->dev, 0);
+}
+
+// kernels of one iteration
+static long iteration_launches(const op2b_batch_s *b) {
+  const long stages = (b->p32.bytes ? 1 : 0) + (b->p64.bytes ? 1 : 0);
+  long step = 2;
+  if (b->res_kernel == OP2B_BATCH_RES_COLOUR) {
+    for (size_t c = 0; c + 1 < b->colour_off.size(); c++)
+      step += b->colour_off[c + 1] > b->colour_off[c];
+  } else if (b->res_kernel != OP2B_BATCH_RES_GATHER || !b->linked) {
+    step = 3;
+  }
+  return stages * 2 * step + (stages == 2 ? 1 : 0) + 1;
+}
+
+// the adt_calc of the current q, which the first step of a run reads (the
+// caller may have changed q since the last one)
+static void enqueue_first_adt(op2b_batch_s *b, cudaStream_t s) {
+  bool ok;
+  const int g = item_grid(b, b->ncells);
+  if (b->p32.bytes)
+    k_b_adt<float><<<g, b->block, 0, s>>>(b->dev.w32.cells, b->dev.w32.count,
+                                          reinterpret_cast<const int4 *>(b->p32.pcell),
+                                          (const float *)b->p32.x, (const float *)b->p32.q,
+                                          (float *)b->p32.adt0, consts_or<float>(ok));
+  k_b_adt<double><<<g, b->block, 0, s>>>(b->dev.w64.cells, b->dev.w64.count,
+                                         reinterpret_cast<const int4 *>(b->p64.pcell),
+                                         (const double *)b->p64.x, (const double *)b->p64.q,
+                                         (double *)b->p64.adt0, consts_or<double>(ok));
+}
+
+// The records of the batch's maps, found again when any renumbering has dropped
+// the cached ones since (a captured iteration holds their arrays).
+static bool batch_records(op2b_batch_s *b) {
+  if (b->generation == gather_generation()) return true;
+  op_map pecell = b->h64.pecell, pedge = b->h64.pedge, pbecell = b->h64.pbecell;
+  b->slots = get_corner_records(pecell, pedge);
+  b->inv_bound = get_inverse_map(pbecell);
+  if (!b->slots || !b->inv_bound || !b->slots->usable) {
+    if (b->slots && !b->slots->usable)
+      set_error("op2b_batch: a cell has more than four edges");
+    return false;
+  }
+  const BresRecords *br = b->slots->corners ? get_bres_records(pbecell, b->h64.pbedge) : nullptr;
+  b->linked = br && link_boundary_records(b->slots, br, pbecell);
+  b->generation = gather_generation();
+  b->graph_dirty = true;
+  return true;
+}
+
+// Elements per item: the caller's, else 2048, less (not below 256 or a block)
+// where that leaves under 16 items an SM -- 637,000 cells are 311 items of
+// 2048, two or three CTAs an SM, and 2490 of 256.
+static void set_chunk(op2b_batch_s *b) {
+  int n = b->part_size;
+  if (n <= 0)
+    for (n = 2048; n > std::max(kMinChunk, b->block) &&
+                   (long long)b->ncells < 16LL * rt().nsm * n;)
+      n /= 2;
+  b->dev.chunk = n;
 }
 
 static bool fill_dats(const op2b_airfoil_dats *h, PrecisionDats &d, int want_bytes) {
@@ -480,7 +641,7 @@ static bool fill_dats(const op2b_airfoil_dats *h, PrecisionDats &d, int want_byt
 
 // the colours of the batch's edges for OP2B_BATCH_RES_COLOUR: a parallel
 // (Jones-Plassmann) OP_COLOR2 plan of res_calc's two increments over pecell,
-// built once (before any capture) and kept in the plan cache
+// kept in the plan cache (asked for again by every run: the cache may have been emptied)
 static bool build_colouring(op2b_batch_s *b) {
   op_arg args[2] = {op_arg_dat(b->h64.p_res, 0, b->h64.pecell, 4, "double", OP_INC),
                     op_arg_dat(b->h64.p_res, 1, b->h64.pecell, 4, "double", OP_INC)};
@@ -491,9 +652,16 @@ static bool build_colouring(op2b_batch_s *b) {
     if (!op2b_last_error()[0]) set_error("op2b_batch: colouring the edges failed");
     return false;
   }
+  if (b->colour_elems != pl->col_reord_d) b->graph_dirty = true;
   b->colour_elems = pl->col_reord_d;
   b->colour_off.assign(pl->pub.color2_offsets, pl->pub.color2_offsets + pl->pub.ncolors + 1);
   return true;
+}
+
+static void batch_streams_free(op2b_batch_s *b) {
+  if (b->side) cudaStreamDestroy(b->side);
+  if (b->fork) cudaEventDestroy(b->fork);
+  if (b->join) cudaEventDestroy(b->join);
 }
 
 extern "C" {
@@ -519,7 +687,7 @@ op2b_batch op2b_batch_create(const op2b_airfoil_dats *fp32, const op2b_airfoil_d
   }
   b->h64 = *fp64;
   if (fp32) b->h32 = *fp32;
-  op_map pecell = fp64->pecell, pedge = fp64->pedge, pbecell = fp64->pbecell;
+  op_map pecell = fp64->pecell;
   b->ncells = pecell->to->size;
   if (cell_off[0] != 0 || cell_off[ninst] != b->ncells || edge_off[0] != 0 ||
       edge_off[ninst] != pecell->from->size) {
@@ -527,11 +695,7 @@ op2b_batch op2b_batch_create(const op2b_airfoil_dats *fp32, const op2b_airfoil_d
     delete b;
     return nullptr;
   }
-  b->slots = get_slot_records(pecell, pedge);
-  b->inv_bound = get_inverse_map(pbecell);
-  if (!b->slots || !b->inv_bound || !b->slots->usable) {
-    if (b->slots && !b->slots->usable)
-      set_error("op2b_batch_create: a cell has more than four edges");
+  if (!batch_records(b)) {
     delete b;
     return nullptr;
   }
@@ -551,7 +715,7 @@ op2b_batch op2b_batch_create(const op2b_airfoil_dats *fp32, const op2b_airfoil_d
   };
   BatchDev &d = b->dev;
   d.ninst = ninst;
-  d.chunk = 2048;
+  set_chunk(b);
   d.tol = 1e-6;
   d.promote_tol = 1e-4;
   d.max_iter = 1000000;
@@ -591,6 +755,20 @@ op2b_batch op2b_batch_create(const op2b_airfoil_dats *fp32, const op2b_airfoil_d
   }
   d.promote = (WorkItem *)A(sizeof(WorkItem) * (cap_c + 1));
   d.npromote = (int *)A(sizeof(int));
+  d.built = (int *)A(sizeof(int));
+  if (b->p32.bytes) b->p32.adt0 = A(sizeof(float) * (size_t)b->ncells);
+  b->p64.adt0 = A(sizeof(double) * (size_t)b->ncells);
+  if (!b->p64.adt0 || (b->p32.bytes && !b->p32.adt0) ||
+      cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
+    set_error("op2b_batch_create: out of device memory");
+    for (void *p : b->owned)
+      if (p) cudaFree(p);
+    batch_streams_free(b);
+    delete b;
+    return nullptr;
+  }
   void *mh = nullptr, *md = nullptr;
   if (cudaHostAlloc(&mh, 4096, cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&md, mh, 0) != cudaSuccess) {
@@ -636,7 +814,7 @@ int op2b_batch_set(op2b_batch b, const char *key, double value) {
       set_error("op2b_batch_set: part_size must be in [%d, %d]", kMinChunk, 1 << 24);
       return -1;
     }
-    d.chunk = (int)value;  // the work lists of the next iteration use it
+    b->part_size = (int)value;  // the work lists of the next iteration use it
   } else {
     set_error("op2b_batch_set: unknown key '%s'", key);
     return -1;
@@ -646,6 +824,7 @@ int op2b_batch_set(op2b_batch b, const char *key, double value) {
     b->block = 256;
     return -1;
   }
+  set_chunk(b);
   b->graph_dirty = true;
   return 0;
 }
@@ -656,14 +835,14 @@ int op2b_batch_run(op2b_batch b, int max_iterations, int check_every, int use_gr
   if (!b || !r.ready()) return -1;
   cudaStream_t s = r.stream;
   if (check_every < 1) check_every = 1;
-  if (b->res_kernel == OP2B_BATCH_RES_COLOUR && !b->colour_elems && !build_colouring(b))
-    return -1;
+  if (!batch_records(b)) return -1;
+  if (b->res_kernel == OP2B_BATCH_RES_COLOUR && !build_colouring(b)) return -1;
   if (use_graph && b->graph_dirty) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
     cudaGraph_t g;
     cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    enqueue_iteration(b, s);
+    enqueue_iteration(b, s, true);
     if (!cuda_ok(cudaStreamEndCapture(s, &g), "op2b_batch_run: capture")) return -1;
     if (!cuda_ok(cudaGraphInstantiate(&b->graph, g, 0), "op2b_batch_run: instantiate")) {
       cudaGraphDestroy(g);
@@ -679,17 +858,21 @@ int op2b_batch_run(op2b_batch b, int max_iterations, int check_every, int use_gr
   cudaEventCreate(&e1);
   cudaEventRecord(e0, s);
   int done = 0;
+  if (max_iterations > 0) {
+    enqueue_first_adt(b, s);
+    r.launches += b->p32.bytes ? 2 : 1;
+  }
   while (done < max_iterations) {
     int n = std::min(check_every, max_iterations - done);
     for (int i = 0; i < n; i++) {
       if (use_graph) {
         if (!cuda_ok(cudaGraphLaunch(b->graph, s), "op2b_batch_run: graph launch")) return -1;
       } else {
-        enqueue_iteration(b, s);
-        r.launches += 20;
+        enqueue_iteration(b, s, false);
+        r.launches += iteration_launches(b);
       }
     }
-    if (use_graph) r.launches += 20L * n;
+    if (use_graph) r.launches += iteration_launches(b) * n;
     done += n;
     if (!cuda_ok(cudaStreamSynchronize(s), "op2b_batch_run")) return -1;
     if (m[0] == 0) break;
@@ -760,7 +943,8 @@ int op2b_batch_tune(op2b_batch b, int iters, char *report, int report_len) {
   for (const Cand &c : cands) {
     b->res_kernel = c.res_kernel;
     b->block = c.block;
-    d.chunk = c.part;
+    b->part_size = c.part;
+    set_chunk(b);
     b->graph_dirty = true;
     // reset state before each candidate
     if (sq32) restore(b->p32.q, sq32, qb32);
@@ -786,7 +970,8 @@ int op2b_batch_tune(op2b_batch b, int iters, char *report, int report_len) {
   }
   b->res_kernel = bestc.res_kernel;
   b->block = bestc.block;
-  d.chunk = bestc.part;
+  b->part_size = bestc.part;
+  set_chunk(b);
   b->graph_dirty = true;
   if (sq32) restore(b->p32.q, sq32, qb32);
   restore(b->p64.q, sq64, qb64);
@@ -819,6 +1004,7 @@ void op2b_batch_destroy(op2b_batch b) {
   void *mh = b->owned.back();
   b->owned.pop_back();
   cudaFreeHost(mh);
+  batch_streams_free(b);
   for (void *p : b->owned)
     if (p) cudaFree(p);
   delete b;

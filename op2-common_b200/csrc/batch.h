@@ -36,6 +36,7 @@ struct BatchDev {
   WorkLists w32, w64;  // FP32-phase and FP64-phase work
   WorkItem *promote;   // cells of instances moving from FP32 to FP64
   int *npromote;
+  int *built;        // the item size the lists were built with
   int *mapped;       // mapped host page: [0] active instances, [1] iteration
   int chunk;         // elements per work item
   double tol, promote_tol;

@@ -20,6 +20,8 @@ struct InvMap {
 
 const InvMap *get_inverse_map(op_map map);
 void release_inverse_maps();  // also drops the slot records built on them
+// counts release_inverse_maps: what was built under another count is gone
+long gather_generation();
 
 // Four slots per cell for res_calc's 4-lanes-per-cell gather: other cell,
 // the edge's nodes, role (bit 30 of n2) and valid (bit 31 of n2).  usable is

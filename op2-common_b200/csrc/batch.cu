@@ -119,7 +119,8 @@ __global__ void k_b_res_gather(const WorkItem *items, const int *count, const in
 // records with the boundary edges linked in, corner.cuh), each instance's
 // freestream at its far-field edges: both loops' increments in their order
 template <typename T>
-__global__ void k_b_pair(const WorkItem *items, const int *count, const int4 *rec_o,
+__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)  // float: 64 registers, 1024 threads an SM
+k_b_pair(const WorkItem *items, const int *count, const int4 *rec_o,
                          const int4 *rec_cn, const unsigned *rec_meta, const int *bound,
                          const T *x, const T *q, const T *adt, T *res, const double *qinf,
                          int ncell, AirConst<T> k) {
@@ -477,9 +478,11 @@ template <typename T> static AirConst<T> consts_or(bool &ok) {
 // A launch's CTAs: one an item of a full list up to 16 an SM, whose scheduler
 // then evens out the items (a list shrinks as instances converge; a CTA
 // without an item ends at once), or the caller's blocks_per_sm.
-static int item_grid(const op2b_batch_s *b, long long elements) {
+// Of two precisions the FP64 one gets 4 an SM: most of a solve its list is empty,
+// and 2368 CTAs that find nothing take 4 us a launch.
+static int item_grid(const op2b_batch_s *b, long long elements, int per_sm = 16) {
   const long long items = elements / b->dev.chunk + b->ninst;
-  const long long cap = (long long)rt().nsm * (b->blocks_per_sm > 0 ? b->blocks_per_sm : 16);
+  const long long cap = (long long)rt().nsm * (b->blocks_per_sm > 0 ? b->blocks_per_sm : per_sm);
   return (int)std::max(1LL, std::min(items, cap));
 }
 
@@ -488,7 +491,8 @@ static void enqueue_stage(op2b_batch_s *b, const PrecisionDats &d, const WorkLis
                           cudaStream_t s) {
   bool ok;
   AirConst<T> k = consts_or<T>(ok);
-  const int th = b->block, gc = item_grid(b, b->ncells);
+  const int per_sm = sizeof(T) == 8 && b->p32.bytes ? 4 : 16;
+  const int th = b->block, gc = item_grid(b, b->ncells, per_sm);
   const T *x = (const T *)d.x;
   T *q = (T *)d.q, *qold = (T *)d.qold, *adt = (T *)d.adt, *res = (T *)d.res, *adt0 = (T *)d.adt0;
   const int4 *pcell = reinterpret_cast<const int4 *>(d.pcell);
@@ -500,7 +504,7 @@ static void enqueue_stage(op2b_batch_s *b, const PrecisionDats &d, const WorkLis
                                     d.bound, x, q, a, res, b->dev.qinf, b->ncells, k);
     } else {
       if (b->res_kernel == OP2B_BATCH_RES_ATOMIC)
-        k_b_res_atomic<T><<<item_grid(b, b->h64.pecell->from->size), th, 0, s>>>(
+        k_b_res_atomic<T><<<item_grid(b, b->h64.pecell->from->size, per_sm), th, 0, s>>>(
             w.edges, w.count + 2, reinterpret_cast<const int2 *>(d.pedge),
             reinterpret_cast<const int2 *>(d.pecell), x, q, a, res, k);
       else if (b->res_kernel == OP2B_BATCH_RES_COLOUR)
@@ -518,7 +522,7 @@ static void enqueue_stage(op2b_batch_s *b, const PrecisionDats &d, const WorkLis
                                             reinterpret_cast<const int4 *>(b->slots->n1),
                                             reinterpret_cast<const uint4 *>(b->slots->n2), x, q,
                                             a, res, k);
-      k_b_bres<T><<<item_grid(b, b->inv_bound->nrows), th, 0, s>>>(
+      k_b_bres<T><<<item_grid(b, b->inv_bound->nrows, per_sm), th, 0, s>>>(
           w.brows, w.count + 1, *b->inv_bound, reinterpret_cast<const int2 *>(d.pbedge), d.bound,
           x, q, a, res, b->dev.qinf, k);
     }
@@ -538,7 +542,7 @@ static void enqueue_iteration(op2b_batch_s *b, cudaStream_t s, bool fork) {
   const bool both = b->p32.bytes && b->p64.bytes;
   bool ok;
   if (both)
-    k_b_promote<<<item_grid(b, b->ncells), b->block, 0, s>>>(
+    k_b_promote<<<item_grid(b, b->ncells, 4), b->block, 0, s>>>(
         b->dev.promote, b->dev.npromote, (const float *)b->p32.q, (double *)b->p64.q,
         reinterpret_cast<const int4 *>(b->p64.pcell), (const double *)b->p64.x,
         (double *)b->p64.adt0, consts_or<double>(ok));

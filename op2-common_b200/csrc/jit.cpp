@@ -43,6 +43,7 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <charconv>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -54,6 +55,8 @@
 #include <string>
 #include <vector>
 
+#include <unistd.h>
+
 #include "gather.h"
 #include "op2b_plan.h"
 #include "op2b_runtime.h"
@@ -62,9 +65,20 @@
 namespace op2b {
 namespace {
 
+// A loop's source with its preludes and includes in line.  Kept while it comes
+// from registered text alone (`version` counts registrations); what came from
+// a file is read again by every call, as the file may have changed.
+struct Body {
+  long version = -1;
+  std::string text;
+  size_t hash = 0;
+};
+
 struct Sources {
   std::map<std::string, std::string> kernels;
   std::vector<std::string> preludes;
+  long version = 0;
+  std::map<std::string, Body, std::less<>> bodies;  // by loop name
 };
 Sources &sources() {
   static Sources s;
@@ -92,6 +106,14 @@ std::vector<std::string> search_path() {
     b = e + 1;
   }
   return dirs;
+}
+
+// whether `name` is a registered source or a file on the search path
+bool have_file(const std::string &name) {
+  if (sources().kernels.count(name)) return true;
+  for (const std::string &d : search_path())
+    if (access((d + "/" + name).c_str(), R_OK) == 0) return true;
+  return false;
 }
 
 // a registered source or a file on the search path
@@ -660,8 +682,49 @@ bool upload_constants(Jit &j) {
 }  // namespace
 
 bool jit_has_kernel(const char *name) {
-  std::string src;
-  return name && find_file(std::string(name) + ".h", src);
+  return name && have_file(std::string(name) + ".h");
+}
+
+// whether the text has a line that includes a (possibly absent) file by name
+static bool includes_files(const std::string &text) {
+  for (size_t p = 0; (p = text.find("#include", p)) != std::string::npos; p++) {
+    const size_t e = text.find('\n', p), q = text.find('"', p);
+    if (q != std::string::npos && (e == std::string::npos || q < e)) return true;
+  }
+  return false;
+}
+
+// the loop's whole source; null, with the error set, when there is none
+static const Body *loop_body(const char *name) {
+  Sources &S = sources();
+  const bool types_file = S.preludes.empty() && have_file("user_types.h");
+  auto it = S.bodies.find(name);
+  if (it != S.bodies.end() && it->second.version == S.version && !types_file) return &it->second;
+  Body b;
+  std::vector<std::string> seen;
+  bool registered = !types_file;  // nothing of it read from a file
+  for (auto &p : S.preludes) {
+    registered = registered && !includes_files(p);
+    b.text += expand(p, seen, 0) + "\n";
+  }
+  std::string types;
+  if (S.preludes.empty() && find_file("user_types.h", types)) {
+    seen.push_back("user_types.h");
+    b.text += expand(types, seen, 0) + "\n";
+  }
+  std::string ksrc;
+  const std::string file = std::string(name) + ".h";
+  if (!find_file(file, ksrc)) {
+    set_error("op_par_loop(%s): no device implementation of this loop is registered, and no "
+              "kernel source %s.h was registered or found on OP2B_KERNEL_PATH", name, name);
+    return nullptr;
+  }
+  seen.push_back(file);
+  registered = registered && S.kernels.count(file) && !includes_files(ksrc);
+  b.text += expand(ksrc, seen, 0);
+  b.hash = std::hash<std::string>()(b.text);
+  b.version = registered ? S.version : -1;
+  return &(S.bodies[name] = std::move(b));
 }
 
 void release_jit() {
@@ -721,8 +784,12 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   Runtime &r = rt();
   std::vector<ArgPlan> ap((size_t)nargs);
   bool coloured = false;
-  std::ostringstream key;
-  key << name;
+  std::string key = name;
+  auto num = [&](long v) {
+    char t[24];
+    key.append(t, (size_t)(std::to_chars(t, t + sizeof(t), v).ptr - t));
+    key += ':';
+  };
   for (int i = 0; i < nargs; i++) {
     const op_arg &x = args[i];
     ArgPlan &a = ap[(size_t)i];
@@ -734,7 +801,11 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
       if (!a.bytes) a.ctype = "double", a.bytes = 8;
       a.dim = std::max(x.argtype == OP_ARG_DAT && x.dat ? x.dat->dim : x.dim, 1);
       a.vec = x.argtype == OP_ARG_DAT && x.map && x.idx < -1 ? -x.idx : 0;
-      key << "|off:" << a.ctype << ":" << a.dim << ":" << a.vec;
+      key += "|off:";
+      key += a.ctype;
+      key += ':';
+      num(a.dim);
+      num(a.vec);
       continue;
     }
     if (x.argtype == OP_ARG_DAT) {
@@ -803,8 +874,11 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     } else {
       return set_error("op_par_loop(%s): argument %d: unknown argument kind", name, i), -1;
     }
-    key << "|" << a.kind << ":" << a.ctype << ":" << a.dim << ":" << a.acc << ":" << a.mdim
-        << ":" << a.idx << ":" << a.vec;
+    key += '|';
+    num(a.kind);
+    key += a.ctype;
+    key += ':';
+    for (int v : {a.dim, a.acc, a.mdim, a.idx, a.vec}) num(v);
   }
   // option jit_exact: a loop whose only effect is to increment one dat
   // through one map (no other writes, no global reductions, the dat read by
@@ -838,7 +912,10 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     ok = ok && std::adjacent_find(slots.begin(), slots.end()) == slots.end();
     if (!ok || own < 0 || (long long)args[own].map->from->size * args[own].map->dim >= INT32_MAX)
       own = -1;
-    if (own >= 0) key << "|own" << own;
+    if (own >= 0) {
+      key += "|own";
+      num(own);
+    }
   }
   // option jit_warp: a direct dat that no other argument of the loop names
   // moves through the warp's shared memory in whole rows (coalesced) and the
@@ -853,12 +930,13 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     has_red |= a.kind == INFO || (a.kind == GBL && a.acc != OP_READ && a.acc != OP_WORK);
   }
   if (r.opt_jit_warp && own < 0) {
-    std::map<op_dat, int> uses, writes;
-    for (int i = 0; i < nargs; i++)
-      if (ap[(size_t)i].kind == DIRECT || ap[(size_t)i].kind == INDIRECT) {
-        uses[args[i].dat]++;
-        if (ap[(size_t)i].acc != OP_READ) writes[args[i].dat]++;
-      }
+    auto named = [&](op_dat d, bool written) {  // arguments that name (write) the dat
+      int n = 0;
+      for (int i = 0; i < nargs; i++)
+        n += (ap[(size_t)i].kind == DIRECT || ap[(size_t)i].kind == INDIRECT) &&
+             args[i].dat == d && (!written || ap[(size_t)i].acc != OP_READ);
+      return n;
+    };
     // the warp buffer (256 threads x the widest row, 16-byte padded) shares
     // the 48 KB of static shared memory with op_arg_info's block reduction
     size_t info_bytes = 0;
@@ -877,10 +955,10 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
       // write-only row is stored by the kernel itself (loading it first cost
       // more than the scattered stores); read-only rows only in loops without
       // gathers, whose latency the staging would otherwise add to
-      if (a.kind == DIRECT && !coloured && a.dim > 1 && uses[args[i].dat] == 1 &&
+      if (a.kind == DIRECT && !coloured && a.dim > 1 && named(args[i].dat, false) == 1 &&
           fits((size_t)row + a.bytes) && a.acc != OP_WRITE && (a.acc != OP_READ || !gathers))
         a.stage = 1;
-      if (a.kind == INDIRECT && !a.vec && a.acc == OP_READ && writes[args[i].dat] == 0) {
+      if (a.kind == INDIRECT && !a.vec && a.acc == OP_READ && named(args[i].dat, true) == 0) {
         const uintptr_t base = (uintptr_t)args[i].dat->data_d;
         const int vw = (row % 16 == 0 && base % 16 == 0) ? 16 / a.bytes
                        : (row % 8 == 0 && base % 8 == 0 && a.bytes < 8) ? 8 / a.bytes : 0;
@@ -890,27 +968,25 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
         }
       }
       if (a.kind == INDIRECT && a.acc == OP_INC && !coloured && fits((size_t)row)) a.seg = true;
-      key << "|w" << a.stage << a.vw << a.seg;
+      key += "|w";
+      for (int v : {a.stage, a.vw, (int)a.seg}) num(v);
     }
   }
-  std::string body;
-  std::vector<std::string> seen;
-  for (auto &p : sources().preludes) body += expand(p, seen, 0) + "\n";
-  std::string types;
-  if (sources().preludes.empty() && find_file("user_types.h", types)) {
-    seen.push_back("user_types.h");
-    body += expand(types, seen, 0) + "\n";
+  const Body *body = loop_body(name);
+  if (!body) return -1;
+  static std::string consts;  // the constants' names, types and dimensions
+  static long consts_version = -1;
+  if (consts_version != r.const_version || r.consts.empty()) {
+    consts.clear();
+    for (auto &kv : r.consts)
+      consts += "|c:" + kv.first + ":" + r.const_types[kv.first] + ":" +
+                std::to_string(kv.second.size());
+    consts_version = r.const_version;
   }
-  std::string ksrc;
-  if (!find_file(std::string(name) + ".h", ksrc)) {
-    set_error("op_par_loop(%s): no device implementation of this loop is registered, and no "
-              "kernel source %s.h was registered or found on OP2B_KERNEL_PATH", name, name);
-    return -1;
-  }
-  seen.push_back(std::string(name) + ".h");
-  body += expand(ksrc, seen, 0);
-  for (auto &kv : r.consts) key << "|c:" << kv.first << ":" << r.const_types[kv.first] << ":" << kv.second.size();
-  key << "|s:" << std::hash<std::string>()(body) << "|col:" << coloured;
+  key += consts;
+  key += "|s:";
+  num((long)body->hash);
+  num(coloured);
   // each op_arg_info's block reduction keeps every thread's value, element and
   // payload in static shared memory (256 threads a block)
   size_t info_smem = 0;
@@ -927,11 +1003,11 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   // the colouring (built once per loop signature and cached with the plans)
   const Plan *plan = nullptr;
   if (coloured && set->size > 0 && !(plan = colour_plan(name, set, nargs, args))) return -1;
-  Jit &j = cache()[key.str()];
+  Jit &j = cache()[key];
   if (!j.fn) {
-    const std::string src = generate(name, ap, body, coloured, own);
+    const std::string src = generate(name, ap, body->text, coloured, own);
     if (!compile(name, src, j)) {
-      cache().erase(key.str());
+      cache().erase(key);
       return -1;
     }
   }
@@ -1168,6 +1244,7 @@ int op2b_register_kernel(const char *name, const char *source) {
   if (n.size() < 2 || n.compare(n.size() - 2, 2, ".h") != 0) n += ".h";
   if (source) op2b::sources().kernels[n] = source;
   else op2b::sources().kernels.erase(n);  // forget it
+  op2b::sources().version++;
   op2b::release_jit();  // sources changed: compile afresh
   return 0;
 }
@@ -1178,6 +1255,7 @@ int op2b_register_prelude(const char *source) {
     return -1;
   }
   op2b::sources().preludes.push_back(source);
+  op2b::sources().version++;
   op2b::release_jit();
   return 0;
 }

@@ -279,25 +279,25 @@ static char *copy_str(const char *s) {
   return d;
 }
 
+// `type` up to a ':' (as in "double:soa") is `name`
+static bool type_is(const char *type, const char *name) {
+  const size_t n = strlen(name);
+  return strncmp(type, name, n) == 0 && (type[n] == 0 || type[n] == ':');
+}
+
 int type_bytes(const char *type) {
   if (!type) return 0;
-  std::string t(type);
-  size_t c = t.find(':');
-  if (c != std::string::npos) t = t.substr(0, c);
-  if (t == "double") return 8;
-  if (t == "float") return 4;
-  if (t == "int" || t == "uint") return 4;
-  if (t == "ll" || t == "ull" || t == "long") return 8;
-  if (t == "bool") return 1;
+  if (type_is(type, "double")) return 8;
+  if (type_is(type, "float")) return 4;
+  if (type_is(type, "int") || type_is(type, "uint")) return 4;
+  if (type_is(type, "ll") || type_is(type, "ull") || type_is(type, "long")) return 8;
+  if (type_is(type, "bool")) return 1;
   return 0;
 }
 
 bool is_real(const char *type, int bytes) {
   if (!type) return false;
-  std::string t(type);
-  size_t c = t.find(':');
-  if (c != std::string::npos) t = t.substr(0, c);
-  return (bytes == 8 && t == "double") || (bytes == 4 && t == "float");
+  return (bytes == 8 && type_is(type, "double")) || (bytes == 4 && type_is(type, "float"));
 }
 
 LaunchCtx Runtime::ctx() { return LaunchCtx{stream, nsm, &launches, opt_pdl != 0}; }
@@ -327,9 +327,10 @@ bool Runtime::ready() {
 // launch, stay off most calls.  Totals are the sampled mean times the calls.
 void Runtime::begin_loop(const char *name) {
   cur_loop = name;
+  cur_stat = &loop_stat(name);
   cur_ev0 = cur_ev1 = nullptr;
   if (!opt_timing) return;
-  const long calls = stats[cur_loop].calls;
+  const long calls = cur_stat->calls;
   if (opt_timing_stride > 1 && calls % opt_timing_stride != 0 && !profile_times_loops()) return;
   if (ev_free.size() < 2) {
     for (int i = 0; i < 64; i++) {
@@ -345,7 +346,7 @@ void Runtime::begin_loop(const char *name) {
 }
 
 void Runtime::end_loop(double bytes) {
-  LoopStat &s = stats[cur_loop];
+  LoopStat &s = *cur_stat;
   s.calls++;
   s.bytes_per_call = bytes;
   if (!opt_timing || !cur_ev0) return;

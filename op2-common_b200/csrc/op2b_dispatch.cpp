@@ -107,19 +107,25 @@ struct Sig {
   }
 };
 
+// the Airfoil constants, looked up again when any constant was declared since
 template <typename T> AirConst<T> air_consts(bool &ok) {
-  AirConst<T> k{};
+  static AirConst<T> k{};
+  static long version = -1;
   Runtime &r = rt();
+  ok = true;
+  if (version == r.const_version && !r.consts.empty()) return k;
+  version = -1;
   const double *gam = r.const_ptr("gam", 1), *gm1 = r.const_ptr("gm1", 1),
                *cfl = r.const_ptr("cfl", 1), *eps = r.const_ptr("eps", 1),
                *qinf = r.const_ptr("qinf", 4);
   ok = gam && gm1 && cfl && eps && qinf;
-  if (!ok) return k;
+  if (!ok) return AirConst<T>{};
   k.gam = (T)*gam;
   k.gm1 = (T)*gm1;
   k.cfl = (T)*cfl;
   k.eps = (T)*eps;
   for (int i = 0; i < 4; i++) k.qinf[i] = (T)qinf[i];
+  version = r.const_version;
   return k;
 }
 
@@ -570,7 +576,7 @@ int loop_bres_calc(const char *name, op_set set, int nargs, op_arg *a) {
   s.dat(4, 4, OP_INC, pbecell, 0);
   s.dat(5, 1, OP_READ, nullptr, -1);
   if (s.ok && a[1].dat != a[0].dat) return s.fail(1, "arguments 0 and 1 must be the same dat"), kSigMismatch;
-  if (s.ok && (type_bytes(a[5].dat->type) != 4 || std::string(a[5].dat->type).rfind("int", 0) != 0))
+  if (s.ok && (type_bytes(a[5].dat->type) != 4 || strncmp(a[5].dat->type, "int", 3) != 0))
     return s.fail(5, "the boundary flag must be an int dat"), kSigMismatch;
   int rb = s.real_bytes({0, 2, 3, 4});
   if (!s.ok) return kSigMismatch;
@@ -955,20 +961,17 @@ int op_par_loop_c(char const *name, op_set set, int nargs, op_arg *args) {
   }
   for (const Entry &e : kLoops)
     if (strcmp(e.name, name) == 0) {
-      // with a kernel source to fall back on, a signature mismatch is not
-      // reported: the application's own loop of that name runs instead
-      const bool fallback = jit_has_kernel(name);
-      r.quiet_errors = fallback;
+      // an error is reported once the call is known not to be an
+      // application's own loop that shares a name with an Airfoil loop but not
+      // its arguments: that runs its kernel source, if it has one (looked for
+      // only then: the search may read files)
+      r.quiet_errors = true;
       int rc = e.fn(name, set, nargs, args);
       r.quiet_errors = false;
-      if (rc != kSigMismatch) {
-        if (rc != 0 && fallback) set_error("%s", op2b_last_error());  // report it now
-        return rc;
-      }
-      // an application's own loop that shares a name with an Airfoil loop
-      // but not its arguments: run its kernel source if it has one
-      if (!jit_has_kernel(name)) return -1;
-      break;
+      if (rc == 0) return 0;
+      if (rc == kSigMismatch && jit_has_kernel(name)) break;
+      set_error("%s", std::string(op2b_last_error()).c_str());
+      return -1;
     }
   if (r.outstanding() && !r.flush_pending()) return -1;
   if (r.spec.inplace && !r.restore_spec()) return -1;

@@ -153,7 +153,7 @@ struct Runtime {
   std::vector<std::unique_ptr<op_set_core>> sets;
   std::vector<std::unique_ptr<op_map_core>> maps;
   std::vector<std::unique_ptr<op_dat_core>> dats;
-  std::map<std::string, std::vector<double>> consts;
+  std::map<std::string, std::vector<double>, std::less<>> consts;
   std::map<std::string, std::string> const_types;  // "double", "float" or "int"
   long const_version = 0;                          // bumped by every op_decl_const
   std::map<const int *, op_map> map_ptrs;  // user array -> map (op_renumber_ptr)
@@ -170,10 +170,11 @@ struct Runtime {
   unsigned long long *check_d = nullptr;  // device word for op_decl_map's range check
 
   // timing
-  std::map<std::string, LoopStat> stats;
+  std::map<std::string, LoopStat, std::less<>> stats;  // found by name without a copy of it
   std::vector<cudaEvent_t> ev_free;
   std::vector<PendingTime> pending;
   std::string cur_loop;
+  LoopStat *cur_stat = nullptr;  // cur_loop's, from begin_loop to end_loop
   cudaEvent_t cur_ev0 = nullptr, cur_ev1 = nullptr;
 
   PendingLoop pend;
@@ -206,7 +207,11 @@ struct Runtime {
   bool materialize_save();  // op2b_dispatch.cpp: the renamed save_soln's copy
   bool restore_spec();   // op2b_dispatch.cpp: put the old adt back if adt is ahead
   void begin_loop(const char *name);
-  void count_call(const char *name) { stats[name].calls++; }  // a call with no launch
+  LoopStat &loop_stat(const char *name) {
+    auto it = stats.find(name);
+    return it != stats.end() ? it->second : stats[name];
+  }
+  void count_call(const char *name) { loop_stat(name).calls++; }  // a call with no launch
   void end_loop(double bytes);
   void resolve_timing();
   const double *const_ptr(const char *name, int dim);

@@ -94,10 +94,11 @@ class Airfoil:
                    (b"res_calc", self.edges, mk(self.a_res), 8),
                    (b"bres_calc", self.bedges, mk(self.a_bres), 6),
                    (b"update", self.cells, mk(self.a_upd), len(upd))]
+        self._par_loop = L.load().op_par_loop_c
 
     def _loop(self, i):
         name, s, arr, n = self._c[i]
-        if L.load().op_par_loop_c(name, s, n, arr) != 0:
+        if self._par_loop(name, s, n, arr) != 0:
             raise L.Op2Error(L.last_error())
 
     def iterate(self, niter: int, history: bool = True):

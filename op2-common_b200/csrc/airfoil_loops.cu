@@ -391,7 +391,7 @@ __device__ __forceinline__ RedTriple block_reduce(RedTriple t) {
 
 // One pass over the cells: q = qold - res/adt, res = 0, and the block's
 // partial (sum del^2, max del^2, first index of the max).  The last block to
-// arrive reduces all partials in block order and writes `out`.
+// arrive reduces all partials in a fixed order and writes `out`.
 // With ADT the kernel also computes, from each cell's new q, the time step
 // that the following adt_calc computes (same arithmetic on the same stored q
 // values) and writes it into `next`, a second array of the runtime's (option
@@ -403,50 +403,57 @@ template <typename T> struct AdtNext {
   AirConst<T> k;
 };
 
-template <typename T, int THREADS, bool ADT, bool KEEP_RES = false>
-__global__ void __launch_bounds__(THREADS)
-k_update(int ncell, const T *__restrict__ qold, T *__restrict__ q, T *__restrict__ res,
-         const T *adt, RedSlot *__restrict__ parts, unsigned *__restrict__ counter,
-         RedSlot *__restrict__ out, RedSlot *host_out, long long seq, AdtNext<T> an, int rev) {
-  grid_dependency_wait();
-  RedTriple t{0.0, -INFINITY, LLONG_MAX};
-  int stride = gridDim.x * THREADS;
-  for (int i = blockIdx.x * THREADS + threadIdx.x; i < ncell; i += stride) {
-    const int n = rev ? ncell - 1 - i : i;
-    T qo[4], r[4], qn[4];
-    T x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y;
-    if constexpr (ADT) {  // the node gathers first: they do not depend on the update
-      const int4 c = __ldg(an.pcell + n);
-      Vec<T>::ld2(an.x + 2 * (size_t)c.x, x1x, x1y);
-      Vec<T>::ld2(an.x + 2 * (size_t)c.y, x2x, x2y);
-      Vec<T>::ld2(an.x + 2 * (size_t)c.z, x3x, x3y);
-      Vec<T>::ld2(an.x + 2 * (size_t)c.w, x4x, x4y);
-    }
-    Vec<T>::ld4(qold + 4 * (size_t)n, qo);
-    Vec<T>::ld4_rw(res + 4 * (size_t)n, r);
-    const T a_old = __ldg(adt + n);
-    double adti = 1.0f / (double)a_old;
+// q = qold - res/adt of cell n, its del^2 into the thread's triple; qn: the new q
+template <typename T, bool KEEP_RES>
+__device__ __forceinline__ void update_cell(int n, const T *__restrict__ qold, T *__restrict__ q,
+                                            T *__restrict__ res, const T *adt, RedTriple &t,
+                                            T (&qn)[4]) {
+  T qo[4], r[4];
+  Vec<T>::ld4(qold + 4 * (size_t)n, qo);
+  Vec<T>::ld4_rw(res + 4 * (size_t)n, r);
+  const T a_old = __ldg(adt + n);
+  double adti = 1.0f / (double)a_old;
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-      double del = adti * (double)r[m];
-      qn[m] = (T)((double)qo[m] - del);
-      double sq = del * del;
-      t.sum += sq;
-      if (sq > t.maxv || (sq == t.maxv && n < t.idx)) {  // the lowest cell on ties
-        t.maxv = sq;
-        t.idx = n;
-      }
+  for (int m = 0; m < 4; m++) {
+    double del = adti * (double)r[m];
+    qn[m] = (T)((double)qo[m] - del);
+    double sq = del * del;
+    t.sum += sq;
+    if (sq > t.maxv || (sq == t.maxv && n < t.idx)) {  // the lowest cell on ties
+      t.maxv = sq;
+      t.idx = n;
     }
-    Vec<T>::st4(q + 4 * (size_t)n, qn);
-    if constexpr (!KEEP_RES) {
-      T z[4] = {(T)0, (T)0, (T)0, (T)0};
-      Vec<T>::st4(res + 4 * (size_t)n, z);
-    }
-    if constexpr (ADT)
-      an.next[n] = air_adt<T>(x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y, qn[0], qn[1], qn[2],
-                              qn[3], an.k);
   }
+  Vec<T>::st4(q + 4 * (size_t)n, qn);
+  if constexpr (!KEEP_RES) {
+    T z[4] = {(T)0, (T)0, (T)0, (T)0};
+    Vec<T>::st4(res + 4 * (size_t)n, z);
+  }
+}
+
+__device__ __forceinline__ void publish(const RedTriple &a, RedSlot *__restrict__ out,
+                                        RedSlot *host_out, long long seq) {
+  *out = RedSlot{a.sum, a.maxv, a.idx, 0};
+  if (host_out) {
+    volatile RedSlot *h = host_out;
+    h->sum = a.sum;
+    h->maxv = a.maxv;
+    h->idx = a.idx;
+    h->pad = red_check(a.sum, a.maxv, a.idx, seq);
+  }
+}
+
+// the blocks' triples to one, published by the last block to arrive
+template <int THREADS>
+__device__ __forceinline__ void grid_reduce(RedTriple t, RedSlot *__restrict__ parts,
+                                            unsigned *__restrict__ counter,
+                                            RedSlot *__restrict__ out, RedSlot *host_out,
+                                            long long seq) {
   t = block_reduce<THREADS>(t);
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) publish(t, out, host_out, seq);
+    return;
+  }
   __shared__ bool last;
   if (threadIdx.x == 0) {
     parts[blockIdx.x] = RedSlot{t.sum, t.maxv, t.idx, 0};
@@ -464,17 +471,65 @@ k_update(int ncell, const T *__restrict__ qold, T *__restrict__ q, T *__restrict
   }
   a = block_reduce<THREADS>(a);
   if (threadIdx.x == 0) {
-    *out = RedSlot{a.sum, a.maxv, a.idx, 0};
-    if (host_out) {
-      volatile RedSlot *h = host_out;
-      h->sum = a.sum;
-      h->maxv = a.maxv;
-      h->idx = a.idx;
-      __threadfence_system();
-      h->pad = seq;  // published last
-    }
+    publish(a, out, host_out, seq);
     *counter = 0u;  // ready for the next launch (same stream, so ordered)
   }
+}
+
+template <typename T, int THREADS, bool ADT, bool KEEP_RES = false>
+__global__ void __launch_bounds__(THREADS)
+k_update(int ncell, const T *__restrict__ qold, T *__restrict__ q, T *__restrict__ res,
+         const T *adt, RedSlot *__restrict__ parts, unsigned *__restrict__ counter,
+         RedSlot *__restrict__ out, RedSlot *host_out, long long seq, AdtNext<T> an, int rev) {
+  grid_dependency_wait();
+  RedTriple t{0.0, -INFINITY, LLONG_MAX};
+  int stride = gridDim.x * THREADS;
+  for (int i = blockIdx.x * THREADS + threadIdx.x; i < ncell; i += stride) {
+    const int n = rev ? ncell - 1 - i : i;
+    T qn[4];
+    T x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y;
+    if constexpr (ADT) {  // the node gathers first: they do not depend on the update
+      const int4 c = __ldg(an.pcell + n);
+      Vec<T>::ld2(an.x + 2 * (size_t)c.x, x1x, x1y);
+      Vec<T>::ld2(an.x + 2 * (size_t)c.y, x2x, x2y);
+      Vec<T>::ld2(an.x + 2 * (size_t)c.z, x3x, x3y);
+      Vec<T>::ld2(an.x + 2 * (size_t)c.w, x4x, x4y);
+    }
+    update_cell<T, KEEP_RES>(n, qold, q, res, adt, t, qn);
+    if constexpr (ADT)
+      an.next[n] = air_adt<T>(x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y, qn[0], qn[1], qn[2],
+                              qn[3], an.k);
+  }
+  grid_reduce<THREADS>(t, parts, counter, out, host_out, seq);
+}
+
+// The update with the adt_calc after it (res recorded as zero) on a mesh of at
+// most a cell a thread: what the program waits for, the reduction, is published
+// before the time steps are computed, and one block of up to 1024 cells needs
+// no second round.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+k_update_small(int ncell, const T *__restrict__ qold, T *__restrict__ q, T *__restrict__ res,
+               const T *adt, RedSlot *__restrict__ parts, unsigned *__restrict__ counter,
+               RedSlot *__restrict__ out, RedSlot *host_out, long long seq, AdtNext<T> an,
+               int rev) {
+  grid_dependency_wait();
+  RedTriple t{0.0, -INFINITY, LLONG_MAX};
+  const int i = blockIdx.x * THREADS + threadIdx.x, n = rev ? ncell - 1 - i : i;
+  const bool in = i < ncell;
+  T qn[4], x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y;
+  if (in) {
+    const int4 c = __ldg(an.pcell + n);
+    Vec<T>::ld2(an.x + 2 * (size_t)c.x, x1x, x1y);
+    Vec<T>::ld2(an.x + 2 * (size_t)c.y, x2x, x2y);
+    Vec<T>::ld2(an.x + 2 * (size_t)c.z, x3x, x3y);
+    Vec<T>::ld2(an.x + 2 * (size_t)c.w, x4x, x4y);
+    update_cell<T, true>(n, qold, q, res, adt, t, qn);
+  }
+  grid_reduce<THREADS>(t, parts, counter, out, host_out, seq);
+  if (in)
+    an.next[n] = air_adt<T>(x1x, x1y, x2x, x2y, x3x, x3y, x4x, x4y, qn[0], qn[1], qn[2], qn[3],
+                            an.k);
 }
 
 template <typename T>
@@ -482,24 +537,27 @@ cudaError_t launch_update(const LaunchCtx &c, int ncell, const T *qold, T *q, T 
                           const T *adt, const RedScratch &s, const int *pcell, const T *x,
                           T *adt_next, const AirConst<T> *k, bool keep_res, bool reverse) {
   constexpr int TH = 256;
-  int grid = grid_for(c, ncell, TH, 4);
-  if (grid > s.capacity) grid = s.capacity;
   const int rev = reverse ? 1 : 0;
+  AdtNext<T> an{};
+  if (adt_next) an = AdtNext<T>{reinterpret_cast<const int4 *>(pcell), x, adt_next, *k};
   cudaError_t e;
-  if (adt_next) {
-    const AdtNext<T> an{reinterpret_cast<const int4 *>(pcell), x, adt_next, *k};
-    e = keep_res ? launch_dependent(c, k_update<T, TH, true, true>, grid, TH, 0, ncell, qold, q,
-                                    res, adt, s.parts, s.counter, s.out, s.host_out, s.seq, an, rev)
-                 : launch_dependent(c, k_update<T, TH, true>, grid, TH, 0, ncell, qold, q, res,
-                                    adt, s.parts, s.counter, s.out, s.host_out, s.seq, an, rev);
-  } else {
-    e = keep_res ? launch_dependent(c, k_update<T, TH, false, true>, grid, TH, 0, ncell, qold, q,
-                                    res, adt, s.parts, s.counter, s.out, s.host_out, s.seq,
-                                    AdtNext<T>{}, rev)
-                 : launch_dependent(c, k_update<T, TH, false>, grid, TH, 0, ncell, qold, q, res,
-                                    adt, s.parts, s.counter, s.out, s.host_out, s.seq,
-                                    AdtNext<T>{}, rev);
-  }
+  auto run = [&](auto kern, int threads, int grid) {
+    if (grid > s.capacity) grid = s.capacity;
+    return launch_dependent(c, kern, grid, threads, 0, ncell, qold, q, res, adt, s.parts,
+                            s.counter, s.out, s.host_out, s.seq, an, rev);
+  };
+  // as many CTAs as the SMs hold (four of the FP64 kernel, six of the FP32 one)
+  auto grid = [&](auto kern) { return grid_resident(c, kern, ncell, TH, 8); };
+  if (adt_next && keep_res && ncell > 0 && ncell <= 1024)
+    e = run(k_update_small<T, 1024>, 1024, 1);
+  else if (adt_next && keep_res && ncell > 0 && ncell <= 4 * TH * c.nsm)
+    e = run(k_update_small<T, TH>, TH, (ncell + TH - 1) / TH);
+  else if (adt_next)
+    e = keep_res ? run(k_update<T, TH, true, true>, TH, grid(k_update<T, TH, true, true>))
+                 : run(k_update<T, TH, true>, TH, grid(k_update<T, TH, true>));
+  else
+    e = keep_res ? run(k_update<T, TH, false, true>, TH, grid(k_update<T, TH, false, true>))
+                 : run(k_update<T, TH, false>, TH, grid(k_update<T, TH, false>));
   c.count();
   return e != cudaSuccess ? e : cudaGetLastError();
 }

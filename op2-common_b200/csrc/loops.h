@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <string.h>
 
 #include "airfoil_math.cuh"
 
@@ -57,6 +58,22 @@ struct RedSlot {
   long long pad;
 };
 
+// The word that completes a slot published to the host: no order among the
+// slot's stores is needed, as the host takes the values once the word fits
+// them and the call's sequence number (a slot half of the last call's does
+// not, unless the old values equal the new).
+static __host__ __device__ __forceinline__ long long red_check(double sum, double maxv,
+                                                               long long idx, long long seq) {
+  unsigned long long a, b;
+  memcpy(&a, &sum, 8);
+  memcpy(&b, &maxv, 8);
+  unsigned long long h = (unsigned long long)seq * 0x9e3779b97f4a7c15ull;
+  h = (h ^ a) * 0xbf58476d1ce4e5b9ull;
+  h = (h ^ (h >> 29) ^ b) * 0x94d049bb133111ebull;
+  h = (h ^ (h >> 32) ^ (unsigned long long)idx) * 0xd6e8feb86659fd93ull;
+  return (long long)(h ^ (h >> 31));
+}
+
 // Device scratch of the update reduction: `capacity` partial slots, a ticket
 // counter (zero between launches) and the final slot.
 struct RedScratch {
@@ -64,8 +81,8 @@ struct RedScratch {
   unsigned *counter;
   RedSlot *out;
   int capacity;
-  // mapped pinned host copy of the result; `pad` receives `seq` after the
-  // values, so the host can poll it instead of copying and synchronising
+  // mapped pinned host copy of the result; its `pad` is red_check of the values
+  // and `seq`, so the host can poll it instead of copying and synchronising
   RedSlot *host_out;
   long long seq;
 };

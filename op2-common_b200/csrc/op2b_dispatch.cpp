@@ -140,17 +140,27 @@ bool consts_match(const SpecAdt &sp, int rb) {
   return ok && memcmp(&k, &sp.kf, sizeof(k)) == 0;
 }
 
-// Spin until the device publishes `seq` at *flag.  Every few thousand spins
-// the stream is queried so a failed kernel is reported instead of waited
-// for; the wait gives up after 120 s.
-bool wait_for_sequence(volatile long long *flag, long long seq, const char *what) {
+// Spin until the device has published the slot of sequence number `seq` in the
+// mapped page (red_check).  Every few thousand spins the stream is queried so
+// a failed kernel is reported instead of waited for; the wait gives up after
+// 120 s.
+bool wait_for_result(const RedSlot *page, long long seq, RedSlot &got, const char *what) {
   Runtime &r = rt();
-  auto t0 = std::chrono::steady_clock::now();
-  for (long spins = 0; *flag != seq; spins++) {
+  const volatile RedSlot *h = page;
+  auto fits = [&] {
+    got.pad = h->pad;
+    std::atomic_thread_fence(std::memory_order_acquire);
+    got.sum = h->sum;
+    got.maxv = h->maxv;
+    got.idx = h->idx;
+    return got.pad == red_check(got.sum, got.maxv, got.idx, seq);
+  };
+  const auto t0 = std::chrono::steady_clock::now();
+  for (long spins = 0; !fits(); spins++) {
     if ((spins & 4095) == 4095) {
       cudaError_t q = cudaStreamQuery(r.stream);
       if (q != cudaSuccess && q != cudaErrorNotReady) return cuda_ok(q, what);
-      if (q == cudaSuccess && *flag != seq) {
+      if (q == cudaSuccess && !fits()) {
         set_error("%s: the stream finished without publishing the result", what);
         return false;
       }
@@ -160,7 +170,6 @@ bool wait_for_sequence(volatile long long *flag, long long seq, const char *what
       }
     }
   }
-  std::atomic_thread_fence(std::memory_order_acquire);
   return true;
 }
 
@@ -803,17 +812,18 @@ int loop_update(const char *name, op_set set, int nargs, op_arg *a) {
   // queue the res_calc + bres_calc that usually follow before waiting
   launch_speculative_res(r, a, rb);
   // gbl results are valid when op_par_loop returns: the kernel's last block
-  // publishes them in the mapped page, sequence number last
-  volatile RedSlot *h = reinterpret_cast<volatile RedSlot *>(r.pinned);
-  if (!wait_for_sequence(&h->pad, r.red.seq, "op_par_loop(update): reduction read-back"))
+  // publishes them in the mapped page
+  RedSlot got;
+  if (!wait_for_result(reinterpret_cast<const RedSlot *>(r.pinned), r.red.seq, got,
+                       "op_par_loop(update): reduction read-back"))
     return -1;
   if (C == 0) return 0;
-  *reinterpret_cast<double *>(a[4].data) += h->sum;
+  *reinterpret_cast<double *>(a[4].data) += got.sum;
   if (nargs == 8) {
     double *mx = reinterpret_cast<double *>(a[5].data);
-    if (h->maxv > *mx) {
-      *mx = h->maxv;
-      *reinterpret_cast<int *>(a[7].data) = (int)h->idx;
+    if (got.maxv > *mx) {
+      *mx = got.maxv;
+      *reinterpret_cast<int *>(a[7].data) = (int)got.idx;
     }
   }
   return 0;

@@ -43,7 +43,9 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <atomic>
 #include <charconv>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -186,7 +188,21 @@ int type_size(const std::string &t) {
   return 0;
 }
 
+// Global reductions of a loop that runs in one launch: every (argument,
+// component) is one 8-byte entry.  Blocks leave their partials in `parts_d`, the
+// last one to finish combines them in a fixed order and publishes them, with a
+// check word, in the runtime's mapped page, which the host polls: no identities
+// uploaded, no copy back, no atomics on one address by every warp.
+constexpr int kMaxRedEntries = 64;
+constexpr size_t kRedPageOffset = 1024;  // of the mapped page (the update's slot lies before it)
+
+unsigned long long red_mix(unsigned long long h, unsigned long long x) {
+  h = (h ^ x) * 0xbf58476d1ce4e5b9ull;
+  return h ^ (h >> 29);
+}
+
 struct Jit {
+  void *parts_d = nullptr;  // ticket (16 bytes), then the blocks' entries
   cudaLibrary_t lib = nullptr;
   cudaKernel_t fn = nullptr;
   std::vector<std::string> cnames, clowered;
@@ -254,14 +270,19 @@ __device__ void op2b_amax(float *a, float v) {
 }
 __device__ void op2b_amin(int *a, int v) { atomicMin(a, v); }
 __device__ void op2b_amax(int *a, int v) { atomicMax(a, v); }
+__device__ unsigned long long op2b_mix(unsigned long long h, unsigned long long x) {
+  h = (h ^ x) * 0xbf58476d1ce4e5b9ull;
+  return h ^ (h >> 29);
+}
 template <typename T> __device__ T op2b_min(T a, T b) { return b < a ? b : a; }
 template <typename T> __device__ T op2b_max(T a, T b) { return b > a ? b : a; }
 )";
 
+// red: the entries of the loop's global reductions, or 0 (none, or by atomics)
 // own >= 0: the owner-computes loop (option jit_exact) for the increments of
 // argument own's dat; the others of its increment arguments share its map
 std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std::string &body,
-                     bool coloured, int own = -1) {
+                     bool coloured, int own, int red) {
   Runtime &r = rt();
   std::ostringstream s;
   s << "// libop2b: generated loop for the user kernel '" << name << "'\n";
@@ -290,6 +311,9 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
   if (coloured) s << ", const int *op2b_perm, int op2b_first";
   // owner computes: op2b_n targets, each with its (element, slot) entries
   if (own >= 0) s << ", const long long *op2b_ioff, const int *op2b_ient, const int *op2b_rows";
+  // block reductions: ticket and partials, the mapped result, the call's number
+  if (red) s << ", unsigned *op2b_ticket, unsigned long long *op2b_parts, "
+                "volatile unsigned long long *op2b_host, unsigned long long op2b_seq";
   s << ") {\n";
   for (size_t i = 0; i < ap.size(); i++) {
     const ArgPlan &a = ap[i];
@@ -588,17 +612,69 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
       << "        for (int k = 0; k < " << a.dim << "; k++) op2b_ip" << i << "[blockIdx.x * "
       << a.dim << " + k] = sp[b * " << a.dim << " + k];\n      }\n    }\n  }\n";
   }
-  for (size_t i = 0; i < ap.size(); i++) {
-    const ArgPlan &a = ap[i];
-    if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
-    const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
-    s << "  for (int k = 0; k < " << a.dim << "; k++) {\n    " << a.ctype << " v = op2b_l" << i
-      << "[k];\n    for (int o = 16; o > 0; o >>= 1) { " << a.ctype
-      << " w = __shfl_down_sync(0xffffffffu, v, o); v = " << op << "; }\n"
-      << "    if ((threadIdx.x & 31) == 0) ";
-    if (a.acc == OP_INC) s << "atomicAdd(op2b_d" << i << " + k, v);\n";
-    else s << (a.acc == OP_MIN ? "op2b_amin" : "op2b_amax") << "(op2b_d" << i << " + k, v);\n";
-    s << "  }\n";
+  if (red) {
+    // one pass: `value(entry)` through the warps' shuffles into op2b_rs, then a
+    // thread an entry over the block's eight warps
+    s << "  __shared__ unsigned long long op2b_rs[8][" << red << "];\n  __shared__ bool op2b_last;\n";
+    for (int pass = 0; pass < 2; pass++) {
+      int t = 0;
+      for (size_t i = 0; i < ap.size(); i++) {
+        const ArgPlan &a = ap[i];
+        if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
+        const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
+        s << "#pragma unroll\n  for (int k = 0; k < " << a.dim << "; k++) {\n    " << a.ctype
+          << " v = ";
+        if (pass == 0)
+          s << "op2b_l" << i << "[k];\n";
+        else
+          s << identity(a.ctype, a.acc) << ";\n    for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) {\n"
+            << "      const " << a.ctype << " w = *(const volatile " << a.ctype << " *)(op2b_parts + (size_t)b * "
+            << red << " + " << t << " + k);\n      v = " << op << ";\n    }\n";
+        s << "    for (int o = 16; o > 0; o >>= 1) { " << a.ctype
+          << " w = __shfl_down_sync(0xffffffffu, v, o); v = " << op << "; }\n"
+          << "    if ((threadIdx.x & 31) == 0) *(" << a.ctype << " *)&op2b_rs[threadIdx.x >> 5]["
+          << t << " + k] = v;\n  }\n";
+        t += a.dim;
+      }
+      s << "  __syncthreads();\n";
+      t = 0;
+      for (size_t i = 0; i < ap.size(); i++) {
+        const ArgPlan &a = ap[i];
+        if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
+        const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
+        s << "  if (threadIdx.x >= " << t << " && threadIdx.x < " << t + a.dim << ") {\n    " << a.ctype
+          << " v = *(" << a.ctype << " *)&op2b_rs[0][threadIdx.x];\n"
+          << "    for (int j = 1; j < 8; j++) { const " << a.ctype << " w = *(" << a.ctype
+          << " *)&op2b_rs[j][threadIdx.x]; v = " << op << "; }\n"
+          << "    unsigned long long u = 0;\n    *(" << a.ctype << " *)&u = v;\n";
+        if (pass == 0)
+          s << "    op2b_parts[(size_t)blockIdx.x * " << red << " + threadIdx.x] = u;\n    __threadfence();\n";
+        else
+          s << "    op2b_rs[0][threadIdx.x] = u;\n    op2b_host[threadIdx.x] = u;\n";
+        s << "  }\n";
+        t += a.dim;
+      }
+      s << "  __syncthreads();\n";
+      if (pass == 0)
+        s << "  if (threadIdx.x == 0) op2b_last = atomicAdd(op2b_ticket, 1u) == gridDim.x - 1;\n"
+             "  __syncthreads();\n  if (!op2b_last) return;\n  __threadfence();\n";
+    }
+    s << "  if (threadIdx.x == 0) {\n    unsigned long long h = op2b_seq * 0x9e3779b97f4a7c15ull;\n"
+         "    for (int t = 0; t < " << red << "; t++) h = op2b_mix(h, op2b_rs[0][t]);\n"
+         "    op2b_host[" << red << "] = h;\n    *op2b_ticket = 0u;\n  }\n";
+  } else {
+    for (size_t i = 0; i < ap.size(); i++) {
+      const ArgPlan &a = ap[i];
+      if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
+      const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
+      s << "  for (int k = 0; k < " << a.dim << "; k++) {\n    " << a.ctype << " v = op2b_l" << i
+        << "[k];\n    for (int o = 16; o > 0; o >>= 1) { " << a.ctype
+        << " w = __shfl_down_sync(0xffffffffu, v, o); v = " << op << "; }\n"
+        << "    if ((threadIdx.x & 31) == 0) ";
+      if (a.acc == OP_INC) s << "atomicAdd(op2b_d" << i << " + k, v);\n";
+      else s << (a.acc == OP_MIN ? "op2b_amin" : "op2b_amax") << "(op2b_d" << i << " + k, v);\n";
+      s << "  }\n";
+    }
   }
   s << "}\n";
   return s.str();
@@ -731,6 +807,7 @@ void release_jit() {
   for (auto &kv : cache()) {
     if (kv.second.lib) cudaLibraryUnload(kv.second.lib);
     cudaFree(kv.second.gbl_d);
+    cudaFree(kv.second.parts_d);
   }
   cache().clear();
 }
@@ -778,6 +855,33 @@ const Plan *colour_plan(const char *name, op_set set, int nargs, const op_arg *a
     return nullptr;
   }
   return pl;
+}
+
+// Spin until the loop's reductions are in the mapped page: the entries, then
+// their check word.  The stream is queried now and then, so a failed kernel is
+// reported instead of waited for; gives up after 120 s.
+static bool wait_for_entries(const char *page, int n, unsigned long long seq, const char *name) {
+  const volatile unsigned long long *p = (const volatile unsigned long long *)page;
+  auto fits = [&] {
+    const unsigned long long want = p[n];
+    std::atomic_thread_fence(std::memory_order_acquire);
+    unsigned long long h = seq * 0x9e3779b97f4a7c15ull;
+    for (int t = 0; t < n; t++) h = red_mix(h, p[t]);
+    return h == want;
+  };
+  const auto t0 = std::chrono::steady_clock::now();
+  for (long spins = 1; !fits(); spins++) {
+    if (spins & 1023) continue;
+    const cudaError_t q = cudaStreamQuery(rt().stream);
+    if (q != cudaSuccess && q != cudaErrorNotReady) return cuda_ok(q, "op_par_loop: globals");
+    const bool late = std::chrono::steady_clock::now() - t0 > std::chrono::seconds(120);
+    if ((q == cudaSuccess && !fits()) || late) {
+      set_error("op_par_loop(%s): %s", name, late ? "no reduction result after 120 s"
+                                                  : "the loop ended without its reduction result");
+      return false;
+    }
+  }
+  return true;
 }
 
 int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
@@ -929,6 +1033,12 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     has_info |= a.kind == INFO;
     has_red |= a.kind == INFO || (a.kind == GBL && a.acc != OP_READ && a.acc != OP_WORK);
   }
+  // the global reductions' entries, when blocks can combine them: one launch,
+  // no op_arg_info (whose per-block results are copied back anyway)
+  int red = 0;
+  for (auto &a : ap)
+    if (a.kind == GBL && a.acc != OP_READ && a.acc != OP_WORK) red += a.dim;
+  if (coloured || has_info || red > kMaxRedEntries) red = 0;
   if (r.opt_jit_warp && own < 0) {
     auto named = [&](op_dat d, bool written) {  // arguments that name (write) the dat
       int n = 0;
@@ -942,7 +1052,8 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     size_t info_bytes = 0;
     for (auto &a : ap)
       if (a.kind == INFO) info_bytes += 256 * (16 + (size_t)a.dim * a.bytes);
-    const size_t budget = info_bytes < 46 * 1024 ? 46 * 1024 - info_bytes : 0;
+    const size_t taken = info_bytes + 64 * (size_t)red;  // the reductions' eight warps an entry
+    const size_t budget = taken < 46 * 1024 ? 46 * 1024 - taken : 0;
     auto fits = [&](size_t row_bytes) {
       return row_bytes <= 128 && 256 * ((row_bytes + 15) & ~(size_t)15) <= budget;
     };
@@ -1005,7 +1116,7 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   if (coloured && set->size > 0 && !(plan = colour_plan(name, set, nargs, args))) return -1;
   Jit &j = cache()[key];
   if (!j.fn) {
-    const std::string src = generate(name, ap, body->text, coloured, own);
+    const std::string src = generate(name, ap, body->text, coloured, own, red);
     if (!compile(name, src, j)) {
       cache().erase(key);
       return -1;
@@ -1015,8 +1126,12 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   // globals: device copies (OP_READ values, reduction identities)
   std::vector<size_t> goff((size_t)nargs, 0);
   size_t gbytes = 0;
+  auto is_red = [&](const ArgPlan &a) {
+    return a.kind == GBL && a.acc != OP_READ && a.acc != OP_WORK;
+  };
   for (int i = 0; i < nargs; i++)
-    if (ap[(size_t)i].kind == GBL || ap[(size_t)i].kind == OFF) {  // OFF: zeroed scratch
+    if ((ap[(size_t)i].kind == GBL && !(red && is_red(ap[(size_t)i]))) ||
+        ap[(size_t)i].kind == OFF) {  // OFF: zeroed scratch
       goff[(size_t)i] = gbytes;
       gbytes += ((size_t)ap[(size_t)i].dim * ap[(size_t)i].bytes + 15) & ~(size_t)15;
     }
@@ -1037,7 +1152,7 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   }
   for (int i = 0; i < nargs; i++) {
     const ArgPlan &a = ap[(size_t)i];
-    if (a.kind != GBL) continue;
+    if (a.kind != GBL || (red && is_red(a))) continue;
     char *dst = gh.data() + goff[(size_t)i];
     if (a.acc == OP_READ || a.acc == OP_INC || a.acc == OP_WORK) {
       if (a.acc != OP_INC) memcpy(dst, args[i].data, (size_t)a.dim * a.bytes);
@@ -1069,6 +1184,11 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
                                          r.stream),
                          "op_par_loop: globals"))
     return -1;
+  if (red && !j.parts_d) {
+    const size_t pb = 16 + 8 * (size_t)red * (size_t)max_grid;
+    if (!cuda_ok(cudaMalloc(&j.parts_d, pb), "op_par_loop: globals")) return -1;
+    cudaMemsetAsync(j.parts_d, 0, 16, r.stream);
+  }
   // parameters
   std::vector<void *> ptrs;
   ptrs.reserve((size_t)nargs * 4 + 1);  // kp keeps pointers into ptrs: no reallocation
@@ -1121,6 +1241,15 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
     kp.push_back(&ient);
     kp.push_back(&irows);
   }
+  void *ticket = j.parts_d, *parts = red ? (char *)j.parts_d + 16 : nullptr;
+  void *page = (char *)r.pinned_dev + kRedPageOffset;
+  unsigned long long seq = red ? (unsigned long long)++r.red_seq : 0;
+  if (red) {
+    kp.push_back(&ticket);
+    kp.push_back(&parts);
+    kp.push_back(&page);
+    kp.push_back(&seq);
+  }
   r.begin_loop(name);
   // one launch over the set, or one per colour over its slice of col_reord
   const int ncol = plan ? plan->pub.ncolors : 1;
@@ -1155,7 +1284,20 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   bool reduce = false;
   for (auto &a : ap) reduce |= a.kind == GBL && a.acc != OP_READ && a.acc != OP_WORK;
   if (!reduce) return 0;
-  if (!cuda_ok(cudaMemcpyAsync(gh.data(), j.gbl_d, gbytes, cudaMemcpyDeviceToHost, r.stream),
+  if (red) {
+    if (n == 0) return 0;
+    if (!wait_for_entries((const char *)r.pinned + kRedPageOffset, red, seq, name)) return -1;
+    const char *src = (const char *)r.pinned + kRedPageOffset;
+    gh.assign((size_t)red * 8, 0);
+    size_t at = 0;
+    for (int i = 0; i < nargs; i++) {
+      const ArgPlan &a = ap[(size_t)i];
+      if (!is_red(a)) continue;
+      goff[(size_t)i] = at;
+      for (int k = 0; k < a.dim; k++, src += 8, at += (size_t)a.bytes)
+        memcpy(gh.data() + at, src, (size_t)a.bytes);
+    }
+  } else if (!cuda_ok(cudaMemcpyAsync(gh.data(), j.gbl_d, gbytes, cudaMemcpyDeviceToHost, r.stream),
                "op_par_loop: globals") ||
       !cuda_ok(cudaStreamSynchronize(r.stream), "op_par_loop: globals"))
     return -1;

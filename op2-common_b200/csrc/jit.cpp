@@ -201,6 +201,16 @@ unsigned long long red_mix(unsigned long long h, unsigned long long x) {
   return h ^ (h >> 29);
 }
 
+// The colours of one launch (as the generated source declares it).  A coloured loop of up to
+// kClusterElements elements runs all its colours in one launch of one cluster of
+// up to eight CTAs: boundary loops of a few thousand elements, whose colours
+// took a launch of about 2.5 us each.
+struct Colours {
+  int n;
+  int at[33];
+};
+constexpr int kClusterElements = 16384;
+
 struct Jit {
   void *parts_d = nullptr;  // ticket (16 bytes), then the blocks' entries
   cudaLibrary_t lib = nullptr;
@@ -248,6 +258,7 @@ template <typename T> struct op2b_vec {
   __device__ operator const T **() const { return (const T **)p; }
   __device__ operator const T *const *() const { return p; }
 };
+struct op2b_colours { int n; int at[33]; };
 __device__ void op2b_amin(double *a, double v) {
   unsigned long long *p = (unsigned long long *)a, old = *p, as;
   do { as = old; if (__longlong_as_double((long long)as) <= v) return;
@@ -307,8 +318,9 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
       s << ", double *op2b_iv" << i << ", long long *op2b_ix" << i << ", " << a.ctype
         << " *op2b_ip" << i << ", const " << a.ctype << " *op2b_ic" << i;
   }
-  // coloured: this launch runs the elements op2b_perm[op2b_first, +op2b_n)
-  if (coloured) s << ", const int *op2b_perm, int op2b_first";
+  // coloured: this launch runs op2b_c.n colours one after the other, colour k
+  // the elements op2b_perm[op2b_c.at[k], op2b_c.at[k + 1])
+  if (coloured) s << ", const int *op2b_perm, op2b_colours op2b_c";
   // owner computes: op2b_n targets, each with its (element, slot) entries
   if (own >= 0) s << ", const long long *op2b_ioff, const int *op2b_ient, const int *op2b_rows";
   // block reductions: ticket and partials, the mapped result, the call's number
@@ -389,9 +401,14 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
       }
     }
   } else if (coloured) {
-    s << "  for (int op2b_i = blockIdx.x * blockDim.x + threadIdx.x; op2b_i < op2b_n;"
-         " op2b_i += gridDim.x * blockDim.x) {\n"
-         "    const int op2b_e = op2b_perm[op2b_first + op2b_i];\n";
+    // (several colours a launch: the launch is one cluster, whose barrier
+    // orders a colour's writes before the next colour's reads)
+    s << "  for (int op2b_k = 0; op2b_k < op2b_c.n; op2b_k++) {\n"
+         "  if (op2b_k) asm volatile(\"barrier.cluster.arrive.release;\\n\\t"
+         "barrier.cluster.wait.acquire;\" ::: \"memory\");\n"
+         "  for (int op2b_i = op2b_c.at[op2b_k] + blockIdx.x * blockDim.x + threadIdx.x;"
+         " op2b_i < op2b_c.at[op2b_k + 1]; op2b_i += gridDim.x * blockDim.x) {\n"
+         "    const int op2b_e = op2b_perm[op2b_i];\n";
   } else {
     s << "  for (int op2b_e = blockIdx.x * blockDim.x + threadIdx.x; op2b_e < op2b_n;"
          " op2b_e += gridDim.x * blockDim.x) {\n";
@@ -593,6 +610,7 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
     }
   }
   s << "  }\n";
+  if (coloured) s << "  }\n";
   for (size_t i = 0; i < ap.size(); i++) {
     const ArgPlan &a = ap[i];
     if (a.kind != INFO) continue;
@@ -1252,27 +1270,52 @@ int jit_par_loop(const char *name, op_set set, int nargs, op_arg *args) {
   }
   r.begin_loop(name);
   // one launch over the set, or one per colour over its slice of col_reord
+  // (or all colours of a small set in one cluster)
   const int ncol = plan ? plan->pub.ncolors : 1;
   const int *perm = plan ? plan->col_reord_d : nullptr;
-  int first = 0;
+  Colours span{1, {0}};
   if (plan) {
     kp.push_back(&perm);
-    kp.push_back(&first);
+    kp.push_back(&span);
   }
+  const bool one = plan && ncol > 1 && ncol <= 32 && set->size <= kClusterElements;
   unsigned grid = 0;  // of the last launch (a loop with op_arg_info has one)
-  for (int c = 0; c < ncol && set->size > 0 && n > 0; c++) {
+  for (int c = 0; c < (one ? 1 : ncol) && set->size > 0 && n > 0; c++) {
     if (plan) {
-      first = plan->pub.color2_offsets[c];
-      n = plan->pub.color2_offsets[c + 1] - first;
+      const int *at = plan->pub.color2_offsets;
+      span.n = one ? ncol : 1;
+      n = 0;
+      for (int k = 0; k <= span.n; k++) {
+        span.at[k] = at[c + k];
+        if (k) n = std::max(n, at[c + k] - at[c + k - 1]);
+      }
     }
     if (n <= 0) continue;
     // a thread per element, unless per-block reduction partials bound the
-    // grid (op_arg_info) or the global reductions' atomics should stay few
+    // grid (op_arg_info, the block reductions: 32 CTAs an SM took 33 us for 8's 29) or the atomics
+    // should stay few
     grid = (unsigned)std::min<long long>(((long long)n + 255) / 256,
                                          has_red ? max_grid : (long long)INT32_MAX);
-    if (!cuda_ok(cudaLaunchKernel((const void *)j.fn, dim3(grid), dim3(256), kp.data(), 0,
-                                  r.stream),
-                 "op_par_loop: launch")) {
+    cudaError_t e;
+    if (one) {
+      unsigned cl = 1;  // a power of two, at most the portable eight
+      while (cl < 8 && cl < grid) cl *= 2;
+      grid = cl;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(grid);
+      cfg.blockDim = dim3(256);
+      cfg.stream = r.stream;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cl;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      e = cudaLaunchKernelExC(&cfg, (const void *)j.fn, kp.data());
+    } else {
+      e = cudaLaunchKernel((const void *)j.fn, dim3(grid), dim3(256), kp.data(), 0, r.stream);
+    }
+    if (!cuda_ok(e, "op_par_loop: launch")) {
       r.end_loop(bytes);
       return -1;
     }

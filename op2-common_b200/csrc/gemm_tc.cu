@@ -54,7 +54,7 @@ struct GemmArgs {
   int epi;
   int k_per_split;
   int *err;
-  int staged;  // k_gemm_ws<16>: C (and Z) 16-byte aligned rows: stores through shared memory
+  int staged;  // k_gemm_ws<16>: C (and Z) 16-byte aligned rows: stored by TMA
 };
 
 // bias[col .. col + n) into v (16-byte loads when aligned)
@@ -524,118 +524,70 @@ __device__ __forceinline__ WsTile ws_tile(const GemmArgs &g, int t, int mtiles, 
   return w;
 }
 
-// The persistent kernel's epilogue through shared memory (16 epilogue warps,
-// 32 rows x 32 columns a warp a tile, taken in two halves of 16 columns).
-// Each lane computes its row's values with the arithmetic of epilogue16 and
-// writes them into the warp's staging rows (padded: 16-byte accesses free of
-// bank conflicts); the warp then stores whole row segments -- four lanes a
-// 64-byte BF16 row, eight a 128-byte FP32 row -- instead of each lane its own
-// row 16 bytes at a time.  Two staging areas: C, and Z for bias + SiLU.
-// Z's BF16 rows follow C's BF16 rows; FP32 rows of C (no Z) take the space of both.
-constexpr int kEpiRowF32 = 32 * 4 + 16, kEpiRowBf16 = 32 * 2 + 16;
-constexpr int kEpiAreaBytes = 32 * kEpiRowBf16;  // offset of Z's area
-constexpr int kEpiStageBytes =
-    32 * kEpiRowF32 > 2 * kEpiAreaBytes ? 32 * kEpiRowF32 : 2 * kEpiAreaBytes;  // per warp
+// The persistent kernel's epilogue by TMA (16 epilogue warps, 32 rows x 32
+// columns a warp a tile): each lane computes its row's values with the
+// arithmetic of epilogue16, and the warp's block leaves through 2 KiB of shared
+// memory an output (two, C and Z for bias + SiLU).  A lane's own row segments
+// cost an L1 cycle a row and instruction, and rows gathered by the warp's own
+// loads and stores still a round trip through its registers.
+constexpr int kEpiStageBytes = 2 * kOutBytes;  // per warp
 
-__device__ __forceinline__ void stage_bf16x16(uint8_t *area, int lane, int h, const float *v) {
-#pragma unroll
-  for (int j = 0; j < 2; j++) {
-    uint4 w;
-    __nv_bfloat162 *p = reinterpret_cast<__nv_bfloat162 *>(&w);
-#pragma unroll
-    for (int i = 0; i < 4; i++) p[i] = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
-    *reinterpret_cast<uint4 *>(area + lane * kEpiRowBf16 + h * 32 + j * 16) = w;
+__device__ __forceinline__ void epilogue_tma(const GemmArgs &g, uint8_t *stage, int lane, int row,
+                                             int y, int col, int n, const CUtensorMap *tc,
+                                             const CUtensorMap *tz, float (&v)[32]) {
+  const bool live = row < g.M, inside = y < g.M;
+  const int n0 = min(16, n), n1 = min(16, n - 16);
+  uint32_t p[16];
+  if (g.epi == OP2B_EPI_STORE_F32 || g.epi == OP2B_EPI_BIAS_BF16 ||
+      g.epi == OP2B_EPI_BIAS_SILU_BF16) {
+    if (g.bias) {
+      add_bias16(v, g.bias, col, n0);
+      if (n1 > 0) add_bias16(v + 16, g.bias, col + 16, n1);
+    }
   }
-}
-
-__device__ __forceinline__ void stage_f32x16(uint8_t *area, int lane, int h, const float *v) {
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    *reinterpret_cast<float4 *>(area + lane * kEpiRowF32 + h * 64 + j * 16) =
-        make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-}
-
-__device__ __forceinline__ void store_rows_bf16(const uint8_t *area, int lane, int ncols,
-                                                __nv_bfloat16 *dst, long ld, int row0, int col0,
-                                                int M) {
-  const int seg = lane & 3;
-#pragma unroll
-  for (int pass = 0; pass < 4; pass++) {
-    const int r = pass * 8 + (lane >> 2);
-    if (row0 + r < M && seg * 8 < ncols)
-      *reinterpret_cast<uint4 *>(dst + (long)(row0 + r) * ld + col0 + seg * 8) =
-          *reinterpret_cast<const uint4 *>(area + r * kEpiRowBf16 + seg * 16);
-  }
-}
-
-__device__ __forceinline__ void store_rows_f32(const uint8_t *area, int lane, int ncols,
-                                               float *dst, long ld, int row0, int col0, int M) {
-  const int seg = lane & 7;
-#pragma unroll
-  for (int pass = 0; pass < 8; pass++) {
-    const int r = pass * 4 + (lane >> 3);
-    if (row0 + r < M && seg * 4 < ncols)
-      *reinterpret_cast<float4 *>(dst + (long)(row0 + r) * ld + col0 + seg * 4) =
-          *reinterpret_cast<const float4 *>(area + r * kEpiRowF32 + seg * 16);
-  }
-}
-
-// half h (columns col0 + 16h ..) of the lane's row into the staging areas
-__device__ __forceinline__ void epilogue_half(const GemmArgs &g, uint8_t *stage, int lane,
-                                              int row, int col, int n, int h, float *v) {
-  uint8_t *areaC = stage, *areaZ = stage + kEpiAreaBytes;
-  const bool live = row < g.M;
-  switch (g.epi) {
-    case OP2B_EPI_STORE_F32:
-      if (g.bias && n > 0) add_bias16(v, g.bias, col, n);
-      stage_f32x16(areaC, lane, h, v);
-      return;
-    case OP2B_EPI_BIAS_BF16:
-      if (g.bias && n > 0) add_bias16(v, g.bias, col, n);
-      if (g.R && live && n > 0) {
-        float rr[16];
-        load_bf16x16(g.R + (long)row * g.ldr + col, rr, n);
-        FOR_LT_N(i) v[i] += rr[i];
-      }
-      stage_bf16x16(areaC, lane, h, v);
-      return;
-    case OP2B_EPI_BIAS_SILU_BF16:
-      if (g.bias && n > 0) add_bias16(v, g.bias, col, n);
-      stage_bf16x16(areaZ, lane, h, v);
-#pragma unroll
-      for (int i = 0; i < 16; i++) v[i] = silu(v[i]);
-      stage_bf16x16(areaC, lane, h, v);
-      return;
-    case OP2B_EPI_SILU_GRAD_BF16:
-      if (live && n > 0) {
-        float z[16];
-        load_bf16x16(g.R + (long)row * g.ldr + col, z, n);
-        FOR_LT_N(i) v[i] *= silu_grad(z[i]);
-      }
-      stage_bf16x16(areaC, lane, h, v);
-      return;
-    default:
-      stage_bf16x16(areaC, lane, h, v);
-  }
-}
-
-// the staged rows of the warp out to C (and Z)
-__device__ __forceinline__ void epilogue_store(const GemmArgs &g, const uint8_t *stage, int lane,
-                                               int row0, int col0, int ncols) {
   if (g.epi == OP2B_EPI_STORE_F32) {
-    store_rows_f32(stage, lane, ncols, reinterpret_cast<float *>(g.C), g.ldc, row0, col0, g.M);
+    put_rows(stage, lane, tc, col, y, inside, reinterpret_cast<const uint32_t *>(v), false);
+    if (n1 > 0)
+      put_rows(stage + kOutBytes, lane, tc, col + 16, y, inside,
+               reinterpret_cast<const uint32_t *>(v + 16), false);
     return;
   }
-  if (g.epi == OP2B_EPI_BIAS_SILU_BF16 && g.Z)
-    store_rows_bf16(stage + kEpiAreaBytes, lane, ncols, g.Z, g.ldc, row0, col0, g.M);
-  store_rows_bf16(stage, lane, ncols, reinterpret_cast<__nv_bfloat16 *>(g.C), g.ldc, row0, col0,
-                  g.M);
+  if (g.epi == OP2B_EPI_BIAS_SILU_BF16) {
+    if (g.Z) {
+      pack16(v, p);
+      pack16(v + 16, p + 8);
+      put_rows(stage + kOutBytes, lane, tz, col, y, inside, p, false);
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = silu(v[i]);
+  } else if (g.R && live && (g.epi == OP2B_EPI_BIAS_BF16 || g.epi == OP2B_EPI_SILU_GRAD_BF16)) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int nh = h ? n1 : n0;
+      if (nh <= 0) break;
+      float rr[16], *u = v + 16 * h;
+      load_bf16x16(g.R + (long)row * g.ldr + col + 16 * h, rr, nh);
+      if (g.epi == OP2B_EPI_BIAS_BF16) {
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+          if (i < nh) u[i] += rr[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+          if (i < nh) u[i] *= silu_grad(rr[i]);
+      }
+    }
+  }
+  pack16(v, p);
+  pack16(v + 16, p + 8);
+  put_rows(stage, lane, tc, col, y, inside, p, false);
 }
 
 template <int EW, bool AMN, bool BMN>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
-          const __grid_constant__ CUtensorMap tb, int mtiles, int ntiles, int ntotal) {
+          const __grid_constant__ CUtensorMap tb, const __grid_constant__ CUtensorMap tc,
+          const __grid_constant__ CUtensorMap tz, int mtiles, int ntiles, int ntotal) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // full[kWsStages], empty[kWsStages], acc_full[2], acc_empty[2], done
   __shared__ __align__(8) uint64_t bars[2 * kWsStages + 5];
@@ -784,40 +736,22 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b)) : "memory");
         continue;
       }
-      if (EW == 16 && g.staged) {  // 32 columns: the row-coalesced epilogue
-        // the warp's columns of the matrix (nt is rounded up to 16; N is not)
-        const int nv = min(ce, g.N - w.n0) - c0;
-#pragma unroll 1
-        for (int h = 0; h < 2; h++) {
-          uint32_t r[16];
+      if (EW == 16 && g.staged) {  // 32 columns, out by TMA
+        float v[32];
+        if (w.nk > 0) {
+          tmem_ld32(src + (uint32_t)c0, v);
+        } else {
 #pragma unroll
-          for (int k = 0; k < 16; k++) r[k] = 0u;
-          if (w.nk > 0 && c0 + 16 * h < ce) {
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                  "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                  "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                : "r"(src + (uint32_t)(c0 + 16 * h)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          }
-          if (h == 1) {  // the warp's part has been read: the MMAs may reuse it
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b))
-                           : "memory");
-          }
-          float v[16];
-#pragma unroll
-          for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
-          epilogue_half(g, epi_stage, lane, row, w.n0 + c0 + 16 * h,
-                        min(16, nv - 16 * h), h, v);
+          for (int k = 0; k < 32; k++) v[k] = 0.0f;
         }
+        // the warp's part has been read: the MMAs may reuse it
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        epilogue_store(g, epi_stage, lane, w.m0 + quarter * 32, w.n0 + c0, nv);
-        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b)) : "memory");
+        // (columns past N, and accumulator columns past the tile's nt, are clipped)
+        epilogue_tma(g, epi_stage, lane, row, w.m0 + quarter * 32, w.n0 + c0,
+                     min(kCols, g.N - w.n0 - c0), &tc, &tz, v);
         continue;
       }
       for (int cc = c0; cc < ce; cc += 16) {
@@ -845,6 +779,7 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
         if (row < g.M) epilogue16(g, row, w.n0 + cc, r);
       }
     }
+    if (EW == 16 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   // every issued MMA has finished once "done" has arrived; loads the MMA
@@ -935,7 +870,8 @@ bool operand_map_mn(CUtensorMap *m, const void *base, int mn, int K, long ld) {
 
 template <int EW, bool AMN, bool BMN>
 cudaError_t launch_ws(const GemmArgs &g, const CUtensorMap &ta, const CUtensorMap &tb,
-                      dim3 grid, int nsm, cudaStream_t s) {
+                      const CUtensorMap &tc, const CUtensorMap &tz, dim3 grid, int nsm,
+                      cudaStream_t s) {
   const size_t smem_w =
       (size_t)kWsStages * 2 * kStageBytes + (EW == 16 ? 16 * kEpiStageBytes : 0) + 1024;
   static bool attr[16] = {};  // per device, once
@@ -950,7 +886,7 @@ cudaError_t launch_ws(const GemmArgs &g, const CUtensorMap &ta, const CUtensorMa
   }
   const long long total = (long long)grid.x * grid.y * grid.z;
   const int ctas = (int)std::min<long long>(total, nsm > 0 ? nsm : 148);
-  k_gemm_ws<EW, AMN, BMN><<<ctas, 64 + 32 * EW, smem_w, s>>>(g, ta, tb, (int)grid.x,
+  k_gemm_ws<EW, AMN, BMN><<<ctas, 64 + 32 * EW, smem_w, s>>>(g, ta, tb, tc, tz, (int)grid.x,
                                                              (int)grid.y, (int)total);
   return cudaGetLastError();
 }
@@ -1082,11 +1018,15 @@ extern "C" int op2b_gemm_bf16(int M, int N, int K, const void *A, long a_m, long
       if (ws) {
         int nsm = 0;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (a_mn && b_mn) e = launch_ws<16, true, true>(g, ta, tb, grid, nsm, s);
-        else if (a_mn) e = launch_ws<16, true, false>(g, ta, tb, grid, nsm, s);
-        else if (b_mn) e = launch_ws<16, false, true>(g, ta, tb, grid, nsm, s);
-        else if (rt().opt_gemm_ws == 2) e = launch_ws<16, false, false>(g, ta, tb, grid, nsm, s);
-        else e = launch_ws<8, false, false>(g, ta, tb, grid, nsm, s);
+        CUtensorMap tc{}, tz{};
+        if (g.staged)
+          g.staged = tc_store_map(&tc, C, epi == OP2B_EPI_STORE_F32, N, M, ldc) &&
+                     (!Z || tc_store_map(&tz, Z, false, N, M, ldc));
+        if (a_mn && b_mn) e = launch_ws<16, true, true>(g, ta, tb, tc, tz, grid, nsm, s);
+        else if (a_mn) e = launch_ws<16, true, false>(g, ta, tb, tc, tz, grid, nsm, s);
+        else if (b_mn) e = launch_ws<16, false, true>(g, ta, tb, tc, tz, grid, nsm, s);
+        else if (rt().opt_gemm_ws == 2) e = launch_ws<16, false, false>(g, ta, tb, tc, tz, grid, nsm, s);
+        else e = launch_ws<8, false, false>(g, ta, tb, tc, tz, grid, nsm, s);
       } else {
         const size_t smem_t = (size_t)kTmaStages * 2 * kStageBytes + 1024;
         static bool attr_t[16] = {};

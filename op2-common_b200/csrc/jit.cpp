@@ -1427,6 +1427,9 @@ int op2b_register_kernel(const char *name, const char *source) {
   }
   std::string n(name);
   if (n.size() < 2 || n.compare(n.size() - 2, 2, ".h") != 0) n += ".h";
+  auto it = op2b::sources().kernels.find(n);
+  if (it != op2b::sources().kernels.end() ? source && it->second == source : !source)
+    return 0;  // as it was: what is compiled stands
   if (source) op2b::sources().kernels[n] = source;
   else op2b::sources().kernels.erase(n);  // forget it
   op2b::sources().version++;

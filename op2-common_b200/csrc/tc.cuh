@@ -154,5 +154,64 @@ __device__ __forceinline__ bool mbar_wait_or_fail(uint32_t bar, uint32_t parity,
   return true;
 }
 
+// 32 columns of the lane's row
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, float *v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 floats to 16 BF16 (element 2i in the low half of word i)
+__device__ __forceinline__ void pack16(const float *v, uint32_t *r) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    r[i] = *reinterpret_cast<const uint32_t *>(&t);
+  }
+}
+
+// A warp's 32 rows x 64 bytes out to global memory by TMA: 16 words of each
+// lane's row, to column x (in elements of the map) of the rows from y on.  `out`:
+// the warp's 2 KiB of shared memory, in the 64-byte swizzle; rows past the
+// matrix are clipped.  `add`: an FP32 reduction instead of a store.
+constexpr int kOutBytes = 32 * 64;
+__device__ __forceinline__ void put_rows(uint8_t *out, int lane, const CUtensorMap *m, int x, int y,
+                                         bool inside, const uint32_t *v, bool add) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    *reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+        make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0 && inside) {
+    if (add)
+      asm volatile(
+          "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group "
+          "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+          "r"(x), "r"(y), "r"(smem_u32(out))
+          : "memory");
+    else
+      asm volatile(
+          "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group "
+          "[%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(m)),
+          "r"(x), "r"(y), "r"(smem_u32(out))
+          : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+
 }  // namespace
 }  // namespace op2b

@@ -55,6 +55,7 @@ struct GemmArgs {
   int k_per_split;
   int *err;
   int staged;  // k_gemm_ws<16>: C (and Z) 16-byte aligned rows: stored by TMA
+  int r_tma;   // and R's rows too: fetched by TMA, through the map of Z
 };
 
 // bias[col .. col + n) into v (16-byte loads when aligned)
@@ -504,7 +505,7 @@ k_gemm_tma(GemmArgs g, const __grid_constant__ CUtensorMap ta,
 // also ends when another role has recorded a failure; on failure the CTA
 // waits (bounded) for its issued loads and MMAs, frees tensor memory and
 // returns.
-constexpr int kWsStages = 4;
+constexpr int kWsStages = 5;
 
 struct WsTile {
   int m0, n0, nt, kb, nk;
@@ -525,62 +526,90 @@ __device__ __forceinline__ WsTile ws_tile(const GemmArgs &g, int t, int mtiles, 
 }
 
 // The persistent kernel's epilogue by TMA (16 epilogue warps, 32 rows x 32
-// columns a warp a tile): each lane computes its row's values with the
-// arithmetic of epilogue16, and the warp's block leaves through 2 KiB of shared
-// memory an output (two, C and Z for bias + SiLU).  A lane's own row segments
-// cost an L1 cycle a row and instruction, and rows gathered by the warp's own
-// loads and stores still a round trip through its registers.
+// columns a warp a tile, 16 columns at a time): each lane computes its row's
+// values with the arithmetic of epilogue16 and puts them into the warp's 2 KiB
+// of shared memory an output (C, and Z for bias + SiLU or C's second 16 columns
+// in FP32; in the 64-byte swizzle), which leave by TMA.  A lane's own row
+// segments cost an L1 cycle a row and instruction, and rows gathered by the
+// warp's own loads and stores still a round trip through its registers.
+// `r_in`: the block of R that TMA brought into the second 2 KiB (null: R from
+// memory).
 constexpr int kEpiStageBytes = 2 * kOutBytes;  // per warp
 
-__device__ __forceinline__ void epilogue_tma(const GemmArgs &g, uint8_t *stage, int lane, int row,
-                                             int y, int col, int n, const CUtensorMap *tc,
-                                             const CUtensorMap *tz, float (&v)[32]) {
-  const bool live = row < g.M, inside = y < g.M;
-  const int n0 = min(16, n), n1 = min(16, n - 16);
-  uint32_t p[16];
-  if (g.epi == OP2B_EPI_STORE_F32 || g.epi == OP2B_EPI_BIAS_BF16 ||
-      g.epi == OP2B_EPI_BIAS_SILU_BF16) {
-    if (g.bias) {
-      add_bias16(v, g.bias, col, n0);
-      if (n1 > 0) add_bias16(v + 16, g.bias, col + 16, n1);
-    }
-  }
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint4 *out_chunk(uint8_t *out, int lane, int i) {
+  return reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
+}
+
+__device__ __forceinline__ void put_bf16x16(uint8_t *out, int lane, int h, const float *v) {
+  uint32_t p[8];
+  pack16(v, p);
+  *out_chunk(out, lane, 2 * h) = make_uint4(p[0], p[1], p[2], p[3]);
+  *out_chunk(out, lane, 2 * h + 1) = make_uint4(p[4], p[5], p[6], p[7]);
+}
+
+// columns col .. col + 16 (n of them inside the matrix), half h of the warp's 32
+__device__ __forceinline__ void epilogue_half(const GemmArgs &g, uint8_t *stage, int lane, int row,
+                                              int col, int n, int h, uint8_t *r_in,
+                                              float (&v)[16]) {
+  if (g.bias && (g.epi == OP2B_EPI_STORE_F32 || g.epi == OP2B_EPI_BIAS_BF16 ||
+                 g.epi == OP2B_EPI_BIAS_SILU_BF16))
+    add_bias16(v, g.bias, col, n);
   if (g.epi == OP2B_EPI_STORE_F32) {
-    put_rows(stage, lane, tc, col, y, inside, reinterpret_cast<const uint32_t *>(v), false);
-    if (n1 > 0)
-      put_rows(stage + kOutBytes, lane, tc, col + 16, y, inside,
-               reinterpret_cast<const uint32_t *>(v + 16), false);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *out_chunk(stage + h * kOutBytes, lane, i) =
+          make_uint4(__float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]),
+                     __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
     return;
   }
   if (g.epi == OP2B_EPI_BIAS_SILU_BF16) {
-    if (g.Z) {
-      pack16(v, p);
-      pack16(v + 16, p + 8);
-      put_rows(stage + kOutBytes, lane, tz, col, y, inside, p, false);
-    }
+    if (g.Z) put_bf16x16(stage + kOutBytes, lane, h, v);
 #pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = silu(v[i]);
-  } else if (g.R && live && (g.epi == OP2B_EPI_BIAS_BF16 || g.epi == OP2B_EPI_SILU_GRAD_BF16)) {
+    for (int i = 0; i < 16; i++) v[i] = silu(v[i]);
+  } else if (g.R && row < g.M) {
+    float rr[16];
+    if (r_in) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int nh = h ? n1 : n0;
-      if (nh <= 0) break;
-      float rr[16], *u = v + 16 * h;
-      load_bf16x16(g.R + (long)row * g.ldr + col + 16 * h, rr, nh);
-      if (g.epi == OP2B_EPI_BIAS_BF16) {
+      for (int j = 0; j < 2; j++) {
+        const uint4 q = *out_chunk(r_in, lane, 2 * h + j);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-          if (i < nh) u[i] += rr[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-          if (i < nh) u[i] *= silu_grad(rr[i]);
+        for (int i = 0; i < 4; i++) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[i]));
+          rr[8 * j + 2 * i] = f.x;
+          rr[8 * j + 2 * i + 1] = f.y;
+        }
       }
+    } else {
+      load_bf16x16(g.R + (long)row * g.ldr + col, rr, n);
+    }
+    if (g.epi == OP2B_EPI_BIAS_BF16) {
+      FOR_LT_N(i) v[i] += rr[i];
+    } else {
+      FOR_LT_N(i) v[i] *= silu_grad(rr[i]);
     }
   }
-  pack16(v, p);
-  pack16(v + 16, p + 8);
-  put_rows(stage, lane, tc, col, y, inside, p, false);
+  put_bf16x16(stage, lane, h, v);
+}
+
+__device__ __forceinline__ void store_block(const CUtensorMap *m, const uint8_t *out, int x,
+                                            int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+          reinterpret_cast<uint64_t>(m)),
+      "r"(x), "r"(y), "r"(smem_u32(out))
+      : "memory");
 }
 
 template <int EW, bool AMN, bool BMN>
@@ -589,8 +618,8 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
           const __grid_constant__ CUtensorMap tb, const __grid_constant__ CUtensorMap tc,
           const __grid_constant__ CUtensorMap tz, int mtiles, int ntiles, int ntotal) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // full[kWsStages], empty[kWsStages], acc_full[2], acc_empty[2], done
-  __shared__ __align__(8) uint64_t bars[2 * kWsStages + 5];
+  // full[kWsStages], empty[kWsStages], acc_full[2], acc_empty[2], done, R's[EW]
+  __shared__ __align__(8) uint64_t bars[2 * kWsStages + 5 + EW];
   __shared__ uint32_t s_taddr;
   __shared__ int s_fail, s_loaded, s_mma;
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -614,6 +643,7 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
       mbar_init(acc_empty(b), EW);
     }
     mbar_init(done, 1);
+    for (int e = 0; e < EW; e++) mbar_init(done + 8 + 8 * e, 1);
     s_fail = 0;
     s_loaded = 0;
     s_mma = 0;
@@ -716,6 +746,22 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
     const int c0 = ((warp - 2) >> 2) * kCols;
     // the warp's staging rows, after the operand ring (EW == 16 only)
     uint8_t *epi_stage = smem + (size_t)kWsStages * 2 * kStageBytes + (warp - 2) * kEpiStageBytes;
+    // the warp's block of R of its next tile, on its way while the tile's MMAs
+    // run (200,001 x 128 x 384 with bias and residual 60.5 -> RES1 us: a lane's own
+    // 32-byte pieces of a row waited for memory in every tile)
+    const uint32_t r_bar = done + 8 + 8 * (warp - 2);
+    int r_sent = 0, r_used = 0;
+    auto fetch_r = [&](int t) {
+      if (EW != 16 || !g.r_tma || t >= ntotal) return;
+      const WsTile w = ws_tile(g, t, mtiles, ntiles);
+      if (c0 >= w.nt) return;
+      if (lane == 0) {
+        mbar_expect_tx(r_bar, kOutBytes);
+        tma_load_2d(smem_u32(epi_stage + kOutBytes), &tz, w.n0 + c0, w.m0 + quarter * 32, r_bar);
+      }
+      r_sent++;
+    };
+    fetch_r(blockIdx.x);
     int i = 0;
     for (int t = blockIdx.x; t < ntotal; t += gridDim.x, i++) {
       const WsTile w = ws_tile(g, t, mtiles, ntiles);
@@ -734,37 +780,59 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
         __syncwarp();
         if (lane == 0)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b)) : "memory");
+        fetch_r(t + gridDim.x);
         continue;
       }
       if (EW == 16 && g.staged) {  // 32 columns, out by TMA
-        float v[32];
-        if (w.nk > 0) {
-          tmem_ld32(src + (uint32_t)c0, v);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 32; k++) v[k] = 0.0f;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        ok = true;
+        if (r_sent > r_used) {
+          ok = mbar_wait_or_fail(r_bar, (uint32_t)(r_used & 1), fail);
+          if (ok) r_used++;
         }
-        // the warp's part has been read: the MMAs may reuse it
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        ok = __all_sync(0xffffffffu, ok);  // (and the stores have read the staging memory)
+        if (!ok) {
+          if (lane == 0) atomicExch(&s_fail, 1);
+          break;
+        }
+        const int col = w.n0 + c0, nc = min(kCols, g.N - col), y = w.m0 + quarter * 32;
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+          uint32_t r[16] = {};
+          if (w.nk > 0) tmem_ld16(src + (uint32_t)(c0 + 16 * h), r);
+          float v[16];
+#pragma unroll
+          for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
+          if (h) {  // the warp's part has been read: the MMAs may reuse it
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b))
+                           : "memory");
+          }
+          // (accumulator columns past the tile's nt are read and clipped)
+          if (16 * h < nc)
+            epilogue_half(g, epi_stage, lane, row, col + 16 * h, min(16, nc - 16 * h), h,
+                          g.r_tma ? epi_stage + kOutBytes : nullptr, v);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty(b)) : "memory");
-        // (columns past N, and accumulator columns past the tile's nt, are clipped)
-        epilogue_tma(g, epi_stage, lane, row, w.m0 + quarter * 32, w.n0 + c0,
-                     min(kCols, g.N - w.n0 - c0), &tc, &tz, v);
+        if (lane == 0 && y < g.M) {
+          store_block(&tc, epi_stage, col, y);
+          if (g.epi == OP2B_EPI_STORE_F32) {
+            if (nc > 16) store_block(&tc, epi_stage + kOutBytes, col + 16, y);
+          } else if (g.epi == OP2B_EPI_BIAS_SILU_BF16 && g.Z) {
+            store_block(&tz, epi_stage + kOutBytes, col, y);
+          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        fetch_r(t + gridDim.x);  // (every lane has read R)
         continue;
       }
       for (int cc = c0; cc < ce; cc += 16) {
         uint32_t r[16];
         if (w.nk > 0) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-              "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(src + (uint32_t)cc));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          tmem_ld16(src + (uint32_t)cc, r);
         } else {
 #pragma unroll
           for (int k = 0; k < 16; k++) r[k] = 0u;
@@ -779,6 +847,7 @@ k_gemm_ws(GemmArgs g, const __grid_constant__ CUtensorMap ta,
         if (row < g.M) epilogue16(g, row, w.n0 + cc, r);
       }
     }
+    if (r_sent > r_used && !mbar_wait(r_bar, (uint32_t)(r_used & 1))) s_fail = 1;
     if (EW == 16 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
@@ -1022,6 +1091,10 @@ extern "C" int op2b_gemm_bf16(int M, int N, int K, const void *A, long a_m, long
         if (g.staged)
           g.staged = tc_store_map(&tc, C, epi == OP2B_EPI_STORE_F32, N, M, ldc) &&
                      (!Z || tc_store_map(&tz, Z, false, N, M, ldc));
+        g.r_tma = g.staged && R && !Z && ldr >= N &&
+                  (epi == OP2B_EPI_BIAS_BF16 || epi == OP2B_EPI_SILU_GRAD_BF16) &&
+                  (reinterpret_cast<uintptr_t>(R) & 15) == 0 && ldr % 8 == 0 &&
+                  tc_store_map(&tz, const_cast<void *>(R), false, N, M, ldr);
         if (a_mn && b_mn) e = launch_ws<16, true, true>(g, ta, tb, tc, tz, grid, nsm, s);
         else if (a_mn) e = launch_ws<16, true, false>(g, ta, tb, tc, tz, grid, nsm, s);
         else if (b_mn) e = launch_ws<16, false, true>(g, ta, tb, tc, tz, grid, nsm, s);

@@ -120,11 +120,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t *r) {
 }
 
 // one 32-byte sector of a lane's row
-__device__ __forceinline__ void st_sector(void *p, const uint32_t *r) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
 __device__ __forceinline__ void ld_sector(const void *p, uint32_t *r) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
@@ -153,23 +148,34 @@ __device__ __forceinline__ void load_weights(uint32_t dst, const __nv_bfloat16 *
   }
 }
 
-// Input stages of 128 rows x 64 columns.  With the hidden layers kept, two of
-// the four give way to the epilogue warps' 2 KiB each, from which Z, A and y leave
-// by TMA (a lane's own row segments would cost an L1 cycle a row and
-// instruction); without, only y is written, and the deeper ring is worth more.
-__host__ __device__ constexpr int mlp_ring(bool store) { return store ? 2 : 4; }
+// Input stages of 128 rows x 64 columns: as many of four as the weights and the
+// epilogue warps' staging leave room for.  The results leave by TMA from 2 KiB a
+// warp, blocks of 32 columns (a lane's own row segments cost an L1 cycle a row and
+// instruction), or from 1 KiB, blocks of 16, where only y is written and a third
+// stage is to be had that way: 458,396 rows of the edge MLP took 172 us with four
+// stages and y stored by the lanes, 162 with two and 2 KiB, 158 with three and 1 KiB.
+// (The row gathers as TMA gathers of four rows: 222 us, 2.4K cycles a stage.)
+__host__ __device__ constexpr bool mlp_narrow(int nc, bool store) { return nc == 6 && !store; }
+__host__ __device__ constexpr int mlp_ring(int nc, bool store) {
+  return nc < 6 ? 4 : mlp_narrow(nc, store) ? 3 : 2;
+}
+__host__ __device__ constexpr int mlp_out(int nc, bool store) {
+  return mlp_narrow(nc, store) ? kOutBytes / 2 : kOutBytes;
+}
 
 // NC: 64-column blocks of the input (1, 2, 4 or 6); STORE: keep Z0, A0, Z1, A1
 template <int NC, bool STORE>
 __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constant__ MlpArgs g,
                                                             int ntiles) {
-  constexpr int kRing = mlp_ring(STORE);
+  constexpr int kRing = mlp_ring(NC, STORE);
+  constexpr int kOut = mlp_out(NC, STORE);
+  constexpr bool kNarrow = mlp_narrow(NC, STORE);
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *s_w0 = smem, *s_w1 = s_w0 + NC * kStageBytes, *s_w2 = s_w1 + 2 * kStageBytes;
   uint8_t *s_ring = s_w2 + 2 * kStageBytes;
-  uint8_t *s_out = s_ring + kRing * kStageBytes;  // STORE: kOutBytes a warp
-  float *s_bias = reinterpret_cast<float *>(s_out + (STORE ? kEpiWarps * kOutBytes : 0));  // 3 x 128
+  uint8_t *s_out = s_ring + kRing * kStageBytes;  // kOut a warp
+  float *s_bias = reinterpret_cast<float *>(s_out + kEpiWarps * kOut);  // 3 x 128
   // full[kRing], empty[kRing], first_full[2], acc_full[2], h_full[2], d_free[3], done
   uint64_t *bars = reinterpret_cast<uint64_t *>(s_bias + 3 * kW);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 10);
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
     const int c0 = (((warp - kEpiWarp0) >> 2) & 1) * 64;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
     const uint32_t hid = hid_of(s) + lanes + (uint32_t)(c0 / 2);
-    uint8_t *out = s_out + (warp - kEpiWarp0) * kOutBytes;
+    uint8_t *out = s_out + (warp - kEpiWarp0) * kOut;
     bool ok = true;
     auto wait_for = [&](uint32_t bar, int n) {  // the n-th completion (from 0) of bar
       ok = __all_sync(0xffffffffu, mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail));
@@ -412,7 +418,6 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
           for (int k = 0; k < 4; k++) ld_sector(g.R + row * g.ldr + c0 + k * 16, res[k]);
         }
         if (!wait_for(acc_full(s), 2 * jj + 1)) break;
-        __nv_bfloat16 *y = reinterpret_cast<__nv_bfloat16 *>(g.Y) + row * g.ldy + c0;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
           float v[32];
@@ -433,9 +438,10 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
               }
             }
             pack16(u, p + 8 * m);
-            if (!STORE && live) st_sector(y + k * 32 + m * 16, p + 8 * m);
+            if (kNarrow)
+              put_rows<2>(out, lane, &g.my, c0 + k * 32 + m * 16, y0, y0 < g.M, p + 8 * m, false);
           }
-          if (STORE) put_rows(out, lane, &g.my, c0 + k * 32, y0, y0 < g.M, p, false);
+          if (!kNarrow) put_rows(out, lane, &g.my, c0 + k * 32, y0, y0 < g.M, p, false);
         }
       } else {  // the decoder: nout <= 16 FP32 columns
         if (!wait_for(acc_full(s), 2 * jj + 1)) break;
@@ -452,7 +458,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
         }
       }
     }
-    if (STORE && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   // every issued MMA has finished once "done" has arrived
@@ -473,8 +479,8 @@ int sm_count(int dev) {
 }
 
 constexpr size_t mlp_smem(int nc, bool store) {
-  return (size_t)(nc + 4 + mlp_ring(store)) * kStageBytes + (store ? kEpiWarps * kOutBytes : 0) +
-         3 * kW * sizeof(float) + (2 * mlp_ring(store) + 11) * sizeof(uint64_t) + 1024;
+  return (size_t)(nc + 4 + mlp_ring(nc, store)) * kStageBytes + kEpiWarps * mlp_out(nc, store) +
+         3 * kW * sizeof(float) + (2 * mlp_ring(nc, store) + 11) * sizeof(uint64_t) + 1024;
 }
 
 template <int NC, bool STORE>
@@ -1104,15 +1110,16 @@ extern "C" int op2b_gnn_mlp(int M, int nparts, const op2b_mlp_part *parts, const
       set_error("%s: input part %d cannot be described as a tensor map", what, i);
       return -1;
     }
-  if (store && !(tc_store_map(&g.mz[0], z0, false, kW, M, kW) &&
-                 tc_store_map(&g.mz[1], z1, false, kW, M, kW) &&
-                 tc_store_map(&g.ma[0], a0, false, kW, M, kW) &&
-                 tc_store_map(&g.ma[1], a1, false, kW, M, kW) &&
-                 (nout != kW || tc_store_map(&g.my, y, false, kW, M, ldy)))) {
+  const int nc = nparts == 1 ? (g.k0 <= 64 ? 1 : 2) : 2 * nparts;
+  if ((store && !(tc_store_map(&g.mz[0], z0, false, kW, M, kW) &&
+                  tc_store_map(&g.mz[1], z1, false, kW, M, kW) &&
+                  tc_store_map(&g.ma[0], a0, false, kW, M, kW) &&
+                  tc_store_map(&g.ma[1], a1, false, kW, M, kW))) ||
+      (nout == kW &&
+       !tc_store_map(&g.my, y, false, kW, M, ldy, mlp_narrow(nc, store) ? 32 : 64))) {
     set_error("%s: the results cannot be described as tensor maps", what);
     return -1;
   }
-  const int nc = nparts == 1 ? (g.k0 <= 64 ? 1 : 2) : 2 * nparts;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = store ? launch_mlp<true>(g, nc, s, dev) : launch_mlp<false>(g, nc, s, dev);
   if (rt().initialised) rt().launches++;

@@ -17,7 +17,9 @@ bool tc_operand_map(CUtensorMap *m, const void *base, int rows, int K, long ld);
 // gemm_tc.cu: a row-major BF16 or FP32 matrix as a tensor map of boxes of 64
 // bytes x 32 rows with the 64-byte swizzle (what one warp stores at a time);
 // false if it cannot be encoded
-bool tc_store_map(CUtensorMap *m, void *base, bool f32, int cols, int rows, long ld);
+bool tc_store_map(CUtensorMap *m, void *base, bool f32, int cols, int rows, long ld,
+                  int bytes = 64);
+
 
 namespace {
 
@@ -185,14 +187,18 @@ __device__ __forceinline__ void pack16(const float *v, uint32_t *r) {
 // lane's row, to column x (in elements of the map) of the rows from y on.  `out`:
 // the warp's 2 KiB of shared memory, in the 64-byte swizzle; rows past the
 // matrix are clipped.  `add`: an FP32 reduction instead of a store.
+// CH: 16-byte pieces of a row; 2 take half of that, 32 bytes a row, in the 32-byte
+// swizzle.
 constexpr int kOutBytes = 32 * 64;
+template <int CH = 4>
 __device__ __forceinline__ void put_rows(uint8_t *out, int lane, const CUtensorMap *m, int x, int y,
                                          bool inside, const uint32_t *v, bool add) {
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-    *reinterpret_cast<uint4 *>(out + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+  for (int i = 0; i < CH; i++)
+    *reinterpret_cast<uint4 *>(
+        out + lane * (16 * CH) + ((i ^ (CH == 4 ? (lane >> 1) & 3 : (lane >> 2) & 1)) << 4)) =
         make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();

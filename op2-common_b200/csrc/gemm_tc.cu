@@ -969,6 +969,10 @@ bool tc_operand_map(CUtensorMap *m, const void *base, int rows, int K, long ld) 
   return operand_map(m, base, rows, K, ld);
 }
 
+bool tc_operand_map_mn(CUtensorMap *m, const void *base, int mn, int K, long ld) {
+  return operand_map_mn(m, base, mn, K, ld);
+}
+
 bool tc_store_map(CUtensorMap *m, void *base, bool f32, int cols, int rows, long ld, int bytes) {
   EncodeTiled enc = encode_tiled();
   if (!enc) return false;

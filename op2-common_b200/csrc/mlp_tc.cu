@@ -800,8 +800,12 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 // blocks of X (the tiled product read it once a block), X's indexed blocks come
 // from their own rows (no gathered copy), and the column sums are one more
 // product, with a block of ones.  Operand tiles (64 rows x 128 columns, MN-major)
-// arrive by cp.async into a ring of 12 x 16 KiB.  The partial results are added
-// to the gradient with 16-byte reductions.
+// arrive in a ring of 12 x 16 KiB: direct rows of a line or more by TMA, two boxes
+// of 64 columns, from a warp of its own (a proxy fence between them had TMA's loads
+// wait for one another), the others by cp.async (narrow rows: TMA takes as long for
+// 16 bytes as for 128).  With all of them by cp.async, at most eight stages in
+// flight, the edge MLP's 635,000 rows took 276 us, so 209.  The partial results
+// are added to the gradient with 16-byte reductions.
 struct MlpDwJob {
   const __nv_bfloat16 *d;  // [M][ldd], nout columns
   long ldd;
@@ -809,15 +813,18 @@ struct MlpDwJob {
   MlpPart part[3];
   float *gw, *gb;
   int cta0, ctas;  // the CTAs of the job
+  int tma;         // bit t: operand t (d, then X's parts) by TMA
+  CUtensorMap map[4];
 };
 struct MlpDwArgs {
   int M, njobs;
   MlpDwJob job[3];
   int *err;
 };
-constexpr int kDwRing = 12, kDwLag = 8;
+constexpr int kDwRing = 12, kDwLag = 8;  // (12: every stage is always the same operand's)
 constexpr int kDwProducers = 4;                       // warps
-constexpr int kDwThreads = 32 * (kDwProducers + 4);   // + MMA warp (4) and three idle until the end
+// + MMA warp (4), TMA warp (5) and two idle until the end
+constexpr int kDwThreads = 32 * (kDwProducers + 4);
 constexpr size_t kDwSmem = (size_t)kDwRing * kStageBytes + 2048 + (2 * kDwRing + 3) * 8 + 1024;
 
 __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
@@ -845,7 +852,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kDwRing; s++) {
-      mbar_init(full(s), kDwProducers);
+      mbar_init(full(s), J.tma >> s % (P + 1) & 1 ? 1 : kDwProducers);
       mbar_init(empty(s), 1);
     }
     mbar_init(done, 1);
@@ -869,7 +876,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   const long nblk = ((long)g.M + 63) / 64, me = (int)blockIdx.x - J.cta0;
   const int b0 = (int)(nblk * me / J.ctas), b1 = (int)(nblk * (me + 1) / J.ctas);
 
-  if (warp < kDwProducers) {
+  const int tma = J.tma;
+  if (warp < kDwProducers && tma != (2 << P) - 1) {
     // 16 lanes a row of 256 bytes: thread t copies chunk t % 16 of the rows
     // t / 16 + 8 i, so its place moves by 1024 bytes with i
     const int c = threadIdx.x & 15, r0 = threadIdx.x >> 4;
@@ -880,7 +888,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0)
-        for (int s = handed; s < upto; s++) mbar_arrive(full(s % kDwRing));
+        for (int s = handed; s < upto; s++)
+          if (!(tma >> s % (P + 1) & 1)) mbar_arrive(full(s % kDwRing));
       handed = upto;
     };
     // the four operands' first chunk, row stride in bytes and whether the
@@ -914,6 +923,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
 #pragma unroll
       for (int t = 0; t < 4; t++) {  // d, then X's blocks
         if (t > P) break;
+        if (tma >> t & 1) {  // (an empty group: stages and groups count alike)
+          asm volatile("cp.async.commit_group;" ::: "memory");
+          it++;
+          continue;
+        }
         const int st = it % kDwRing;
         if (it >= kDwRing) {
           const uint32_t par = (uint32_t)((it / kDwRing - 1) & 1);
@@ -955,6 +969,27 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     hand_on(it);
+  } else if (warp == kDwProducers + 1 && lane == 0) {
+    int it = 0;
+    bool ok = true;
+    for (int b = b0; b < b1 && ok; b++)
+      for (int t = 0; t <= P; t++, it++) {
+        if (!(tma >> t & 1)) continue;
+        const int st = it % kDwRing;
+        if (it >= kDwRing &&
+            !mbar_wait_or_fail(empty(st), (uint32_t)((it / kDwRing - 1) & 1), fail)) {
+          atomicExch(&s_fail, 1);
+          ok = false;
+          break;
+        }
+        const uint32_t to = smem_u32(s_ring + (size_t)st * kStageBytes);
+        mbar_expect_tx(full(st), kStageBytes);  // (rows and columns outside: zeros)
+        tma_load_2d(to, &J.map[t], 0, b * 64, full(st));
+        tma_load_2d(to + kStageBytes / 2, &J.map[t], 64, b * 64, full(st));
+      }
+    if (*fail)  // the loads that nobody waits for any more
+      for (int s = max(0, it - kDwRing); s < it; s++)
+        if (tma >> s % (P + 1) & 1) mbar_wait(full(s % kDwRing), (uint32_t)((s / kDwRing) & 1));
   } else if (warp == kDwProducers && lane == 0) {
     const uint32_t mn = 1u << 15 | 1u << 16;  // A and B MN-major
     const uint32_t idesc = umma_idesc(kW) | mn, idesc1 = umma_idesc(16) | 1u << 15;
@@ -1235,14 +1270,31 @@ extern "C" int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
-  // CTAs by the tiles a job reads per 64 rows, at least four blocks of rows each
+  // CTAs by the tiles a job reads per 64 rows, a gathered one counting half as much
+  // again (edge MLP of 635,000 rows: 228 us without, 209 with; twice as much: 225),
+  // at least four blocks of rows each
   const int nsm = sm_count(dev), most = std::max(1, ((M + 63) / 64 + 3) / 4);
-  int total = 0, at = 0;
-  for (const MlpDwJob &J : g.job) total += 1 + J.nparts;
-  for (MlpDwJob &J : g.job) {
+  int total = 0, at = 0, cost[3];
+  for (int l = 0; l < 3; l++) {
+    cost[l] = 2 + 2 * g.job[l].nparts;
+    for (int i = 0; i < g.job[l].nparts; i++) cost[l] += g.job[l].part[i].rows ? 1 : 0;
+    total += cost[l];
+  }
+  for (int l = 0; l < 3; l++) {
+    MlpDwJob &J = g.job[l];
     J.cta0 = at;
-    J.ctas = std::max(1, std::min(most, nsm * (1 + J.nparts) / total));
+    J.ctas = std::max(1, std::min(most, nsm * cost[l] / total));
     at += J.ctas;
+    for (int t = 0; t <= J.nparts; t++) {
+      const MlpPart &X = J.part[t ? t - 1 : 0];
+      const int cols = t ? X.cols : J.nout;
+      if (cols < 64 || (t && X.rows)) continue;
+      if (!tc_operand_map_mn(&J.map[t], t ? X.p : J.d, cols, M, t ? X.ld : J.ldd)) {
+        set_error("%s: an operand cannot be described as a tensor map", what);
+        return -1;
+      }
+      J.tma |= 1 << t;
+    }
   }
   static bool attr[16] = {};
   if (!attr[dev]) {

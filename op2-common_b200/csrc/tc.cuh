@@ -14,6 +14,8 @@ int *tc_error_flag(const char *what, int *device = nullptr);
 // gemm_tc.cu: a K-major BF16 operand (rows x K, row stride ld elements) as a
 // tensor map of 64 x 128 boxes with the 128-byte swizzle
 bool tc_operand_map(CUtensorMap *m, const void *base, int rows, int K, long ld);
+// gemm_tc.cu: an MN-major one (K rows of mn values) in boxes of 64 x 64
+bool tc_operand_map_mn(CUtensorMap *m, const void *base, int mn, int K, long ld);
 // gemm_tc.cu: a row-major BF16 or FP32 matrix as a tensor map of boxes of 64
 // bytes x 32 rows with the 64-byte swizzle (what one warp stores at a time);
 // false if it cannot be encoded

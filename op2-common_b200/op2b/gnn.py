@@ -278,23 +278,26 @@ class GraphNet:
         ws = dict(N=N, E=E, train=train)
         if self.gemm_tma:
             # one kernel a MLP: the node and edge states and the aggregates, in
-            # training those of every step and the hidden layers
+            # training those of every step and the hidden layers.  Every pass writes
+            # these before it reads them, so they are not cleared (107 fills, 2.9 ms of
+            # the first training step at 8 x 200x100)
+            n = lambda *shape, dt=bf: torch.empty(*shape, dtype=dt, device="cuda")
             keep = S if train else 0
-            ws["h"] = [z(N, w) for _ in range(keep + 1)]
-            ws["e"] = [z(E, w) for _ in range(keep + 1)]
-            ws["agg"] = [z(N, w) for _ in range(max(keep, 1))]
+            ws["h"] = [n(N, w) for _ in range(keep + 1)]
+            ws["e"] = [n(E, w) for _ in range(keep + 1)]
+            ws["agg"] = [n(N, w) for _ in range(max(keep, 1))]
             ws["out"] = z(N, OUT, dt=f32)
             if train:
                 ws["act"] = {}
                 for name, _layers in self.lay:
                     rows = E if name.startswith("edge") or name == "enc_edge" else N
-                    ws["act"][name] = [z(rows, w) for _ in range(4)]
+                    ws["act"][name] = [n(rows, w) for _ in range(4)]
                 R = max(N, E)
                 ws["dOut"] = z(N, OUT)
-                ws["dH"], ws["dE"] = z(N, w, dt=f32), z(E, w, dt=f32)
-                ws["dAgg"], ws["dX"] = z(N, w, dt=f32), z(E, 2 * w, dt=f32)
-                ws["dyN"], ws["dyE"] = z(N, w), z(E, w)
-                ws["d0"], ws["d1"] = z(R, w), z(R, w)
+                ws["dH"], ws["dE"] = n(N, w, dt=f32), n(E, w, dt=f32)
+                ws["dAgg"], ws["dX"] = n(N, w, dt=f32), n(E, 2 * w, dt=f32)
+                ws["dyN"], ws["dyE"] = n(N, w), n(E, w)
+                ws["d0"], ws["d1"] = n(R, w), n(R, w)
                 ws["loss"] = z(1, dt=f32)
             self._ws[key] = ws
             return ws

@@ -798,15 +798,25 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 // The CTAs are shared out among the layers by the bytes each reads, and a CTA
 // keeps its layer's whole 128 x (up to 384) gradient in tensor memory while it
 // walks its share of the rows, 64 at a time: d is read once for all column
-// blocks of X (the tiled product read it once a block), X's indexed blocks come
-// from their own rows (no gathered copy), and the column sums are one more
-// product, with a block of ones.  Operand tiles (64 rows x 128 columns, MN-major)
+// blocks of X (the tiled product read it once a block), and X's indexed blocks come
+// from their own rows (no gathered copy).  Operand tiles (64 rows x 128 columns, MN-major)
 // arrive in a ring of 12 x 16 KiB: direct rows of a line or more by TMA, two boxes
 // of 64 columns, from a warp of its own (a proxy fence between them had TMA's loads
 // wait for one another), the others by cp.async (narrow rows: TMA takes as long for
 // 16 bytes as for 128).  With all of them by cp.async, at most eight stages in
-// flight, the edge MLP's 635,000 rows took 276 us, so 209.  The partial results
-// are added to the gradient with 16-byte reductions.
+// flight, the edge MLP's 635,000 rows took 276 us, so 209.
+// Four more warps hold the sums' rounding to that of the layer by layer products,
+// whose CTAs add up a few thousand rows each: the tensor core's accumulation
+// drifts with its length.  An accumulator is left after J.flush blocks of rows
+// and the MMAs go on in the free 128 columns of tensor memory, each accumulator at
+// blocks of its own; the warps meanwhile add the one left to the gradient or, of
+// a single 128 x 128 one, to a running sum in tensor memory (20,000 rows of three parts
+// 37.9 -> 33.8 us).  And they add d's columns up from its stages with FP32 additions, the
+// running sum compensated.  Error against FP64 sums of the same operands at 635,000
+// rows, as a part of the norm, for one accumulator a CTA, now and layer by layer:
+// dW1 2.3e-5, 2.2e-6, 2.3e-6; with a mean of one standard deviation 4.9e-5, 2.5e-6,
+// 2.6e-6 and db1 (a product with ones before) 1.3e-5, 9e-8, 2.8e-7.  It costs 1 to 2 % of
+// the edge MLP's kernel and 1.3 % of a training step.
 struct MlpDwJob {
   const __nv_bfloat16 *d;  // [M][ldd], nout columns
   long ldd;
@@ -814,6 +824,7 @@ struct MlpDwJob {
   MlpPart part[3];
   float *gw, *gb;
   int cta0, ctas;  // the CTAs of the job
+  int flush;       // blocks of 64 rows an accumulator
   int tma;         // bit t: operand t (d, then X's parts) by TMA
   CUtensorMap map[4];
 };
@@ -823,10 +834,10 @@ struct MlpDwArgs {
   int *err;
 };
 constexpr int kDwRing = 12, kDwLag = 8;  // (12: every stage is always the same operand's)
-constexpr int kDwProducers = 4;                       // warps
-// + MMA warp (4), TMA warp (5) and two idle until the end
-constexpr int kDwThreads = 32 * (kDwProducers + 4);
-constexpr size_t kDwSmem = (size_t)kDwRing * kStageBytes + 2048 + (2 * kDwRing + 3) * 8 + 1024;
+constexpr int kDwProducers = 4, kDwSumWarp0 = 6, kDwSumWarps = 4;  // warps; 4: MMA, 5: TMA
+constexpr int kDwThreads = 32 * (kDwSumWarp0 + kDwSumWarps);
+constexpr size_t kDwSmem =
+    (size_t)kDwRing * kStageBytes + kDwSumWarps * kW * 4 + (2 * kDwRing + 6) * 8 + 1024;
 
 __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
@@ -834,17 +845,54 @@ __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, fl
                : "memory");
 }
 
+// 32 columns cc .. of row n of an accumulator (and of the one before it, if any),
+// added to the gradient
+__device__ __forceinline__ void dw_add(const MlpDwJob &J, uint32_t acc, bool two, uint32_t sum, int n,
+                                       int cc) {
+  float v[32];
+  tmem_ld32(acc, v);
+  if (two) {
+    float u[32];
+    tmem_ld32(sum, u);
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] += u[i];
+  }
+  float *w = J.gw + (long)n * J.kin + cc;
+  if (n < J.nout) {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (cc + 4 * i < J.kin) red_add4(w + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  }
+}
+
+// 32 columns of an accumulator into the sum of the ones before it (`first`: none)
+__device__ __forceinline__ void dw_keep(uint32_t acc, uint32_t sum, bool first) {
+  float v[32];
+  tmem_ld32(acc, v);
+  if (!first) {
+    float u[32];
+    tmem_ld32(sum, u);
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] += u[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 32; i += 8) tmem_st8(sum + i, reinterpret_cast<const uint32_t *>(v + i));
+}
+
 __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant__ MlpDwArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t *s_ring = smem, *s_ones = smem + (size_t)kDwRing * kStageBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(s_ones + 2048);
-  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kDwRing + 1);
-  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  uint8_t *s_ring = smem;
+  float(*s_sum)[kW] = reinterpret_cast<float(*)[kW]>(smem + (size_t)kDwRing * kStageBytes);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_sum + kDwSumWarps);
+  uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kDwRing + 3);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1), *s_place = &s_fail + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int s) { return smem_u32(&bars[s]); };
   auto empty = [&](int s) { return smem_u32(&bars[kDwRing + s]); };
   const uint32_t done = smem_u32(&bars[2 * kDwRing]);
+  const uint32_t acc_full = smem_u32(&bars[2 * kDwRing + 1]);   // one to be added and left
+  const uint32_t acc_empty = smem_u32(&bars[2 * kDwRing + 2]);  // it has been
   volatile int *fail = &s_fail;
   int q = 0;
   while (q + 1 < g.njobs && (int)blockIdx.x >= g.job[q + 1].cta0) q++;
@@ -854,9 +902,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < kDwRing; s++) {
       mbar_init(full(s), J.tma >> s % (P + 1) & 1 ? 1 : kDwProducers);
-      mbar_init(empty(s), 1);
+      mbar_init(empty(s), s % (P + 1) == 0 ? 1 + kDwSumWarps : 1);  // (d: and its sums)
     }
     mbar_init(done, 1);
+    mbar_init(acc_full, 1);
+    mbar_init(acc_empty, kDwSumWarps);
     s_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -866,16 +916,33 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
                  "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  for (int i = threadIdx.x; i < 512; i += kDwThreads)  // 16 x 64 BF16 ones
-    reinterpret_cast<uint32_t *>(s_ones)[i] = 0x3f803f80u;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_taddr;
   // the CTA's blocks of 64 rows
   const long nblk = ((long)g.M + 63) / 64, me = (int)blockIdx.x - J.cta0;
-  const int b0 = (int)(nblk * me / J.ctas), b1 = (int)(nblk * (me + 1) / J.ctas);
+  const int b0 = (int)(nblk * me / J.ctas), b1 = (int)(nblk * (me + 1) / J.ctas), nb = b1 - b0;
+  // accumulator p's place (128 columns) in tensor memory and the free one's; the
+  // MMA and the sum warps exchange them alike
+  int acc_at[3] = {0, 1, 2}, spare = 3;
+  constexpr int kSumAt = 1;  // one accumulator only: the sum of the ones before it
+  // blocks until accumulator p is full, each at blocks of its own (the last block's
+  // are read by all warps)
+  int until[3];
+#pragma unroll
+  for (int p = 0; p < 3; p++) until[p] = J.flush - p * (J.flush / P);
+  auto is_full = [&](int p, int b) {
+    if (--until[p] > 0) return false;
+    until[p] = J.flush;
+    return b + 1 < nb;
+  };
+  auto exchange = [&](int p) {  // (p is a constant of an unrolled loop)
+    const int t = acc_at[p];
+    acc_at[p] = spare;
+    spare = t;
+    return t;
+  };
 
   const int tma = J.tma;
   if (warp < kDwProducers && tma != (2 << P) - 1) {
@@ -992,65 +1059,116 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
       for (int s = max(0, it - kDwRing); s < it; s++)
         if (tma >> s % (P + 1) & 1) mbar_wait(full(s % kDwRing), (uint32_t)((s / kDwRing) & 1));
   } else if (warp == kDwProducers && lane == 0) {
-    const uint32_t mn = 1u << 15 | 1u << 16;  // A and B MN-major
-    const uint32_t idesc = umma_idesc(kW) | mn, idesc1 = umma_idesc(16) | 1u << 15;
-    const uint32_t ones = smem_u32(s_ones);
-    int it = 0;
-    bool ok = true;
-    auto wait = [&](int st, int n) {
-      ok = ok && mbar_wait_or_fail(full(st), (uint32_t)(n & 1), fail);
+    const uint32_t idesc = umma_idesc(kW) | 1u << 15 | 1u << 16;  // A and B MN-major
+    int it = 0, left = 0;
+    bool ok = true, fresh[3] = {true, true, true};
+    auto wait = [&](uint32_t bar, int n) {
+      ok = ok && mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail);
       if (!ok) atomicExch(&s_fail, 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     };
-    for (int b = b0; b < b1 && ok; b++) {
+    for (int b = 0; b < nb && ok; b++) {
       const int sd = it % kDwRing;
-      wait(sd, it / kDwRing);
+      wait(full(sd), it / kDwRing);
       it++;
       const uint32_t a = smem_u32(s_ring + (size_t)sd * kStageBytes);
-      for (int p = 0; p < P && ok; p++) {
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        if (p >= P || !ok) break;
         const int st = it % kDwRing;
-        wait(st, it / kDwRing);
+        wait(full(st), it / kDwRing);
         it++;
         if (!ok) break;
         const uint32_t x = smem_u32(s_ring + (size_t)st * kStageBytes);
 #pragma unroll
         for (int k = 0; k < 4; k++)
-          umma_ss(tmem + (uint32_t)p * kW, umma_desc_mn(a + k * 2048), umma_desc_mn(x + k * 2048),
-                  idesc, b > b0 || k > 0);
+          umma_ss(tmem + (uint32_t)(acc_at[p] * kW), umma_desc_mn(a + k * 2048),
+                  umma_desc_mn(x + k * 2048), idesc, !fresh[p] || k > 0);
+        fresh[p] = false;
         umma_commit(empty(st));
+        if (is_full(p, b)) {
+          if (left > 0) wait(acc_empty, left - 1);  // the place it goes on in has been read
+          left++;
+          umma_commit(acc_full);
+          exchange(p);
+          fresh[p] = true;
+        }
       }
       if (!ok) break;
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        umma_ss(tmem + 3u * kW, umma_desc_mn(a + k * 2048), umma_desc(ones), idesc1,
-                b > b0 || k > 0);
       umma_commit(empty(sd));
     }
     umma_commit(done);
+#pragma unroll
+    for (int p = 0; p < 3; p++) s_place[p] = acc_at[p];
+    s_place[3] = P == 1 && left > 0;
+  } else if (warp >= kDwSumWarp0) {
+    // warp w sums the rows 16 (w - 6) .. of every block of d, a lane four columns
+    const int r0 = (warp - kDwSumWarp0) * 16;
+    const uint32_t col = (uint32_t)((lane >> 4) * (kStageBytes / 2) + (lane & 1) * 8);
+    const int chunk = (lane & 15) >> 1;
+    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, rest[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int left = 0;
+    bool ok = true;
+    auto wait = [&](uint32_t bar, int n) {
+      ok = __all_sync(0xffffffffu, mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail));
+      if (!ok && lane == 0) atomicExch(&s_fail, 1);
+      return ok;
+    };
+    for (int b = 0; b < nb && ok; b++) {
+      const int it = b * (P + 1), st = it % kDwRing;
+      if (!wait(full(st), it / kDwRing)) break;
+      const uint8_t *d = s_ring + (size_t)st * kStageBytes + col;
+      float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(d + sw128(r0 + r, chunk));
+        part[0] += __uint_as_float(t.x << 16);
+        part[1] += __uint_as_float(t.x & 0xffff0000u);
+        part[2] += __uint_as_float(t.y << 16);
+        part[3] += __uint_as_float(t.y & 0xffff0000u);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {  // (with the last addition's rounding error made good,
+        const float y = part[i] - rest[i], t = sum[i] + y, e = (t - sum[i]) - y;
+        rest[i] = fabsf(e) < INFINITY ? e : 0.0f;  // if there is one: infinities stay)
+        sum[i] = t;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty(st));
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        if (p >= P || !is_full(p, b)) continue;
+        if (!wait(acc_full, left)) break;
+        left++;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t acc = lanes + (uint32_t)(exchange(p) * kW);
+        for (int cc = 0; cc < kW; cc += 32) {
+          if (P == 1) dw_keep(acc + (uint32_t)cc, lanes + (uint32_t)(kSumAt * kW + cc), left == 1);
+          else dw_add(J, acc + (uint32_t)cc, false, 0, (warp & 3) * 32 + lane, p * kW + cc);
+        }
+        if (P == 1) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+      }
+    }
+    reinterpret_cast<float4 *>(s_sum[warp - kDwSumWarp0])[lane] =
+        make_float4(sum[0], sum[1], sum[2], sum[3]);
   }
   __syncthreads();
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!s_fail && b1 > b0) {
+  if (!s_fail && nb > 0 && warp < 8) {
     // warps w and w + 4 share a lane quarter: row n of the gradient is a lane
-    const int n = (warp & 3) * 32 + lane;
-    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64) {
-      float v[32];
-      tmem_ld32(tmem + lanes + (uint32_t)cc, v);
-      float *w = J.gw + (long)n * J.kin + cc;
-      if (n < J.nout) {
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (cc + 4 * i < J.kin) red_add4(w + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      }
-    }
-    if (warp < 4) {
-      float v[32];
-      tmem_ld32(tmem + lanes + 3u * kW, v);
-      if (n < J.nout) atomicAdd(J.gb + n, v[0]);
-    }
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64)
+      dw_add(J, lanes + (uint32_t)(s_place[cc / kW] * kW + cc % kW), s_place[3] != 0,
+             lanes + (uint32_t)(kSumAt * kW + cc), (warp & 3) * 32 + lane, cc);
+  } else if (!s_fail && nb > 0 && warp == 8) {
+    for (int c = lane; c < J.nout; c += 32)
+      atomicAdd(J.gb + c, (s_sum[0][c] + s_sum[1][c]) + (s_sum[2][c] + s_sum[3][c]));
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1271,14 +1389,14 @@ extern "C" int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
-  // CTAs by the tiles a job reads per 64 rows, a gathered one counting half as much
-  // again (edge MLP of 635,000 rows: 228 us without, 209 with; twice as much: 225),
-  // at least four blocks of rows each
+  // CTAs by the tiles a job reads per 64 rows, a gathered one counting twice (edge
+  // MLP of 635,000 rows with random indices: 255 us with half as much again, 247 with
+  // this), at least four blocks of rows each
   const int nsm = sm_count(dev), most = std::max(1, ((M + 63) / 64 + 3) / 4);
   int total = 0, at = 0, cost[3];
   for (int l = 0; l < 3; l++) {
     cost[l] = 2 + 2 * g.job[l].nparts;
-    for (int i = 0; i < g.job[l].nparts; i++) cost[l] += g.job[l].part[i].rows ? 1 : 0;
+    for (int i = 0; i < g.job[l].nparts; i++) cost[l] += g.job[l].part[i].rows ? 2 : 0;
     total += cost[l];
   }
   for (int l = 0; l < 3; l++) {
@@ -1286,6 +1404,9 @@ extern "C" int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int
     J.cta0 = at;
     J.ctas = std::max(1, std::min(most, nsm * cost[l] / total));
     at += J.ctas;
+    // an accumulator's rows: those of a split of the layer by layer product
+    const int pieces = std::max(1, std::min(2 * nsm / J.nparts, M / 256));
+    J.flush = ((M + pieces - 1) / pieces + 63) / 64;
     for (int t = 0; t <= J.nparts; t++) {
       const MlpPart &X = J.part[t ? t - 1 : 0];
       const int cols = t ? X.cols : J.nout;

@@ -31,6 +31,7 @@
 
 #include "op2b_gnn.h"
 #include "op2b_runtime.h"
+#include "ring.h"
 #include "tc.cuh"
 
 namespace op2b {
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
   constexpr int kRing = mlp_ring(NC, STORE);
   constexpr int kOut = mlp_out(NC, STORE);
   constexpr bool kNarrow = mlp_narrow(NC, STORE);
+  constexpr int kTurns = kProducerWarps < kRing ? kProducerWarps : kRing;  // loading warps
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *s_w0 = smem, *s_w1 = s_w0 + NC * kStageBytes, *s_w2 = s_w1 + 2 * kStageBytes;
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
   // full[kRing], empty[kRing], first_full[2], acc_full[2], h_full[2], d_free[3], done
   uint64_t *bars = reinterpret_cast<uint64_t *>(s_bias + 3 * kW);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kRing + 10);
-  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1), *s_last = &s_fail + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int s) { return smem_u32(&bars[s]); };
   auto empty = [&](int s) { return smem_u32(&bars[kRing + s]); };
@@ -235,12 +237,13 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
   if (warp < kProducerWarps) {
     // stage n is one warp's (n % kTurns): the warps' latencies overlap, and each
     // waits only for its own copies.  No more warps than stages: the wait for a
-    // stage's last use then follows, in the same warp, one that implies the use before.  Direct rows (zeros outside the rows and columns)
-    // come by TMA; of indexed ones lane l copies chunk l % 8 of rows
-    // l / 8 + 4 i, eight lanes a row, each lane holding four rows' indices.
+    // stage's last use then follows, in the same warp, one that implies the use
+    // before.
+    // Direct rows (zeros outside the rows and columns) come by TMA; of indexed ones
+    // lane l copies chunk l % 8 of rows l / 8 + 4 i, eight lanes a row, each lane
+    // holding four rows' indices.
     const int kc = lane & 7, r0 = lane >> 3;
     const uint32_t place0 = sw128(r0, kc), place1 = sw128(r0 + 4, kc);  // even, odd i
-    constexpr int kTurns = kProducerWarps < kRing ? kProducerWarps : kRing;
     const int total = warp < kTurns ? nloc * NC : 0;
     int n = warp, j = warp / NC, c = warp % NC;  // stage, local tile, block
     int idx[4] = {0, 0, 0, 0}, next[4] = {0, 0, 0, 0};
@@ -252,7 +255,6 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
       for (int i = 0; i < 4; i++) to[i] = m + 32 * i < g.M ? __ldg(rows + m + 32 * i) : 0;
     };
     if (n < total) load_rows(j, c, idx);
-    int tma = -1;  // the last stage this warp loaded by TMA
     for (; n < total; n += kTurns) {
       const int st = n % kRing;
       const int jn = c + kTurns >= NC ? j + (c + kTurns) / NC : j;
@@ -273,7 +275,6 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
           mbar_expect_tx(full(st), kStageBytes);
           tma_load_2d(dst, &g.mx[NC == 1 ? 0 : c >> 1], cb, m0, full(st));
         }
-        tma = n;
       } else {
         const char *base = reinterpret_cast<const char *>(P.p + cb + kc * 8);
         const long ld = 2 * P.ld;
@@ -295,8 +296,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
       j = jn;
       c = cn;
     }
-    // after a failure, a load that nobody waits for any more
-    if (lane == 0 && *fail && tma >= 0) mbar_wait(full(tma % kRing), (uint32_t)((tma / kRing) & 1));
+    if (lane == 0) s_last[warp] = n - kTurns;
   } else if (warp == kMmaWarp) {
     if (lane == 0) {  // MMA issuer: whatever has its operands next
       const uint32_t idesc = umma_idesc(kW), idesc2 = umma_idesc((g.nout + 15) & ~15);
@@ -463,6 +463,14 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_fwd(const __grid_constan
   __syncthreads();
   // every issued MMA has finished once "done" has arrived
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  if (threadIdx.x == 0 && s_fail) {  // the loads that nobody waits for any more
+#pragma unroll 1
+    for (int st = 0; st < kRing; st++) {
+      const int n = newest_in_flight(st, kRing, s_last, kTurns);
+      if (n >= 0 && !g.part[NC == 1 ? 0 : n % NC >> 1].rows)
+        mbar_wait(full(st), (uint32_t)((n / kRing) & 1));
+    }
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -480,7 +488,7 @@ int sm_count(int dev) {
 
 constexpr size_t mlp_smem(int nc, bool store) {
   return (size_t)(nc + 4 + mlp_ring(nc, store)) * kStageBytes + kEpiWarps * mlp_out(nc, store) +
-         3 * kW * sizeof(float) + (2 * mlp_ring(nc, store) + 11) * sizeof(uint64_t) + 1024;
+         3 * kW * sizeof(float) + (2 * mlp_ring(nc, store) + 13) * sizeof(uint64_t) + 1024;
 }
 
 template <int NC, bool STORE>
@@ -557,7 +565,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
   // full[kBwdRing], empty[kBwdRing], acc_full[2], h_full[2], d_free[2], done
   uint64_t *bars = reinterpret_cast<uint64_t *>(s_out + kEpiWarps * kOutBytes);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kBwdRing + 7);
-  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1);
+  int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1), &s_loaded = *(&s_fail + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int s) { return smem_u32(&bars[s]); };
   auto empty = [&](int s) { return smem_u32(&bars[kBwdRing + s]); };
@@ -621,9 +629,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
         tma_load_2d(smem_u32(s_ring + (size_t)st * kStageBytes), &g.mdy, n % nkb * 64, m0,
                     full(st));
       }
-      if (*fail)  // the loads that nobody waits for any more
-        for (int i = max(0, n - kBwdRing); i < n; i++)
-          mbar_wait(full(i % kBwdRing), (uint32_t)((i / kBwdRing) & 1));
+      s_loaded = n;
     }
   } else if (warp == kMmaWarp) {
     if (lane == 0) {
@@ -783,6 +789,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
   }
   __syncthreads();
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  if (threadIdx.x == 0 && s_fail)  // the loads that nobody waits for any more
+    for (int i = max(0, s_loaded - kBwdRing); i < s_loaded; i++)
+      mbar_wait(full(i % kBwdRing), (uint32_t)((i / kBwdRing) & 1));
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -837,7 +846,7 @@ constexpr int kDwRing = 12, kDwLag = 8;  // (12: every stage is always the same 
 constexpr int kDwProducers = 4, kDwSumWarp0 = 6, kDwSumWarps = 4;  // warps; 4: MMA, 5: TMA
 constexpr int kDwThreads = 32 * (kDwSumWarp0 + kDwSumWarps);
 constexpr size_t kDwSmem =
-    (size_t)kDwRing * kStageBytes + kDwSumWarps * kW * 4 + (2 * kDwRing + 6) * 8 + 1024;
+    (size_t)kDwRing * kStageBytes + kDwSumWarps * kW * 4 + (2 * kDwRing + 7) * 8 + 1024;
 
 __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
@@ -886,6 +895,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   float(*s_sum)[kW] = reinterpret_cast<float(*)[kW]>(smem + (size_t)kDwRing * kStageBytes);
   uint64_t *bars = reinterpret_cast<uint64_t *>(s_sum + kDwSumWarps);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kDwRing + 3);
+  // s_place[0-2]: the accumulators' places at the end, [3]: whether there is a sum of
+  // earlier ones, [4]: stages that the TMA warp went past
   int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1), *s_place = &s_fail + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int s) { return smem_u32(&bars[s]); };
@@ -1055,9 +1066,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
         tma_load_2d(to, &J.map[t], 0, b * 64, full(st));
         tma_load_2d(to + kStageBytes / 2, &J.map[t], 64, b * 64, full(st));
       }
-    if (*fail)  // the loads that nobody waits for any more
-      for (int s = max(0, it - kDwRing); s < it; s++)
-        if (tma >> s % (P + 1) & 1) mbar_wait(full(s % kDwRing), (uint32_t)((s / kDwRing) & 1));
+    s_place[4] = it;
   } else if (warp == kDwProducers && lane == 0) {
     const uint32_t idesc = umma_idesc(kW) | 1u << 15 | 1u << 16;  // A and B MN-major
     int it = 0, left = 0;
@@ -1158,6 +1167,9 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   }
   __syncthreads();
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
+  if (threadIdx.x == 0 && s_fail)  // the loads that nobody waits for any more
+    for (int s = max(0, s_place[4] - kDwRing); s < s_place[4]; s++)
+      if (tma >> s % (P + 1) & 1) mbar_wait(full(s % kDwRing), (uint32_t)((s / kDwRing) & 1));
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!s_fail && nb > 0 && warp < 8) {
@@ -1181,7 +1193,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
 
 constexpr size_t mlp_bwd_smem(int np) {
   return (size_t)(4 + 2 * np + kBwdRing) * kStageBytes + kEpiWarps * kOutBytes +
-         (2 * kBwdRing + 8) * sizeof(uint64_t) + 1024;
+         (2 * kBwdRing + 9) * sizeof(uint64_t) + 1024;
 }
 
 template <int NP> cudaError_t launch_mlp_bwd(const MlpBwdArgs &g, cudaStream_t s, int dev) {

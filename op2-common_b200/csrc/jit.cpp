@@ -631,54 +631,62 @@ std::string generate(const char *name, const std::vector<ArgPlan> &ap, const std
       << a.dim << " + k] = sp[b * " << a.dim << " + k];\n      }\n    }\n  }\n";
   }
   if (red) {
-    // one pass: `value(entry)` through the warps' shuffles into op2b_rs, then a
-    // thread an entry over the block's eight warps
-    s << "  __shared__ unsigned long long op2b_rs[8][" << red << "];\n  __shared__ bool op2b_last;\n";
-    for (int pass = 0; pass < 2; pass++) {
-      int t = 0;
-      for (size_t i = 0; i < ap.size(); i++) {
-        const ArgPlan &a = ap[i];
-        if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
-        const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
-        s << "#pragma unroll\n  for (int k = 0; k < " << a.dim << "; k++) {\n    " << a.ctype
-          << " v = ";
-        if (pass == 0)
-          s << "op2b_l" << i << "[k];\n";
-        else
-          s << identity(a.ctype, a.acc) << ";\n    for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) {\n"
-            << "      const " << a.ctype << " w = *(const volatile " << a.ctype << " *)(op2b_parts + (size_t)b * "
-            << red << " + " << t << " + k);\n      v = " << op << ";\n    }\n";
-        s << "    for (int o = 16; o > 0; o >>= 1) { " << a.ctype
-          << " w = __shfl_down_sync(0xffffffffu, v, o); v = " << op << "; }\n"
-          << "    if ((threadIdx.x & 31) == 0) *(" << a.ctype << " *)&op2b_rs[threadIdx.x >> 5]["
-          << t << " + k] = v;\n  }\n";
-        t += a.dim;
-      }
-      s << "  __syncthreads();\n";
-      t = 0;
-      for (size_t i = 0; i < ap.size(); i++) {
-        const ArgPlan &a = ap[i];
-        if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
-        const char *op = a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)";
-        s << "  if (threadIdx.x >= " << t << " && threadIdx.x < " << t + a.dim << ") {\n    " << a.ctype
-          << " v = *(" << a.ctype << " *)&op2b_rs[0][threadIdx.x];\n"
-          << "    for (int j = 1; j < 8; j++) { const " << a.ctype << " w = *(" << a.ctype
-          << " *)&op2b_rs[j][threadIdx.x]; v = " << op << "; }\n"
-          << "    unsigned long long u = 0;\n    *(" << a.ctype << " *)&u = v;\n";
-        if (pass == 0)
-          s << "    op2b_parts[(size_t)blockIdx.x * " << red << " + threadIdx.x] = u;\n    __threadfence();\n";
-        else
-          s << "    op2b_rs[0][threadIdx.x] = u;\n    op2b_host[threadIdx.x] = u;\n";
-        s << "  }\n";
-        t += a.dim;
-      }
-      s << "  __syncthreads();\n";
-      if (pass == 0)
-        s << "  if (threadIdx.x == 0) op2b_last = atomicAdd(op2b_ticket, 1u) == gridDim.x - 1;\n"
-             "  __syncthreads();\n  if (!op2b_last) return;\n  __threadfence();\n";
+    // two passes over one body: every block combines its threads' values (warps'
+    // shuffles, then a thread an entry over the eight warps) and leaves them, the
+    // last block does the same with the blocks'.  Rolled up, as a user waits for the
+    // compiler at the first call: 65 ms for the step of a diffusion loop (two entries),
+    // 109 with both passes written out and unrolled, 57 with a warp's atomics instead.
+    struct Entry {
+      size_t arg;
+      int at, dim;
+      std::string type, op;
+    };
+    std::vector<Entry> es;
+    for (size_t i = 0, t = 0; i < ap.size(); i++) {
+      const ArgPlan &a = ap[i];
+      if (a.kind != GBL || a.acc == OP_READ || a.acc == OP_WORK) continue;
+      es.push_back({i, (int)t, a.dim, a.ctype,
+                    a.acc == OP_INC ? "v + w" : a.acc == OP_MIN ? "op2b_min(v, w)" : "op2b_max(v, w)"});
+      t += (size_t)a.dim;
     }
-    s << "  if (threadIdx.x == 0) {\n    unsigned long long h = op2b_seq * 0x9e3779b97f4a7c15ull;\n"
-         "    for (int t = 0; t < " << red << "; t++) h = op2b_mix(h, op2b_rs[0][t]);\n"
+    auto each = [&](const Entry &e, const char *indent) -> std::ostringstream & {
+      s << "#pragma unroll\n" << indent << "for (int k = 0; k < " << e.dim << "; k++) { ";
+      return s;
+    };
+    s << "  __shared__ unsigned long long op2b_rs[8][" << red << "];\n  __shared__ bool op2b_last;\n"
+         "#pragma unroll 1\n  for (int op2b_pass = 0; op2b_pass < 2; op2b_pass++) {\n    if (op2b_pass) {\n";
+    for (const Entry &e : es)
+      each(e, "      ") << "op2b_l" << e.arg << "[k] = " << identity(e.type, ap[e.arg].acc) << "; }\n";
+    s << "#pragma unroll 1\n      for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) {\n";
+    for (const Entry &e : es)
+      each(e, "        ") << "const " << e.type << " v = op2b_l" << e.arg << "[k], w = *(const volatile "
+                          << e.type << " *)(op2b_parts + (size_t)b * " << red << " + " << e.at
+                          << " + k); op2b_l" << e.arg << "[k] = " << e.op << "; }\n";
+    s << "      }\n    }\n#pragma unroll 1\n    for (int o = 16; o > 0; o >>= 1) {\n";
+    for (const Entry &e : es)
+      each(e, "      ") << "const " << e.type << " v = op2b_l" << e.arg
+                        << "[k], w = __shfl_down_sync(0xffffffffu, v, o); op2b_l" << e.arg
+                        << "[k] = " << e.op << "; }\n";
+    s << "    }\n    if ((threadIdx.x & 31) == 0) {\n";
+    for (const Entry &e : es)
+      each(e, "      ") << "unsigned long long u = 0; *(" << e.type << " *)&u = op2b_l" << e.arg
+                        << "[k]; op2b_rs[threadIdx.x >> 5][" << e.at << " + k] = u; }\n";
+    s << "    }\n    __syncthreads();\n    if (threadIdx.x < " << red
+      << ") {\n      unsigned long long u = op2b_rs[0][threadIdx.x];\n"
+         "#pragma unroll 1\n      for (int j = 1; j < 8; j++) {\n"
+         "        const unsigned long long x = op2b_rs[j][threadIdx.x];\n";
+    for (const Entry &e : es)
+      s << "        if (threadIdx.x >= " << e.at << " && threadIdx.x < " << e.at + e.dim << ") { const "
+        << e.type << " v = *(const " << e.type << " *)&u, w = *(const " << e.type << " *)&x; *("
+        << e.type << " *)&u = " << e.op << "; }\n";
+    s << "      }\n      if (op2b_pass) {\n        op2b_rs[0][threadIdx.x] = u;\n"
+         "        op2b_host[threadIdx.x] = u;\n      } else {\n"
+         "        op2b_parts[(size_t)blockIdx.x * " << red << " + threadIdx.x] = u;\n"
+         "        __threadfence();\n      }\n    }\n    __syncthreads();\n    if (op2b_pass) break;\n"
+         "    if (threadIdx.x == 0) op2b_last = atomicAdd(op2b_ticket, 1u) == gridDim.x - 1;\n"
+         "    __syncthreads();\n    if (!op2b_last) return;\n    __threadfence();\n  }\n"
+         "  if (threadIdx.x == 0) {\n    unsigned long long h = op2b_seq * 0x9e3779b97f4a7c15ull;\n"
+         "#pragma unroll 1\n    for (int t = 0; t < " << red << "; t++) h = op2b_mix(h, op2b_rs[0][t]);\n"
          "    op2b_host[" << red << "] = h;\n    *op2b_ticket = 0u;\n  }\n";
   } else {
     for (size_t i = 0; i < ap.size(); i++) {

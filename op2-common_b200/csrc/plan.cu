@@ -1185,7 +1185,7 @@ Plan *build_plan(const char *name, op_set set, int part_size, int nargs, op_arg 
                       s);
       if (!cuda_ok(cudaStreamSynchronize(s), "op_plan_get: colouring")) return nullptr;
     } else {
-      int *list_d = dalloc<int>(2 * (size_t)nblocks, own);
+      int *list_d = dalloc<int>(2 * (size_t)nblocks, temp);
       if (!list_d) {
         set_error("op_plan_get(%s): out of device memory", name);
         return nullptr;
@@ -1495,7 +1495,12 @@ const Plan *find_plan(const op_plan *o) {
   return nullptr;
 }
 
-void release_plans() { plan_cache().clear(); }
+// A caller may be reading a plan's device arrays on a stream of its own, which the
+// stream-ordered frees do not wait for.
+void release_plans() {
+  if (!plan_cache().empty()) cudaDeviceSynchronize();
+  plan_cache().clear();
+}
 
 }  // namespace op2b
 
@@ -1568,9 +1573,6 @@ const int *op2b_plan_device_thrcol(const op_plan *plan) {
   return pl ? pl->thrcol_d : nullptr;
 }
 
-void op2b_plan_release_all(void) {
-  cudaStreamSynchronize(rt().stream);
-  release_plans();
-}
+void op2b_plan_release_all(void) { release_plans(); }
 
 }  // extern "C"

@@ -456,7 +456,8 @@ __global__ void k_plan_fill(PlanParams p, const long long *ind_base, const int *
 // ------------------------------------------------------------------ kernel 3
 // greedy block colouring in block order (:798-884) by one CTA, then
 // ncolblk and blkmap (:886-922).  work: one bitmask per target element of
-// every OP_INC/OP_RW indirection; list: 2 x nblocks ints of scratch.
+// every OP_INC/OP_RW indirection; list: 2 x nblocks ints of scratch.  At least two
+// blocks, so of at most PLAN_MAX_PART elements.
 // The sequence is serial: a block's colour needs the masks the block before it
 // left.  So a block costs one trip to its targets' masks and one reduction: the
 // targets' addresses (a trip through the map) are loaded while the block before
@@ -1184,6 +1185,14 @@ Plan *build_plan(const char *name, op_set set, int part_size, int nargs, op_arg 
       cudaMemcpyAsync(ncolblk_d, ncb.data(), sizeof(int) * std::max(nc, 1), cudaMemcpyHostToDevice,
                       s);
       if (!cuda_ok(cudaStreamSynchronize(s), "op_plan_get: colouring")) return nullptr;
+    } else if (nblocks == 1) {
+      // one block has the one colour, without a look at its targets: of OP_COLOR2 it
+      // is the whole set, whose (argument, element) pairs need not fit an int
+      static const int kOne = 1;
+      cudaMemsetAsync(pl->blk_col_d, 0, sizeof(int), s);
+      cudaMemsetAsync(pl->blkmap_d, 0, sizeof(int), s);
+      cudaMemcpyAsync(ncolblk_d, &kOne, sizeof(int), cudaMemcpyHostToDevice, s);
+      cudaMemcpyAsync(ncolors_d, &kOne, sizeof(int), cudaMemcpyHostToDevice, s);
     } else {
       int *list_d = dalloc<int>(2 * (size_t)nblocks, temp);
       if (!list_d) {

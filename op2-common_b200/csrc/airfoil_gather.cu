@@ -380,7 +380,7 @@ struct SlotCache {
   int ring_state = 0;       // flux-ring records: 0 not tried, 1 built, -1 not possible
   int ring_ctas = 0, ring_nt = 0;
   uint2 *ring_buf = nullptr;
-  op_map linked = nullptr;  // pbecell whose boundary records are linked in (fused bres_calc)
+  const BresRecords *linked = nullptr;  // the boundary records linked in (fused bres_calc)
   int link_state = 0;       // 0 not tried, 1 linked, -1 not linkable
   std::vector<void *> owned;
   ~SlotCache() {
@@ -598,7 +598,8 @@ bool link_boundary_records(const SlotRecords *rec, const BresRecords *b, op_map 
   for (auto &p : slot_cache())
     if (&p->rec == rec) sc = p.get();
   if (!sc || !rec->corners) return false;
-  if (sc->link_state != 0) return sc->link_state == 1 && sc->linked == pbecell;
+  // (of one map to the cells and one to the nodes: not another pair's)
+  if (sc->link_state != 0) return sc->link_state == 1 && sc->linked == b;
   sc->link_state = -1;
   if (pbecell->to != sc->inc->to) return false;  // boundary cells must be the same set
   Runtime &r = rt();
@@ -622,7 +623,7 @@ bool link_boundary_records(const SlotRecords *rec, const BresRecords *b, op_map 
   }
   if (!cuda_ok(cudaStreamSynchronize(s), "boundary link")) return false;
   sc->link_state = 1;
-  sc->linked = pbecell;
+  sc->linked = b;
   return true;
 }
 

@@ -122,8 +122,9 @@ cudaError_t launch_bres_calc_records(const LaunchCtx &c, const BresRecords &b, c
 // bres_calc: a boundary cell's boundary edges go into the unused slots of its
 // corner record, after its interior slots and in edge order (meta bit 6, the
 // edge's nodes as corners, o = the boundary edge).  False when some boundary
-// edge finds no unused slot or has a node that is not a corner of its cell, or
-// the corner records are not usable; the loops then run one after the other.
+// edge finds no unused slot or has a node that is not a corner of its cell, the
+// corner records are not usable, or other boundary records (another map to the
+// cells or the nodes) are linked already; the loops then run one after the other.
 bool link_boundary_records(const SlotRecords *s, const BresRecords *b, op_map pbecell);
 // airfoil_pipe.cu: the fused kernel (block 128 or 256).  zero_res: res is
 // known to be all zeros (the update before left it so without writing it):

@@ -547,6 +547,13 @@ class GraphNet:
         self._mlp_bwd("enc_edge", E, dyE, w, ws["_edge_in"].data_ptr(), EDGE_IN, ws=ws)
         self.launches += 2
 
+    def check(self):
+        """Raises if a tensor-core kernel gave up waiting since the last check (its
+        results, and buffers that were not written, are then worthless).  Waits for the
+        device: call it where a result is read anyway."""
+        if _lib().op2b_gemm_error(1) != 0:
+            raise L.Op2Error("a tensor-core kernel gave up waiting: its results are not valid")
+
     def loss_grad(self, dg, node_in, edge_in, target, ws=None, zero_loss=True):
         """Forward, MSE against target (N x 4 float device tensor, normalised
         units), backward.  Returns the device loss accumulator (1 float): this

@@ -207,7 +207,7 @@ def train(net: G.GraphNet, data: Dataset, val: Dataset | None = None, steps=3000
             log(json.dumps(rec))
     ev1.record()
     torch.cuda.synchronize()
-    assert G._lib().op2b_gemm_error(1) == 0, "a tensor-core GEMM timed out"
+    net.check()
     return hist, ev0.elapsed_time(ev1)
 
 
@@ -220,6 +220,7 @@ def evaluate(net, data: Dataset, batch=8):
         ni, ei, tg = data.batch(b * batch, batch)
         out = net.forward(dg, ni, ei, train=False)
         tot += float(((out[:, :4] - tg) ** 2).mean().item())
+    net.check()
     return tot / max(nb, 1)
 
 
@@ -239,6 +240,7 @@ def predict_q(net: G.GraphNet, mesh: Mesh, mach, alpha, bump):
             qi.data_ptr(), q.data_ptr(), net.stream)
     res = q.cpu().numpy()
     net.release()
+    net.check()
     return res
 
 

@@ -8,8 +8,9 @@
  * owns contiguous ranges of cells and edges, declares the Airfoil dats twice
  * (float for the FP32-storage phase, double for the FP64 phase) on the same
  * sets and maps, and passes the per-instance ranges and freestream states.
- * Each loop stage then runs as one persistent launch over the still-active
- * instances; one iteration is a CUDA graph.  Instances start in FP32 storage
+ * A step then runs as two launches over the still-active instances (res_calc with
+ * bres_calc, update with the next adt_calc; a launch a loop with the other res_calc
+ * strategies); one iteration is a CUDA graph.  Instances start in FP32 storage
  * (FP64 update and rms), move to FP64 storage when their rms falls below
  * promote_tol * rms0 or stalls, and stop at rms < tol * rms0 (rms0 = rms after
  * the first iteration).
@@ -45,11 +46,12 @@ op2b_batch op2b_batch_create(const op2b_airfoil_dats *fp32, const op2b_airfoil_d
 /* keys: "tol", "promote_tol", "max_iter", "stall_window", "block" (128, 256,
  * 512), "blocks_per_sm", "res_kernel" (OP2B_BATCH_RES_*), "part_size"
  * (elements per work item, >= 256; the reference's OP_PART_SIZE,
- * op_lib_core.cpp:205-220). */
+ * op_lib_core.cpp:205-220; by default 256 to 2048, by the number of cells). */
 int op2b_batch_set(op2b_batch b, const char *key, double value);
 /* Time every (res_calc strategy: gather, atomics or colouring) x (block size:
- * 128, 256, 512) x (partition size: 512, 2048, 8192) candidate for `iters`
- * iterations, keep the fastest; the solve's state is left untouched. */
+ * 128, 256, 512) x (partition size: the default, reported as 0, 512, 8192)
+ * candidate for `iters` iterations, keep the fastest; the solve's state is left
+ * untouched. */
 int op2b_batch_tune(op2b_batch b, int iters, char *report, int report_len);
 /* Run up to max_iterations iterations (graphs when use_graph), checking for
  * completion every check_every; returns the number of instances still active,

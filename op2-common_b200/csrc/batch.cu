@@ -911,7 +911,8 @@ int op2b_batch_stats(op2b_batch b, int *iters, int *iters32, double *rms0, doubl
 }
 
 // Autotuner: time `iters` iterations of every candidate (res_calc strategy x
-// block size) on the batch as it stands, keep the fastest.  The batch state is
+// block size x item size, the default one among them) on the batch as it stands,
+// keep the fastest.  The batch state is
 // restored afterwards (q, phases and counters), so tuning does not advance the
 // solve.
 int op2b_batch_tune(op2b_batch b, int iters, char *report, int report_len) {
@@ -942,9 +943,9 @@ int op2b_batch_tune(op2b_batch b, int iters, char *report, int report_len) {
   std::vector<Cand> cands;
   for (int rk : {OP2B_BATCH_RES_GATHER, OP2B_BATCH_RES_ATOMIC, OP2B_BATCH_RES_COLOUR})
     for (int blk : {128, 256, 512})
-      for (int part : {512, 2048, 8192}) cands.push_back({rk, blk, part});
+      for (int part : {0, 512, 8192}) cands.push_back({rk, blk, part});  // 0: by the batch's size
   double best = 1e30;
-  Cand bestc = {b->res_kernel, b->block, d.chunk};
+  Cand bestc = {b->res_kernel, b->block, b->part_size};
   std::string rep;
   static const char *kRes[] = {"gather", "atomic", "colour"};
   for (const Cand &c : cands) {

@@ -814,18 +814,19 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 // wait for one another), the others by cp.async (narrow rows: TMA takes as long for
 // 16 bytes as for 128).  With all of them by cp.async, at most eight stages in
 // flight, the edge MLP's 635,000 rows took 276 us, so 209.
-// Four more warps hold the sums' rounding to that of the layer by layer products,
-// whose CTAs add up a few thousand rows each: the tensor core's accumulation
-// drifts with its length.  An accumulator is left after J.flush blocks of rows
-// and the MMAs go on in the free 128 columns of tensor memory, each accumulator at
-// blocks of its own; the warps meanwhile add the one left to the gradient or, of
-// a single 128 x 128 one, to a running sum in tensor memory (20,000 rows of three parts
-// 37.9 -> 33.8 us).  And they add d's columns up from its stages with FP32 additions, the
-// running sum compensated.  Error against FP64 sums of the same operands at 635,000
-// rows, as a part of the norm, for one accumulator a CTA, now and layer by layer:
-// dW1 2.3e-5, 2.2e-6, 2.3e-6; with a mean of one standard deviation 4.9e-5, 2.5e-6,
-// 2.6e-6 and db1 (a product with ones before) 1.3e-5, 9e-8, 2.8e-7.  It costs 1 to 2 % of
-// the edge MLP's kernel and 1.3 % of a training step.
+// Four more warps hold the sums' rounding to that of the layer by layer products, whose
+// CTAs add up a few thousand rows each: the tensor core's accumulation drifts with its
+// length.  An accumulator is left after J.flush blocks of rows, each at blocks of its
+// own.  Of one or two (128 x 128 each) the warps add it to a running sum in tensor
+// memory, of three there is room for none and they add it to the gradient; the MMAs
+// go on meanwhile in the free 128 columns (two: after the warps, the ring filling).
+// And the warps add d's columns up, as products with ones of four blocks (mma.sync on
+// ldmatrix's fragments: a tenth of the instructions of adding values one by one, which
+// held up the producers, 8 us), those by FP32 additions with compensation.  Error against
+// FP64 sums of the same operands at 635,000 rows, as a part of the norm, for one
+// accumulator a CTA, now and layer by layer: dW1 2.3e-5, 2.2e-6, 2.3e-6; with a mean of one
+// standard deviation 4.9e-5, 2.5e-6, 2.6e-6 and db1 1.3e-5, 9e-8, 2.5e-7.  The edge MLP's
+// 635,000 rows take 208 us in place of 207, the node MLP's 160,000 55 for 56.
 struct MlpDwJob {
   const __nv_bfloat16 *d;  // [M][ldd], nout columns
   long ldd;
@@ -845,8 +846,9 @@ struct MlpDwArgs {
 constexpr int kDwRing = 12, kDwLag = 8;  // (12: every stage is always the same operand's)
 constexpr int kDwProducers = 4, kDwSumWarp0 = 6, kDwSumWarps = 4;  // warps; 4: MMA, 5: TMA
 constexpr int kDwThreads = 32 * (kDwSumWarp0 + kDwSumWarps);
+constexpr int kDwStage = 4096;  // what a warp adds to the gradient at a time
 constexpr size_t kDwSmem =
-    (size_t)kDwRing * kStageBytes + kDwSumWarps * kW * 4 + (2 * kDwRing + 7) * 8 + 1024;
+    (size_t)kDwRing * kStageBytes + kDwSumWarps * kDwStage + kW * 4 + (2 * kDwRing + 7) * 8 + 1024;
 
 __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
@@ -854,10 +856,29 @@ __device__ __forceinline__ void red_add4(float *p, float a, float b, float c, fl
                : "memory");
 }
 
-// 32 columns cc .. of row n of an accumulator (and of the one before it, if any),
-// added to the gradient
+// four 8 x 8 blocks of BF16 from the rows that lanes 0-7, 8-15, .. point to, transposed
+__device__ __forceinline__ void ld_blocks(uint32_t addr, uint32_t *r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+// c[0], c[1] += the sums of the lane's two columns (2 (lane % 4) and the next one of eight)
+// over 16 rows: a product with ones, all of whose rows are the same
+__device__ __forceinline__ void add_columns(float (&c)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%4,%4,%4}, "
+      "{%5,%6}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(0x3f803f80u), "r"(b0), "r"(b1));
+}
+
+// 32 rows n .. x 32 columns cc .. of an accumulator (plus the sum of the ones before it, if
+// any), added to the gradient.  Through 4 KiB of shared memory, in the 128-byte swizzle,
+// so that a reduction of the warp covers whole lines of four rows: by the lanes' own rows,
+// 32 lines each, the reductions held up the producers' copies (edge MLP 226 us)
 __device__ __forceinline__ void dw_add(const MlpDwJob &J, uint32_t acc, bool two, uint32_t sum, int n,
-                                       int cc) {
+                                       int cc, uint8_t *stage, int lane) {
   float v[32];
   tmem_ld32(acc, v);
   if (two) {
@@ -866,11 +887,19 @@ __device__ __forceinline__ void dw_add(const MlpDwJob &J, uint32_t acc, bool two
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] += u[i];
   }
-  float *w = J.gw + (long)n * J.kin + cc;
-  if (n < J.nout) {
+  __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 8; i++)
-      if (cc + 4 * i < J.kin) red_add4(w + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  for (int i = 0; i < 8; i++)
+    *reinterpret_cast<float4 *>(stage + sw128(lane, i)) =
+        make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  __syncwarp();
+  const int c = lane & 7;
+  float *w = J.gw + (long)n * J.kin + cc + 4 * c;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int r = 4 * i + (lane >> 3);
+    const float4 t = *reinterpret_cast<const float4 *>(stage + sw128(r, c));
+    if (n + r < J.nout && cc + 4 * c < J.kin) red_add4(w + (long)r * J.kin, t.x, t.y, t.z, t.w);
   }
 }
 
@@ -892,10 +921,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t *s_ring = smem;
-  float(*s_sum)[kW] = reinterpret_cast<float(*)[kW]>(smem + (size_t)kDwRing * kStageBytes);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(s_sum + kDwSumWarps);
+  uint8_t *s_stage = smem + (size_t)kDwRing * kStageBytes;
+  float *s_sum = reinterpret_cast<float *>(s_stage + kDwSumWarps * kDwStage);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(s_sum + kW);
   uint32_t &s_taddr = *reinterpret_cast<uint32_t *>(bars + 2 * kDwRing + 3);
-  // s_place[0-2]: the accumulators' places at the end, [3]: whether there is a sum of
+  // s_place[0-2]: the accumulators' places at the end, [3]: bit p: there is a sum of
   // earlier ones, [4]: stages that the TMA warp went past
   int &s_fail = *reinterpret_cast<int *>(&s_taddr + 1), *s_place = &s_fail + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -934,24 +964,28 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   // the CTA's blocks of 64 rows
   const long nblk = ((long)g.M + 63) / 64, me = (int)blockIdx.x - J.cta0;
   const int b0 = (int)(nblk * me / J.ctas), b1 = (int)(nblk * (me + 1) / J.ctas), nb = b1 - b0;
-  // accumulator p's place (128 columns) in tensor memory and the free one's; the
-  // MMA and the sum warps exchange them alike
+  // accumulator p's place (128 columns) in tensor memory.  Of one or three the MMAs go
+  // on in the free place (one: 0 and 3 in turn), which the MMA and the sum warps
+  // exchange alike; of one or two there is room for the sums of those left before
   int acc_at[3] = {0, 1, 2}, spare = 3;
-  constexpr int kSumAt = 1;  // one accumulator only: the sum of the ones before it
-  // blocks until accumulator p is full, each at blocks of its own (the last block's
-  // are read by all warps)
-  int until[3];
+  const bool sums = P < 3;
+  auto sum_at = [&](int p) { return P == 1 ? 1 : 2 + p; };
+  // the block after which accumulator p is left, each at blocks of its own (after the
+  // last block all warps read them)
+  int leave[3];
 #pragma unroll
-  for (int p = 0; p < 3; p++) until[p] = J.flush - p * (J.flush / P);
+  for (int p = 0; p < 3; p++) leave[p] = J.flush - p * (J.flush / P) - 1;
   auto is_full = [&](int p, int b) {
-    if (--until[p] > 0) return false;
-    until[p] = J.flush;
-    return b + 1 < nb;
+    if (b != leave[p] || b + 1 == nb) return false;
+    leave[p] += J.flush;
+    return true;
   };
   auto exchange = [&](int p) {  // (p is a constant of an unrolled loop)
     const int t = acc_at[p];
-    acc_at[p] = spare;
-    spare = t;
+    if (P != 2) {
+      acc_at[p] = spare;
+      spare = t;
+    }
     return t;
   };
 
@@ -1069,7 +1103,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
     s_place[4] = it;
   } else if (warp == kDwProducers && lane == 0) {
     const uint32_t idesc = umma_idesc(kW) | 1u << 15 | 1u << 16;  // A and B MN-major
-    int it = 0, left = 0;
+    int it = 0, left = 0, kept = 0;
     bool ok = true, fresh[3] = {true, true, true};
     auto wait = [&](uint32_t bar, int n) {
       ok = ok && mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail);
@@ -1081,6 +1115,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
       wait(full(sd), it / kDwRing);
       it++;
       const uint32_t a = smem_u32(s_ring + (size_t)sd * kStageBytes);
+      if (P == 2 && left > 0) wait(acc_empty, left - 1);  // (the ring fills meanwhile)
 #pragma unroll
       for (int p = 0; p < 3; p++) {
         if (p >= P || !ok) break;
@@ -1101,6 +1136,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
           umma_commit(acc_full);
           exchange(p);
           fresh[p] = true;
+          kept |= 1 << p;
         }
       }
       if (!ok) break;
@@ -1109,41 +1145,53 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
     umma_commit(done);
 #pragma unroll
     for (int p = 0; p < 3; p++) s_place[p] = acc_at[p];
-    s_place[3] = P == 1 && left > 0;
+    s_place[3] = sums ? kept : 0;
   } else if (warp >= kDwSumWarp0) {
-    // warp w sums the rows 16 (w - 6) .. of every block of d, a lane four columns
-    const int r0 = (warp - kDwSumWarp0) * 16;
-    const uint32_t col = (uint32_t)((lane >> 4) * (kStageBytes / 2) + (lane & 1) * 8);
-    const int chunk = (lane & 15) >> 1;
-    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, rest[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    int left = 0;
+    // a warp adds up 32 columns of d, a lane two of each eight; of an accumulator that is
+    // left it takes its lane quarter
+    const int w = warp - kDwSumWarp0;
+    uint32_t place[2];  // of the lane's row in the blocks of 16 columns
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int c8 = 4 * w + 2 * u + (lane >> 4);
+      place[u] = (uint32_t)((c8 >> 3) * (kStageBytes / 2)) + sw128((lane >> 3 & 1) * 8 + (lane & 7), c8 & 7);
+    }
+    float part[4][4] = {}, sum[4][2] = {}, rest[4][2] = {};
+    int left = 0, kept = 0;
     bool ok = true;
     auto wait = [&](uint32_t bar, int n) {
       ok = __all_sync(0xffffffffu, mbar_wait_or_fail(bar, (uint32_t)(n & 1), fail));
       if (!ok && lane == 0) atomicExch(&s_fail, 1);
       return ok;
     };
+    auto fold = [&]() {  // four blocks' part into the sum, with the last addition's
+#pragma unroll           // rounding error made good, if there is one: infinities stay
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const float y = part[i][k] - rest[i][k], t = sum[i][k] + y, e = (t - sum[i][k]) - y;
+          rest[i][k] = fabsf(e) < INFINITY ? e : 0.0f;
+          sum[i][k] = t;
+          part[i][k] = 0.0f;
+        }
+    };
     for (int b = 0; b < nb && ok; b++) {
       const int it = b * (P + 1), st = it % kDwRing;
       if (!wait(full(st), it / kDwRing)) break;
-      const uint8_t *d = s_ring + (size_t)st * kStageBytes + col;
-      float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const uint32_t d = smem_u32(s_ring + (size_t)st * kStageBytes);
+      uint32_t r[8][4];  // read at once, so that the stage is free again soon
 #pragma unroll
-      for (int r = 0; r < 16; r++) {
-        const uint2 t = *reinterpret_cast<const uint2 *>(d + sw128(r0 + r, chunk));
-        part[0] += __uint_as_float(t.x << 16);
-        part[1] += __uint_as_float(t.x & 0xffff0000u);
-        part[2] += __uint_as_float(t.y << 16);
-        part[3] += __uint_as_float(t.y & 0xffff0000u);
-      }
+      for (int k = 0; k < 4; k++)
 #pragma unroll
-      for (int i = 0; i < 4; i++) {  // (with the last addition's rounding error made good,
-        const float y = part[i] - rest[i], t = sum[i] + y, e = (t - sum[i]) - y;
-        rest[i] = fabsf(e) < INFINITY ? e : 0.0f;  // if there is one: infinities stay)
-        sum[i] = t;
-      }
+        for (int u = 0; u < 2; u++) ld_blocks(d + place[u] + k * 2048, r[2 * k + u]);
       __syncwarp();
       if (lane == 0) mbar_arrive(empty(st));
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        add_columns(part[2 * (k & 1)], r[k][0], r[k][1]);
+        add_columns(part[2 * (k & 1) + 1], r[k][2], r[k][3]);
+      }
+      if (b % 4 == 3 || b + 1 == nb) fold();
 #pragma unroll
       for (int p = 0; p < 3; p++) {
         if (p >= P || !is_full(p, b)) continue;
@@ -1153,17 +1201,23 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
         const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t acc = lanes + (uint32_t)(exchange(p) * kW);
         for (int cc = 0; cc < kW; cc += 32) {
-          if (P == 1) dw_keep(acc + (uint32_t)cc, lanes + (uint32_t)(kSumAt * kW + cc), left == 1);
-          else dw_add(J, acc + (uint32_t)cc, false, 0, (warp & 3) * 32 + lane, p * kW + cc);
+          if (sums)
+            dw_keep(acc + (uint32_t)cc, lanes + (uint32_t)(sum_at(p) * kW + cc), !(kept >> p & 1));
+          else
+            dw_add(J, acc + (uint32_t)cc, false, 0, (warp & 3) * 32, p * kW + cc,
+                   s_stage + w * kDwStage, lane);
         }
-        if (P == 1) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        kept |= 1 << p;
+        if (sums) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_empty);
       }
     }
-    reinterpret_cast<float4 *>(s_sum[warp - kDwSumWarp0])[lane] =
-        make_float4(sum[0], sum[1], sum[2], sum[3]);
+    if (lane < 4)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *reinterpret_cast<float2 *>(s_sum + 32 * w + 8 * i + 2 * lane) = make_float2(sum[i][0], sum[i][1]);
   }
   __syncthreads();
   if (threadIdx.x == 0 && !mbar_wait(done, 0u)) s_fail = 1;
@@ -1175,12 +1229,14 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   if (!s_fail && nb > 0 && warp < 8) {
     // warps w and w + 4 share a lane quarter: row n of the gradient is a lane
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64)
-      dw_add(J, lanes + (uint32_t)(s_place[cc / kW] * kW + cc % kW), s_place[3] != 0,
-             lanes + (uint32_t)(kSumAt * kW + cc), (warp & 3) * 32 + lane, cc);
+    for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64) {
+      const int p = cc / kW;
+      dw_add(J, lanes + (uint32_t)(s_place[p] * kW + cc % kW), s_place[3] >> p & 1,
+             lanes + (uint32_t)(sum_at(p) * kW + cc % kW), (warp & 3) * 32, cc,
+             s_ring + warp * kDwStage, lane);  // (the ring's stages have all been used)
+    }
   } else if (!s_fail && nb > 0 && warp == 8) {
-    for (int c = lane; c < J.nout; c += 32)
-      atomicAdd(J.gb + c, (s_sum[0][c] + s_sum[1][c]) + (s_sum[2][c] + s_sum[3][c]));
+    for (int c = lane; c < J.nout; c += 32) atomicAdd(J.gb + c, s_sum[c]);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1401,14 +1457,16 @@ extern "C" int op2b_gnn_mlp_dw(int M, const void *const *d, const long *ldd, int
   int dev = 0;
   g.err = tc_error_flag(what, &dev);
   if (!g.err) return -1;
-  // CTAs by the tiles a job reads per 64 rows, a gathered one counting twice (edge
-  // MLP of 635,000 rows with random indices: 255 us with half as much again, 247 with
-  // this), at least four blocks of rows each
+  // CTAs by the operands a job reads, those that come by 16-byte copies (indexed or narrow
+  // rows) counting twice, at least four blocks of rows each.  635,000 rows, graph
+  // network's indices and 8-column encoder: 207 and 157 us; at one and a half 213 and 177,
+  // alike 241 and 243
   const int nsm = sm_count(dev), most = std::max(1, ((M + 63) / 64 + 3) / 4);
   int total = 0, at = 0, cost[3];
   for (int l = 0; l < 3; l++) {
-    cost[l] = 2 + 2 * g.job[l].nparts;
-    for (int i = 0; i < g.job[l].nparts; i++) cost[l] += g.job[l].part[i].rows ? 2 : 0;
+    const MlpDwJob &J = g.job[l];
+    cost[l] = J.nout < 64 ? 2 : 1;
+    for (int i = 0; i < J.nparts; i++) cost[l] += J.part[i].rows || J.part[i].cols < 64 ? 2 : 1;
     total += cost[l];
   }
   for (int l = 0; l < 3; l++) {

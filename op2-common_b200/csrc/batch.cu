@@ -3,7 +3,7 @@
 //
 //  * The instances are one OP2 mesh (concatenated, then renumbered so every
 //    instance owns a contiguous range of cells, edges and boundary cells).
-//  * Each loop stage is ONE persistent launch over a device-side list of work
+//  * Each stage is ONE launch over a device-side list of work
 //    items (instance, [begin, end) chunk); only unconverged instances are
 //    listed, so finished instances cost nothing and launch shapes never change.
 //  * Instances start with FP32 storage (fluxes in FP32, update and rms in
@@ -16,8 +16,8 @@
 //    active instances to mapped host memory.  The whole iteration
 //    (promotion, 2 x {res_calc + bres_calc, update} for both precisions,
 //    convergence) is captured once in a CUDA graph and replayed, the two
-//    precisions' stages on two branches (the one without instances then costs
-//    no time).
+//    precisions' stages on two branches (the launches of the one without
+//    instances, about 4 us each, then run beside the other's).
 //  * As in the runtime's own Airfoil loops, adt_calc is computed by the update
 //    before it (into a second array for the next iteration's first, so the adt
 //    dat keeps the last one), save_soln by the first update (which reads q
@@ -119,7 +119,7 @@ __global__ void k_b_res_gather(const WorkItem *items, const int *count, const in
 // records with the boundary edges linked in, corner.cuh), each instance's
 // freestream at its far-field edges: both loops' increments in their order.
 // Bound by the latency of the gathers, so float runs in 64 registers, 1024 threads an
-// SM (16 instances of 10K-100K cells, an iteration: 63 -> 59 us).  Two launches a
+// SM, double in 128, 512 threads (16 instances of 10K-100K cells, an iteration: 63 -> 59 us).  Two launches a
 // step in place of res_calc 25, bres_calc 20, adt_calc 14 and update 14 us
 // (20 iterations 2.60 -> 1.34 ms with k_b_update and the FP64 stage's own branch).
 template <typename T>

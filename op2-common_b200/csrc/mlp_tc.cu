@@ -39,7 +39,8 @@ namespace {
 
 constexpr int kW = 128;                 // hidden width
 constexpr int kProducerWarps = 3, kMmaWarp = 3, kEpiWarp0 = 4, kEpiWarps = 16;
-// 20 warps: five a scheduler, whose 16K registers allow 96 a thread
+// 20 warps: five a scheduler, whose 16K registers allow 96 a thread (k_mlp_fwd keeps 64
+// to 96 bytes a thread on the stack for it, k_mlp_bwd 8 to 20)
 constexpr int kMlpThreads = 32 * (kEpiWarp0 + kEpiWarps);
 
 struct MlpPart {
@@ -825,8 +826,9 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 // held up the producers, 8 us), those by FP32 additions with compensation.  Error against
 // FP64 sums of the same operands at 635,000 rows, as a part of the norm, for one
 // accumulator a CTA, now and layer by layer: dW1 2.3e-5, 2.2e-6, 2.3e-6; with a mean of one
-// standard deviation 4.9e-5, 2.5e-6, 2.6e-6 and db1 1.3e-5, 9e-8, 2.5e-7.  The edge MLP's
-// 635,000 rows take 208 us in place of 207, the node MLP's 160,000 55 for 56.
+// standard deviation 4.9e-5, 2.5e-6, 2.6e-6 and db1 1.3e-5, 9e-8, 2.5e-7.  In a training
+// step the edge MLP's 635,000 rows take 217 us for 208 with one accumulator, the node MLP's
+// 160,000 53 for 53, the edge encoder's 160 for 182.
 struct MlpDwJob {
   const __nv_bfloat16 *d;  // [M][ldd], nout columns
   long ldd;

@@ -4,7 +4,7 @@ Instances (meshes of uneven size, each with its own Mach number, angle of
 attack and bump height) are concatenated into one OP2 mesh, declared once
 (sets and maps) with the Airfoil dats in float and in double, renumbered
 (op_renumber: every instance then owns contiguous ranges), and solved together:
-one persistent launch per loop stage, one CUDA graph per iteration, FP32
+two launches a step over all instances, one CUDA graph per iteration, FP32
 storage until an instance's rms falls below promote_tol * rms0 (or stalls),
 FP64 to tol * rms0.
 """

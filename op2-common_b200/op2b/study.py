@@ -20,8 +20,8 @@ Each prints one JSON object per line.
   absolute tolerance tol * rms1, rms1 being plain FP64's first-iteration rms.
 * batch: many instances of uneven size and flow condition (cells log-uniform
   in [10K, 500K], Mach in [0.3, 0.7], alpha in [-4, 6] degrees, bump in
-  [0, 0.1]) to rms < tol * rms0 each: the batched form (one persistent launch
-  per loop stage over all instances, a CUDA graph per iteration, autotuned,
+  [0, 0.1]) to rms < tol * rms0 each: the batched form (two launches a step
+  over all instances, a CUDA graph per iteration, autotuned,
   FP32 then FP64 storage) against solving the instances one after another
   with plain FP64 through the OP2 API.
 """

@@ -827,8 +827,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_bwd(const __grid_constan
 // FP64 sums of the same operands at 635,000 rows, as a part of the norm, for one
 // accumulator a CTA, now and layer by layer: dW1 2.3e-5, 2.2e-6, 2.3e-6; with a mean of one
 // standard deviation 4.9e-5, 2.5e-6, 2.6e-6 and db1 1.3e-5, 9e-8, 2.5e-7.  In a training
-// step the edge MLP's 635,000 rows take 217 us for 208 with one accumulator, the node MLP's
-// 160,000 53 for 53, the edge encoder's 160 for 182.
+// step the edge MLP's 635,000 rows take 215 us for 208 with one accumulator, the node MLP's
+// 160,000 53 for 53, the edge encoder's 158 for 182.
 struct MlpDwJob {
   const __nv_bfloat16 *d;  // [M][ldd], nout columns
   long ldd;
@@ -1194,27 +1194,29 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
         add_columns(part[2 * (k & 1) + 1], r[k][2], r[k][3]);
       }
       if (b % 4 == 3 || b + 1 == nb) fold();
+      int which = -1, at = 0;  // the accumulator left after this block: at most one, and its
+                               // code once (unrolled, cold launches took 3 us longer)
 #pragma unroll
-      for (int p = 0; p < 3; p++) {
-        if (p >= P || !is_full(p, b)) continue;
-        if (!wait(acc_full, left)) break;
-        left++;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const uint32_t acc = lanes + (uint32_t)(exchange(p) * kW);
-        for (int cc = 0; cc < kW; cc += 32) {
-          if (sums)
-            dw_keep(acc + (uint32_t)cc, lanes + (uint32_t)(sum_at(p) * kW + cc), !(kept >> p & 1));
-          else
-            dw_add(J, acc + (uint32_t)cc, false, 0, (warp & 3) * 32, p * kW + cc,
-                   s_stage + w * kDwStage, lane);
-        }
-        kept |= 1 << p;
-        if (sums) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty);
+      for (int p = 0; p < 3; p++)
+        if (p < P && is_full(p, b)) which = p, at = exchange(p);
+      if (which < 0) continue;
+      if (!wait(acc_full, left)) break;
+      left++;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll 1
+      for (int cc = 0; cc < kW; cc += 32) {
+        const uint32_t acc = lanes + (uint32_t)(at * kW + cc);
+        if (sums)
+          dw_keep(acc, lanes + (uint32_t)(sum_at(which) * kW + cc), !(kept >> which & 1));
+        else
+          dw_add(J, acc, false, 0, (warp & 3) * 32, which * kW + cc, s_stage + w * kDwStage, lane);
       }
+      kept |= 1 << which;
+      if (sums) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty);
     }
     if (lane < 4)
 #pragma unroll
@@ -1231,6 +1233,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_mlp_dw(const __grid_constant_
   if (!s_fail && nb > 0 && warp < 8) {
     // warps w and w + 4 share a lane quarter: row n of the gradient is a lane
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll 1
     for (int cc = (warp >> 2) * 32; cc < P * kW; cc += 64) {
       const int p = cc / kW;
       dw_add(J, lanes + (uint32_t)(s_place[p] * kW + cc % kW), s_place[3] >> p & 1,
